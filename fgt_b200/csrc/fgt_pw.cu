@@ -6,6 +6,7 @@
 #include <utility>
 #include <vector>
 
+#include "fgt_pw64.cuh"
 #include "fgt_pw_dev.cuh"
 
 namespace fgt {
@@ -21,6 +22,9 @@ struct FormIO {
   const int* n_items;     // item count (device)
   int max_items;          // upper bound of the item count (grid sizing)
   int slab, nslab;        // x-slab grids: planes per slab and slabs per box (1: whole grids)
+  int f64;                // FP64 3D grids on the matrix instructions (fgt_pw64.cu)
+  const int* item_off;    // first item of every box of the order
+  const uint32_t* order;  // form slots, most sources first
   int* next;              // work counter (zero at launch)
 };
 
@@ -869,6 +873,29 @@ int launch_form(PWArgs<T>& a, const FormIO& io, const FormPtrs<T>& fp, DBuf<T>& 
       return 1;
     }
   }
+  if constexpr (std::is_same<T, double>::value && DIM == 3) {
+    if (io.f64) {
+      Form64 f;
+      f.form_box = io.form_box;
+      f.s_lo = io.s_lo;
+      f.s_hi = io.s_hi;
+      f.order = io.order;
+      f.items = io.items;
+      f.n_items = io.n_items;
+      f.item_off = io.item_off;
+      f.n_form = io.n_form;
+      f.ns = io.ns;
+      f.nd = io.nd;
+      f.ncomp = io.ncomp;
+      f.has_q = io.has_q;
+      f.off = fp.off;
+      f.q = fp.q;
+      f.ds = fp.ds;
+      f.rn = fp.rn;
+      f.mp = fp.mp;
+      return form64_launch(W, &a, f, s);
+    }
+  }
   if (need <= (size_t)MAXSMEM) {
     auto k = k_form<T, DIM, W, false, false>;
     set_smem(k, need);
@@ -1126,11 +1153,17 @@ int pw_form(const PWParams& P, const Tree& t, const Lists& L, const SourceSet<T>
     sp = slab_plan(a.g, sizeof(T), order_offset<T>(a.g.G, a.g.K));
   if (sp.nslab > 1) D.mp.zero();
   if (work) work->slabs_form = sp.nslab;
+  // FP64 grids that do not fit in shared memory: the matrix instructions
+  io.f64 = sizeof(T) == 8 && P.dim == 3 &&
+           sizeof(T) * (size_t)a.g.bufsz + order_offset<T>(a.g.G, a.g.K) > (size_t)MAXSMEM &&
+           form64_takes(P.w, P.K, P.G, P.wrap);
   ItemList il;
   build_items(il, L.n_form, small2 ? first.get() : nullptr, oval, L.form_box, src.lo, src.hi,
-              nullptr, nullptr, src.n, thr, true, s, sp.nslab);
+              nullptr, nullptr, src.n, thr, !io.f64, s, sp.nslab, io.f64);
   io.items = il.items;
   io.n_items = il.n_items;
+  io.item_off = il.ioff;
+  io.order = oval;
   io.max_items = il.max_items;
   io.slab = sp.planes;
   io.nslab = sp.nslab;
@@ -1141,7 +1174,7 @@ int pw_form(const PWParams& P, const Tree& t, const Lists& L, const SourceSet<T>
   fp.ds = src.ds;
   fp.rn = src.rn;
   fp.mp = D.mp;
-  DBuf<T> part((size_t)std::max(il.max_partial, 1) * P.nd * 2 * P.nexp, s);
+  DBuf<T> part((size_t)(io.f64 ? 1 : std::max(il.max_partial, 1)) * P.nd * 2 * P.nexp, s);
   fp.partial = part;
   DBuf<T> gs;
   int n;
@@ -1152,8 +1185,10 @@ int pw_form(const PWParams& P, const Tree& t, const Lists& L, const SourceSet<T>
     form_small2_w<T>(P.w, a, io, fp, oval, first, next2, s);
     n += 2;
   }
-  k_form_reduce<T><<<kSMs * 4, 256, 0, s>>>(il.split, il.n_split, P.nd, P.nexp, part, D.mp);
-  FGT_LAUNCH_CHECK();
+  if (!io.f64) {
+    k_form_reduce<T><<<kSMs * 4, 256, 0, s>>>(il.split, il.n_split, P.nd, P.nexp, part, D.mp);
+    FGT_LAUNCH_CHECK();
+  }
   n += 6;
   if (work) {
     DBuf<unsigned long long> c(1, s);

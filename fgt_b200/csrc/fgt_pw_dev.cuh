@@ -281,6 +281,27 @@ __device__ __forceinline__ int sel3(const int* ki, int i) {
   return i == 0 ? ki[0] : (i == 1 ? ki[1] : ki[2]);
 }
 
+// component factor (complex) of evaluation component c at mode ki[]
+template <typename T, int DIM>
+__device__ __forceinline__ void eval_factor(const PWArgs<T>& a, int c, const int* ki, T& fr, T& fi) {
+  if (c == 0) {
+    fr = T(1);
+    fi = T(0);
+    return;
+  }
+  if (c <= DIM) {  // i ts(k_d)/sqrt(delta0)
+    fr = T(0);
+    fi = a.ts[sel3(ki, c - 1)] * a.inv_sqd0;
+    return;
+  }
+  int m = c - 1 - DIM, p, q;
+  if (DIM == 1) { p = 0; q = 0; }
+  else if (DIM == 2) { p = (m == 2) ? 1 : 0; q = (m == 0) ? 0 : 1; }
+  else { p = m < 3 ? m : (m < 5 ? 0 : 1); q = m < 3 ? m : (m == 3 ? 1 : 2); }
+  fr = -a.ts[sel3(ki, p)] * a.ts[sel3(ki, q)] * a.inv_sqd0 * a.inv_sqd0;
+  fi = T(0);
+}
+
 // Stencil cell offsets (T units) along each dimension.  Lin: the sub-grid
 // case, cells base..base+W-1 (offsets fold into address immediates); Tab:
 // the periodic full grid, cells wrap modulo nf (one modulo per dimension).
@@ -929,7 +950,8 @@ __global__ void k_lpt_keys(int n, const int* __restrict__ count, const int* __re
 // cut-off level 0 the root box holds every point) keeps every SM busy
 // instead of one.  The items of a box are consecutive and follow the
 // longest-processing-time order of the boxes.  pslot: slot of the item's
-// partial expansion (form items of split boxes), -1 otherwise.
+// partial expansion (form items of split boxes), -1 otherwise; in lists built
+// by order, the place of the item's box in the order.
 struct WorkItem {
   int slot, part, nparts, pslot;
 };
@@ -946,7 +968,7 @@ struct SplitRec {
 __global__ void k_item_parts(int n, const int* __restrict__ count, const uint32_t* __restrict__ order,
                              const int* __restrict__ box, const int* __restrict__ lo0,
                              const int* __restrict__ hi0, const int* __restrict__ lo1,
-                             const int* __restrict__ hi1, int thr, int nslab,
+                             const int* __restrict__ hi1, int thr, int nslab, int by_order,
                              int* __restrict__ nparts, int* __restrict__ nsplit) {
   const int m = count ? *count : n;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -958,7 +980,7 @@ __global__ void k_item_parts(int n, const int* __restrict__ count, const uint32_
       np = c > thr ? (int)((c + thr - 1) / thr) : 1;
     }
     nparts[i] = np * nslab;
-    nsplit[i] = (nslab == 1 && np > 1) ? np : 0;
+    nsplit[i] = (nslab == 1 && !by_order && np > 1) ? np : 0;
   }
 }
 
@@ -969,7 +991,8 @@ __global__ void k_item_parts(int n, const int* __restrict__ count, const uint32_
 // has a partial slot (the slab kernels add into the box's expansion).
 __global__ void k_item_fill(int n, const int* __restrict__ count, const uint32_t* __restrict__ order,
                             const int* __restrict__ nparts, const int* __restrict__ ioff,
-                            const int* __restrict__ poff, int nslab, WorkItem* __restrict__ items,
+                            const int* __restrict__ poff, int nslab, int by_order,
+                            WorkItem* __restrict__ items,
                             SplitRec* __restrict__ split, int* __restrict__ nsplit_total) {
   const int m = count ? *count : n;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
@@ -979,10 +1002,10 @@ __global__ void k_item_fill(int n, const int* __restrict__ count, const uint32_t
       w.slot = slot;
       w.part = p;
       w.nparts = np;
-      w.pslot = (nslab == 1 && np > 1) ? poff[i] + p : -1;
+      w.pslot = by_order ? i : ((nslab == 1 && np > 1) ? poff[i] + p : -1);
       items[o + p] = w;
     }
-    if (nslab == 1 && np > 1 && split) {
+    if (nslab == 1 && !by_order && np > 1 && split) {
       const int k = atomicAdd(nsplit_total, 1);
       SplitRec r;
       r.slot = slot;
@@ -1011,6 +1034,7 @@ inline int eval_split_threshold(long long n) {
 // records live in the call's workspace.
 struct ItemList {
   DBuf<WorkItem> items;
+  DBuf<int> ioff;  // first item of every list entry
   DBuf<SplitRec> split;
   DBuf<int> n_items, n_split, n_partial;
   int max_items = 0, max_partial = 0;
@@ -1018,14 +1042,15 @@ struct ItemList {
 inline void build_items(ItemList& il, int n, const int* count, const uint32_t* order,
                         const int* box, const int* lo0, const int* hi0, const int* lo1,
                         const int* hi1, long long npts_bound, int thr, bool want_split,
-                        cudaStream_t s, int nslab = 1) {
+                        cudaStream_t s, int nslab = 1, bool by_order = false) {
   // every split box holds more than thr points and has at most 2*points/thr
   // parts; every other box has one
   const long long extra = 2 * (npts_bound / std::max(thr, 1)) + 1;
   il.max_items = (int)std::min<long long>(((long long)n + extra) * nslab, 1ll << 30);
   il.max_partial = (int)std::min<long long>(extra, 1ll << 30);
-  DBuf<int> np(std::max(n, 1), s), ns(std::max(n, 1), s), ioff(std::max(n, 1), s),
-      poff(std::max(n, 1), s);
+  DBuf<int> np(std::max(n, 1), s), ns(std::max(n, 1), s), poff(std::max(n, 1), s);
+  DBuf<int>& ioff = il.ioff;
+  ioff.alloc(std::max(n, 1), s);
   il.items.alloc(std::max(il.max_items, 1), s);
   il.n_items.alloc(1, s);
   il.n_partial.alloc(1, s);
@@ -1038,12 +1063,12 @@ inline void build_items(ItemList& il, int n, const int* count, const uint32_t* o
     return;
   }
   k_item_parts<<<grid_for(n, 256), 256, 0, s>>>(n, count, order, box, lo0, hi0, lo1, hi1, thr,
-                                                 nslab, np, ns);
+                                                 nslab, by_order ? 1 : 0, np, ns);
   FGT_LAUNCH_CHECK();
   exclusive_scan_i32(np, ioff, n, il.n_items, s);
   exclusive_scan_i32(ns, poff, n, il.n_partial, s);
-  k_item_fill<<<grid_for(n, 256), 256, 0, s>>>(n, count, order, np, ioff, poff, nslab, il.items,
-                                                want_split ? il.split.get() : nullptr, il.n_split);
+  k_item_fill<<<grid_for(n, 256), 256, 0, s>>>(n, count, order, np, ioff, poff, nslab,
+                                                by_order ? 1 : 0, il.items, want_split ? il.split.get() : nullptr, il.n_split);
   FGT_LAUNCH_CHECK();
 }
 

@@ -8,6 +8,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "fgt_pw64.cuh"
 #include "fgt_pw_dev.cuh"
 
 namespace fgt {
@@ -36,28 +37,9 @@ struct EvalPtrs {
   int nd, ncomp_max;
   int cell_bins;  // base cells of the sub-grid for the cell order, 0: bank-class order
   int slab, nslab;  // x-slab grids: planes per slab and slabs per box (1: whole grids)
+  const int* item_off;  // first item of every box (e64)
+  int e64;  // FP64 3D grids on the matrix instructions (fgt_pw64.cu)
 };
-
-// component factor (complex) of evaluation component c at mode ki[]
-template <typename T, int DIM>
-__device__ __forceinline__ void eval_factor(const PWArgs<T>& a, int c, const int* ki, T& fr, T& fi) {
-  if (c == 0) {
-    fr = T(1);
-    fi = T(0);
-    return;
-  }
-  if (c <= DIM) {  // i ts(k_d)/sqrt(delta0)
-    fr = T(0);
-    fi = a.ts[sel3(ki, c - 1)] * a.inv_sqd0;
-    return;
-  }
-  int m = c - 1 - DIM, p, q;
-  if (DIM == 1) { p = 0; q = 0; }
-  else if (DIM == 2) { p = (m == 2) ? 1 : 0; q = (m == 0) ? 0 : 1; }
-  else { p = m < 3 ? m : (m < 5 ? 0 : 1); q = m < 3 ? m : (m == 3 ? 1 : 2); }
-  fr = -a.ts[sel3(ki, p)] * a.ts[sel3(ki, q)] * a.inv_sqd0 * a.inv_sqd0;
-  fi = T(0);
-}
 
 // Grid of evaluation component c of expansion L in buffer B (real values).
 template <typename T, int DIM>
@@ -932,6 +914,30 @@ __global__ void k_split_fill(int n, const int* __restrict__ f, const int* __rest
   }
 }
 
+// The launch's arguments for the FP64 matrix-instruction kernels.
+inline Eval64 eval64_args(const EvalPtrs<double>& ep) {
+  Eval64 io;
+  io.loc = ep.loc;
+  io.eval_box = ep.eval_box;
+  io.boxes = ep.boxes;
+  io.nbox_dev = ep.nbox_dev;
+  io.items = ep.items;
+  io.n_items = ep.n_items;
+  io.item_off = ep.item_off;
+  io.nbox = ep.nbox;
+  for (int i = 0; i < 2; i++) {
+    io.off[i] = ep.off[i];
+    io.lo[i] = ep.lo[i];
+    io.hi[i] = ep.hi[i];
+    io.out[i] = ep.out[i];
+    io.n[i] = ep.n[i];
+    io.ncomp[i] = ep.ncomp[i];
+  }
+  io.nd = ep.nd;
+  io.ncomp_max = ep.ncomp_max;
+  return io;
+}
+
 template <typename T, int DIM, int W, bool DERIV>
 int launch_eval_k(PWArgs<T>& a, const EvalPtrs<T>& ep, DBuf<T>& gs, cudaStream_t s) {
   size_t fix = eval_offset<T>(a.g.G, a.g.K);
@@ -948,6 +954,11 @@ int launch_eval_k(PWArgs<T>& a, const EvalPtrs<T>& ep, DBuf<T>& gs, cudaStream_t
     const long padded = (nbins + nthr - 1) / nthr * nthr;
     epk.cell_bins =
         (sizeof(T) == 4 && !a.g.wrap && nb > 0 && padded <= NBINS_MAX) ? (int)nbins : 0;
+  }
+  if constexpr (DIM == 3 && std::is_same<T, double>::value && W % 2 == 0) {
+    if (ep.e64) {
+      return eval64_launch(W, DERIV, &a, eval64_args(ep), s);
+    }
   }
   if constexpr (DIM == 3) {
     if (gb && ep.nslab > 1) {  // x-slab grids
@@ -1056,6 +1067,12 @@ int eval_dim(int dim, int w, PWArgs<T>& a, const EvalPtrs<T>& ep, bool deriv, DB
 
 }  // namespace
 
+// FP64 grids that do not fit in shared memory.
+template <typename T>
+static bool e64_wanted(const Geo& g) {
+  return eval_offset<T>(g.G, g.K) + sizeof(T) * (size_t)g.bufsz > (size_t)MAXSMEM;
+}
+
 template <typename T>
 int pw_eval(const PWParams& P, const Tree& t, const Lists& L, const PWData<T>& D,
             const EvalSet<T>& e0, const EvalSet<T>& e1, int small_eval, PWWork* work,
@@ -1128,13 +1145,17 @@ int pw_eval(const PWParams& P, const Tree& t, const Lists& L, const PWData<T>& D
   ep.items = nullptr;
   ep.n_items = nullptr;
   ep.max_items = 0;
-  // grids too large for shared memory: x-slabs (3D without wrap-around)
+  // grids too large for shared memory (3D without wrap-around): FP64 on the
+  // matrix instructions, else x-slabs
   SlabPlan sp;
-  if (eval_offset<T>(a.g.G, a.g.K) + sizeof(T) * (size_t)a.g.bufsz > (size_t)MAXSMEM)
+  ep.e64 = sizeof(T) == 8 && P.dim == 3 && e64_wanted<T>(a.g) &&
+           eval64_takes(Pe.w, P.K, Pe.G, Pe.wrap);
+  if (!ep.e64 &&
+      eval_offset<T>(a.g.G, a.g.K) + sizeof(T) * (size_t)a.g.bufsz > (size_t)MAXSMEM)
     sp = slab_plan(a.g, sizeof(T), order_offset<T>(a.g.G, a.g.K));
   ep.slab = sp.planes;
   ep.nslab = sp.nslab;
-  if (work) work->slabs_eval = sp.nslab;
+  if (work) work->slabs_eval = ep.e64 ? ceil_div(Pe.G, SLAB64) : sp.nslab;
   ItemList il;
   DBuf<int> first2(1, s), next2(1, s);
   DBuf<T> gs;
@@ -1170,8 +1191,9 @@ int pw_eval(const PWParams& P, const Tree& t, const Lists& L, const PWData<T>& D
                 reinterpret_cast<const uint32_t*>(lbig.get()),
                 L.eval_box, u0 ? e0.lo : e1.lo, u0 ? e0.hi : e1.hi, (u0 && u1) ? e1.lo : nullptr,
                 (u0 && u1) ? e1.hi : nullptr, npts, eval_split_threshold(npts), false, s,
-                sp.nslab);
+                sp.nslab, ep.e64);
     ep.items = il.items;
+    ep.item_off = il.ioff;
     ep.n_items = il.n_items;
     ep.max_items = il.max_items;
     launches += 6 + eval_dim<T>(P.dim, Pe.w, a, ep, deriv, gs, s);
@@ -1209,6 +1231,8 @@ int pw_eval(const PWParams& P, const Tree& t, const Lists& L, const PWData<T>& D
         done = true;
       }
     }
+    if constexpr (sizeof(T) == 8)
+      if (P.dim == 3) done = modal64_launch(&a, eval64_args(ep), std::max(thr, 1), sm, s);
     if (done) {
     } else if (P.dim == 1) {
       set_smem(k_eval_modal<T, 1>, sm);

@@ -20,6 +20,7 @@
 
 #include <algorithm>
 #include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "fgt_prims.cuh"
@@ -1362,9 +1363,23 @@ size_t fixed_smem(const PWArgs<T>& a, int, int) {
   return order_offset<T>(a.g.G, a.g.K);
 }
 
+// Allows `bytes` of dynamic shared memory for a kernel.  The attribute belongs
+// to the kernel, not to the launch, and calls run on several host threads at
+// once: it is raised to the most the kernel can have, so that no thread
+// lowers it between another's set_smem and launch.
 template <typename KernelT>
 void set_smem(KernelT k, size_t bytes) {
-  FGT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  static thread_local std::vector<std::pair<int, KernelT>> done;
+  int dev = 0;
+  FGT_CUDA(cudaGetDevice(&dev));
+  FGT_REQUIRE(bytes <= (size_t)MAXSMEM, FGT_ERR_UNSUPPORTED, "shared memory of a CTA");
+  for (const auto& d : done)
+    if (d.first == dev && d.second == k) return;
+  cudaFuncAttributes at;
+  FGT_CUDA(cudaFuncGetAttributes(&at, k));
+  FGT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                MAXSMEM - (int)at.sharedSizeBytes));
+  done.emplace_back(dev, k);
 }
 
 }  // namespace

@@ -251,15 +251,44 @@ __global__ void __launch_bounds__(RS_THREADS) k_radix_hist(const K* __restrict__
   hist[threadIdx.x * nblocks + blockIdx.x] = h[threadIdx.x];
 }
 
+// Global start of this block's items of digit threadIdx.x.  offs: the scanned
+// counts, or (raw) the counts themselves, [digit][block]: with few blocks
+// every block sums them itself, which saves the scan's launches (up to 64
+// blocks, 2^18 items: 64 KB read from L2 per block).
+constexpr int RS_RAW = 64;
+__device__ __forceinline__ int radix_start(const int* __restrict__ offs, int nblocks, int raw) {
+  if (!raw) return offs[threadIdx.x * nblocks + blockIdx.x];
+  __shared__ int ws[RS_WARPS];
+  int tot = 0, before = 0;
+  for (int b = 0; b < nblocks; b++) {
+    const int c = offs[threadIdx.x * nblocks + b];
+    before += b < (int)blockIdx.x ? c : 0;
+    tot += c;
+  }
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int inc = tot;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += u;
+  }
+  if (lane == 31) ws[w] = inc;
+  __syncthreads();
+  int r = inc - tot + before;
+#pragma unroll
+  for (int k = 0; k < RS_WARPS; k++) r += k < w ? ws[k] : 0;
+  return r;
+}
+
 template <typename K>
 __global__ void __launch_bounds__(RS_THREADS)
     k_radix_scatter(const K* __restrict__ kin, const uint32_t* __restrict__ vin,
                     K* __restrict__ kout, uint32_t* __restrict__ vout, int n, int shift,
-                    const int* __restrict__ offs, int nblocks) {
+                    const int* __restrict__ offs, int nblocks, int raw) {
   __shared__ int base[256];
   __shared__ int wc[RS_WARPS][256];
   int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  base[tid] = offs[tid * nblocks + blockIdx.x];
+  base[tid] = radix_start(offs, nblocks, raw);
   unsigned lt = (1u << lane) - 1u;
   int tbase = blockIdx.x * RS_TILE;
   __syncthreads();
@@ -306,7 +335,7 @@ __global__ void __launch_bounds__(RS_THREADS)
 __global__ void __launch_bounds__(RS_THREADS)
     k_radix_scatter_tile(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
                          uint32_t* __restrict__ kout, uint32_t* __restrict__ vout, int n,
-                         int shift, const int* __restrict__ offs, int nblocks) {
+                         int shift, const int* __restrict__ offs, int nblocks, int raw) {
   __shared__ uint32_t sk[RS_TILE];
   __shared__ uint32_t sv[RS_TILE];
   __shared__ int run[256];    // running count per digit, then the tile's digit start
@@ -318,7 +347,7 @@ __global__ void __launch_bounds__(RS_THREADS)
   const int tbase = blockIdx.x * RS_TILE;
   const int tn = min(RS_TILE, n - tbase);
   run[tid] = 0;
-  gbase[tid] = offs[tid * nblocks + blockIdx.x];
+  gbase[tid] = radix_start(offs, nblocks, raw);
   uint32_t key[RS_ITEMS], val[RS_ITEMS];
   int rk[RS_ITEMS];
 #pragma unroll
@@ -441,11 +470,12 @@ void radix_sort_t(K* keys, uint32_t* vals, K* ktmp, uint32_t* vtmp, int n, int b
   for (int shift = 0; shift < bits; shift += 8) {
     k_radix_hist<K><<<nb, RS_THREADS, 0, s>>>(ka, n, shift, hist, nb);
     FGT_LAUNCH_CHECK();
-    exclusive_scan_i32(hist, hist, 256 * nb, nullptr, s);
+    const int raw = nb <= RS_RAW ? 1 : 0;
+    if (!raw) exclusive_scan_i32(hist, hist, 256 * nb, nullptr, s);
     if constexpr (sizeof(K) == 4)
-      k_radix_scatter_tile<<<nb, RS_THREADS, 0, s>>>(ka, va, kb, vb, n, shift, hist, nb);
+      k_radix_scatter_tile<<<nb, RS_THREADS, 0, s>>>(ka, va, kb, vb, n, shift, hist, nb, raw);
     else
-      k_radix_scatter<K><<<nb, RS_THREADS, 0, s>>>(ka, va, kb, vb, n, shift, hist, nb);
+      k_radix_scatter<K><<<nb, RS_THREADS, 0, s>>>(ka, va, kb, vb, n, shift, hist, nb, raw);
     FGT_LAUNCH_CHECK();
     std::swap(ka, kb);
     std::swap(va, vb);
@@ -474,30 +504,45 @@ void lower_bound_u64(const uint64_t* sorted, int n, const uint64_t* q, int m, in
   FGT_LAUNCH_CHECK();
 }
 
+namespace {
+// A per-thread pinned landing area of small read-backs.
+struct PinnedInts {
+  static constexpr int kMax = 80;
+  int* p = nullptr;
+  int* get() {
+    if (!p) FGT_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&p), sizeof(int) * kMax, 0));
+    return p;
+  }
+  ~PinnedInts() {
+    if (p) cudaFreeHost(p);
+  }
+};
+}  // namespace
+
 int fetch_int(const int* d, cudaStream_t s) {
   int h = 0;
-  FGT_CUDA(cudaMemcpyAsync(&h, d, sizeof(int), cudaMemcpyDeviceToHost, s));
-  FGT_CUDA(cudaStreamSynchronize(s));
+  fetch_span(d, 1, &h, s);
   return h;
 }
 
 void fetch_ints(const int* const* d, int n, int* h, cudaStream_t s) {
-  // a per-thread pinned landing area: the copies queue behind each other
-  // and one synchronisation covers them all
-  struct Pinned {
-    int* p = nullptr;
-    ~Pinned() {
-      if (p) cudaFreeHost(p);
-    }
-  };
-  static thread_local Pinned buf;
-  constexpr int kMax = 16;
-  FGT_REQUIRE(n <= kMax, FGT_ERR_UNSUPPORTED, "too many values in one read-back");
-  if (!buf.p) FGT_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&buf.p), sizeof(int) * kMax, 0));
+  // the copies queue behind each other and one synchronisation covers them all
+  static thread_local PinnedInts buf;
+  int* p = buf.get();
+  FGT_REQUIRE(n <= PinnedInts::kMax, FGT_ERR_UNSUPPORTED, "too many values in one read-back");
   for (int i = 0; i < n; i++)
-    FGT_CUDA(cudaMemcpyAsync(buf.p + i, d[i], sizeof(int), cudaMemcpyDeviceToHost, s));
+    FGT_CUDA(cudaMemcpyAsync(p + i, d[i], sizeof(int), cudaMemcpyDeviceToHost, s));
   FGT_CUDA(cudaStreamSynchronize(s));
-  for (int i = 0; i < n; i++) h[i] = buf.p[i];
+  std::copy(p, p + n, h);
+}
+
+void fetch_span(const int* d, int n, int* h, cudaStream_t s) {
+  static thread_local PinnedInts buf;
+  int* p = buf.get();
+  FGT_REQUIRE(n <= PinnedInts::kMax, FGT_ERR_UNSUPPORTED, "too many values in one read-back");
+  FGT_CUDA(cudaMemcpyAsync(p, d, sizeof(int) * n, cudaMemcpyDeviceToHost, s));
+  FGT_CUDA(cudaStreamSynchronize(s));
+  std::copy(p, p + n, h);
 }
 
 int unique_sorted_u64(const uint64_t* in, int n, uint64_t* out, cudaStream_t s) {

@@ -714,8 +714,7 @@ __global__ void __launch_bounds__(256) k_form_small2(PWArgs<T> a, FormIO io, For
 __global__ void k_first_at_most(const uint64_t* __restrict__ keys, int n, int limit,
                                 int* __restrict__ out) {
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    constexpr uint64_t MAXC = (1ull << (LPT_BITS - 1)) - 1;
-    const uint64_t v = MAXC - (uint64_t)limit;  // count <= limit  <=>  key >= v
+    const uint64_t v = lpt_key(limit);  // count <= limit  <=>  key >= v (limit a power of two)
     int lo = 0, hi = n;
     while (lo < hi) {
       const int mid = (lo + hi) >> 1;

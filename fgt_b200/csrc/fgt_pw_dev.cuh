@@ -919,29 +919,34 @@ __host__ __device__ constexpr size_t eval_offset(int G, int K) {
 }
 
 // Keys of a longest-processing-time order: entry i of a box list (list[i]
-// indexes `box`; the identity when list is null) gets key MAXC - cost, with
-// cost = points of the box in one or two evaluation sets, so an ascending
-// sort puts the most expensive boxes first.  Entries at or beyond *count
-// (when count is given) sort after all others.
-constexpr int LPT_BITS = 25;
+// indexes `box`; the identity when list is null) gets key 254 - bin, bin =
+// the cost's eighth of an octave, with cost = points of the box in one or two
+// evaluation sets, so an ascending sort of one 8-bit pass puts the most
+// expensive boxes first.  Entries at or beyond *count (when count is given)
+// sort after all others.  Powers of two end their bin: costs up to 2^k and
+// costs above it never share a key.
+constexpr int LPT_BITS = 8;
+__device__ __forceinline__ uint64_t lpt_key(long long cost) {
+  if (cost <= 1) return 254;
+  const int b = (int)(__float_as_uint((float)(cost - 1)) >> 20) - (127 << 3) + 1;
+  return (uint64_t)max(0, 254 - b);
+}
 __global__ void k_lpt_keys(int n, const int* __restrict__ count, const int* __restrict__ box,
                            const int* __restrict__ list, const int* __restrict__ lo0,
                            const int* __restrict__ hi0, const int* __restrict__ lo1,
                            const int* __restrict__ hi1, uint64_t* __restrict__ keys,
                            uint32_t* __restrict__ vals) {
   const int m = count ? *count : n;
-  constexpr uint64_t MAXC = (1ull << (LPT_BITS - 1)) - 1;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const int e = list ? list[i] : i;
     vals[i] = (uint32_t)e;
     if (i >= m) {
-      keys[i] = 1ull << (LPT_BITS - 1);
+      keys[i] = 255;
       continue;
     }
     const int b = box[e];
-    long long c = (long long)(hi0[b] - lo0[b]) + (lo1 ? (long long)(hi1[b] - lo1[b]) : 0);
-    c = c < 0 ? 0 : (c > (long long)MAXC ? (long long)MAXC : c);
-    keys[i] = MAXC - (uint64_t)c;
+    const long long c = (long long)(hi0[b] - lo0[b]) + (lo1 ? (long long)(hi1[b] - lo1[b]) : 0);
+    keys[i] = lpt_key(c);
   }
 }
 

@@ -1,8 +1,10 @@
 // Device tree build: bounding box, path keys, level-synchronous refinement,
 // 2:1 level restriction, box tables, sorted point ranges.
 #include <math.h>
+#include <stdlib.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "fgt_tree.cuh"
 
@@ -98,26 +100,6 @@ __global__ void k_box_counts(const uint64_t* __restrict__ bk, int nb, int shift,
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nb; i += gridDim.x * blockDim.x) {
     uint64_t lo = bk[i] << shift, hi = (bk[i] + 1) << shift;
     cnt[i] = dev_lower_bound(sk, ns, hi) - dev_lower_bound(sk, ns, lo);
-  }
-}
-
-// Source count of each box of level l from the exclusive prefix sums S of
-// the per-cell source counts of the full key space (2^(dim*D) cells):
-// count = S[(key+1) << shift] - S[key << shift].
-__global__ void k_box_counts_dense(const uint64_t* __restrict__ bk, int nb, int shift,
-                                   const int* __restrict__ S, int* __restrict__ cnt) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nb; i += gridDim.x * blockDim.x)
-    cnt[i] = S[(bk[i] + 1) << shift] - S[bk[i] << shift];
-}
-
-// Per-cell source counts of the full key space; lanes of a warp that hit
-// the same cell add once (points arrive in input order, often clustered).
-__global__ void k_cell_hist(const uint64_t* __restrict__ keys, int n, int* __restrict__ h) {
-  for (int i0 = blockIdx.x * blockDim.x; i0 < n; i0 += gridDim.x * blockDim.x) {
-    const int i = i0 + threadIdx.x;
-    const unsigned long long k = i < n ? keys[i] : ~0ull;
-    const unsigned peers = __match_any_sync(0xffffffffu, k);
-    if (i < n && (__ffs(peers) - 1) == (int)(threadIdx.x & 31)) atomicAdd(&h[k], __popc(peers));
   }
 }
 
@@ -266,26 +248,6 @@ __global__ void k_point_leaf(const uint64_t* __restrict__ pk, int n,
   }
 }
 
-// Dense leaf table of the finest cells (small key spaces): the leaves'
-// start keys, sorted, cut the 2^(dim*D) cells into the leaves' ranges;
-// table[c] = ordinal of the leaf whose range holds cell c.
-__global__ void k_cell_leaf(const uint64_t* __restrict__ ls, int nl, long long ncell,
-                            uint32_t* __restrict__ table) {
-  for (int o = blockIdx.x; o < nl; o += gridDim.x) {
-    const long long c0 = (long long)ls[o], c1 = o + 1 < nl ? (long long)ls[o + 1] : ncell;
-    for (long long c = c0 + threadIdx.x; c < c1; c += blockDim.x) table[c] = (uint32_t)o;
-  }
-}
-// Leaf ordinal of each point by the dense table (value: the original index).
-__global__ void k_point_leaf_dense(const uint64_t* __restrict__ pk, int n,
-                                   const uint32_t* __restrict__ table, uint32_t* __restrict__ ord,
-                                   uint32_t* __restrict__ idx) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    ord[i] = table[pk[i]];
-    idx[i] = (uint32_t)i;
-  }
-}
-
 // leaf_lo[o] = first sorted position with ordinal >= o, o = 0..nl
 __global__ void k_leaf_point_lo(const uint32_t* __restrict__ ord, int n, int nl,
                                 int* __restrict__ lo) {
@@ -357,6 +319,490 @@ void tree_setup_scalars(int dim, double delta, double eps, int iperiod, const do
 }
 
 namespace {
+// ------------------------------------------------------------- dense tree
+// Tree over dense tables of the key space above the finest level: cell c of
+// level l is key c, the cells of level l start at lev_off(l) of tables that
+// hold all levels 0 .. D-1 one after the other.  A box exists where its
+// parent's cell is flagged non-leaf, so the rank R of a flagged cell among
+// all flagged cells numbers its children: box 1 + mc R + digit (level-major,
+// keys ascending), and every step runs over cells without knowing a level's
+// box count on the host.
+struct CellLevels {
+  int dim, D;
+  __host__ __device__ long long cells(int l) const { return 1ll << (dim * l); }
+  __host__ __device__ long long off(int l) const {
+    return ((1ll << (dim * l)) - 1) / ((1 << dim) - 1);
+  }
+};
+
+// Keys of sources and targets (one launch) and the source counts of the
+// cells of level D-1.  Few cells: counted per block in shared memory first;
+// lanes of a warp that hit the same cell add once.
+constexpr int HIST_SMEM = 4096;
+template <int DIM, bool SMEM>
+__global__ void __launch_bounds__(256)
+    k_keys_hist(const double* __restrict__ xs, int ns, const double* __restrict__ xt, int nt,
+                KeyParams p, uint32_t* __restrict__ ks, uint32_t* __restrict__ kt,
+                int* __restrict__ hist, int ncell) {
+  __shared__ int sh[SMEM ? HIST_SMEM : 1];
+  if (SMEM) {
+    for (int i = threadIdx.x; i < ncell; i += blockDim.x) sh[i] = 0;
+    __syncthreads();
+  }
+  const long long n = (long long)ns + nt;
+  for (long long i0 = (long long)blockIdx.x * blockDim.x; i0 < n;
+       i0 += (long long)gridDim.x * blockDim.x) {
+    const long long i = i0 + threadIdx.x;
+    uint32_t key = 0;
+    const bool src = i < ns;
+    if (i < n) {
+      const double* x = src ? xs + (size_t)i * DIM : xt + (size_t)(i - ns) * DIM;
+      double c[DIM], xi[DIM];
+#pragma unroll
+      for (int k = 0; k < DIM; k++) {
+        c[k] = p.cen0[k];
+        xi[k] = x[k];
+      }
+      for (int l = 0; l < p.D; l++) {
+        uint32_t dig = 0;
+        const double h = p.bsh[l];
+#pragma unroll
+        for (int k = 0; k < DIM; k++) {
+          const bool up = (xi[k] - c[k] >= 0);
+          dig |= (up ? 1u : 0u) << k;
+          c[k] = c[k] + (up ? h : -h);
+        }
+        key = (key << DIM) | dig;
+      }
+      if (src) ks[i] = key;
+      else kt[i - ns] = key;
+    }
+    const uint32_t cell = src ? key >> DIM : 0xffffffffu;
+    const unsigned peers = __match_any_sync(0xffffffffu, cell);
+    if (src && (__ffs(peers) - 1) == (int)(threadIdx.x & 31)) {
+      if (SMEM) atomicAdd(&sh[cell], __popc(peers));
+      else atomicAdd(&hist[cell], __popc(peers));
+    }
+  }
+  if (SMEM) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < ncell; i += blockDim.x)
+      if (sh[i]) atomicAdd(&hist[i], sh[i]);
+  }
+}
+
+// Counts and non-leaf flags of levels lhi .. lhi-q from the counts of level
+// lhi: one block per cell of level lhi-q sums its subtree in shared memory.
+constexpr int PYR_CELLS = 4096;
+__global__ void __launch_bounds__(256)
+    k_pyramid(CellLevels cl, int lhi, int q, int ndiv, int* __restrict__ cnt,
+              unsigned char* __restrict__ flag) {
+  __shared__ int sc[PYR_CELLS];
+  int n = 1 << (cl.dim * q);
+  {
+    const long long o = cl.off(lhi) + (long long)blockIdx.x * n;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+      const int c = cnt[o + i];
+      sc[i] = c;
+      flag[o + i] = c > ndiv ? 1 : 0;
+    }
+  }
+  __syncthreads();
+  const int mc = 1 << cl.dim;
+  for (int l = lhi - 1; l >= lhi - q; l--) {
+    const int m = n >> cl.dim;
+    int v[PYR_CELLS / 2 / 256];
+    int k = 0;
+    for (int i = threadIdx.x; i < m; i += blockDim.x, k++) {
+      int a = 0;
+      for (int j = 0; j < mc; j++) a += sc[i * mc + j];
+      v[k] = a;
+    }
+    __syncthreads();
+    const long long o = cl.off(l) + (long long)blockIdx.x * m;
+    k = 0;
+    for (int i = threadIdx.x; i < m; i += blockDim.x, k++) {
+      sc[i] = v[k];
+      flag[o + i] = v[k] > ndiv ? 1 : 0;
+      if (l == lhi - q) cnt[o + i] = v[k];
+    }
+    __syncthreads();
+    n = m;
+  }
+}
+
+// Level restriction (k_touching_parents) on the flags: every level-(l-1)
+// cell whose closure touches a non-leaf cell of level l becomes non-leaf.
+__device__ __forceinline__ void touch_parents(const CellLevels& cl, int l, uint32_t cell,
+                                              unsigned char* flag) {
+  const int dim = cl.dim, mc = 1 << dim;
+  uint32_t c[FGT_MAXDIM];
+  key_to_coords(cell, l, dim, c);
+  const uint32_t lim = 1u << (l - 1);
+  const long long o = cl.off(l - 1);
+  for (int j = 0; j < mc; j++) {
+    uint32_t q[FGT_MAXDIM];
+    for (int k = 0; k < dim; k++) {
+      const uint32_t m = c[k] >> 1;
+      q[k] = m;
+      if ((j >> k) & 1) {
+        const long long t = (c[k] & 1) ? (long long)m + 1 : (long long)m - 1;
+        if (t >= 0 && t < (long long)lim) q[k] = (uint32_t)t;
+      }
+    }
+    flag[o + (long long)coords_to_key(q, l - 1, dim)] = 1;
+  }
+}
+__global__ void k_restrict(CellLevels cl, int l, unsigned char* __restrict__ flag) {
+  const long long n = cl.cells(l), o = cl.off(l);
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (long long)gridDim.x * blockDim.x)
+    if (flag[o + i]) touch_parents(cl, l, (uint32_t)i, flag);
+}
+// levels lmax .. 2 in one block (few cells)
+__global__ void __launch_bounds__(1024)
+    k_restrict_rest(CellLevels cl, int lmax, unsigned char* flag) {
+  for (int l = lmax; l >= 2; l--) {
+    const int n = (int)cl.cells(l);
+    const long long o = cl.off(l);
+    for (int i = threadIdx.x; i < n; i += blockDim.x)
+      if (flag[o + i]) touch_parents(cl, l, (uint32_t)i, flag);
+    __syncthreads();
+  }
+}
+
+// Exclusive scans over cells in two launches: block sums of 4096 cells, then
+// every block adds the sums before it and writes its cells.  OP gives a
+// cell's value and takes its exclusive prefix.
+constexpr int CS_T = 256, CS_I = 16, CS_TILE = CS_T * CS_I;
+__device__ __forceinline__ int block_sum(int v, int* ws) {
+#pragma unroll
+  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = v;
+  __syncthreads();
+  int r = 0;
+#pragma unroll
+  for (int w = 0; w < CS_T / 32; w++) r += ws[w];
+  __syncthreads();
+  return r;
+}
+template <class OP>
+__global__ void __launch_bounds__(CS_T) k_cells_sum(OP op, long long n, int* __restrict__ part) {
+  __shared__ int ws[CS_T / 32];
+  const long long b = (long long)blockIdx.x * CS_TILE + threadIdx.x * CS_I;
+  int v = 0;
+  for (int j = 0; j < CS_I; j++)
+    if (b + j < n) v += op.value(b + j);
+  v = block_sum(v, ws);
+  if (threadIdx.x == 0) part[blockIdx.x] = v;
+}
+template <class OP>
+__global__ void __launch_bounds__(CS_T) k_cells_scan(OP op, long long n, const int* __restrict__ part) {
+  __shared__ int ws[CS_T / 32];
+  int before = 0;
+  for (int i = threadIdx.x; i < (int)blockIdx.x; i += CS_T) before += part[i];
+  before = block_sum(before, ws);
+  const long long b = (long long)blockIdx.x * CS_TILE + threadIdx.x * CS_I;
+  int v[CS_I], s = 0;
+#pragma unroll
+  for (int j = 0; j < CS_I; j++) {
+    v[j] = b + j < n ? op.value(b + j) : 0;
+    s += v[j];
+  }
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int inc = s;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += u;
+  }
+  if (lane == 31) ws[w] = inc;
+  __syncthreads();
+  int ex = before + inc - s;
+#pragma unroll
+  for (int k = 0; k < CS_T / 32; k++) ex += k < w ? ws[k] : 0;
+#pragma unroll
+  for (int j = 0; j < CS_I; j++) {
+    if (b + j < n) op.put(b + j, ex, v[j]);
+    ex += v[j];
+    if (b + j == n - 1) op.total(ex);
+  }
+}
+
+// Rank of every flagged cell, and the ranks at which the levels start.
+struct RankOp {
+  CellLevels cl;
+  const unsigned char* flag;
+  int *rank, *lev;  // lev: D+1 entries, the last is the total
+  __device__ int value(long long i) const { return flag[i]; }
+  __device__ void put(long long i, int ex, int) const {
+    rank[i] = ex;
+    for (int l = 0; l < cl.D; l++)
+      if (i == cl.off(l)) lev[l] = ex;
+  }
+  __device__ void total(int t) const { lev[cl.D] = t; }
+};
+// Leaves that start at a cell of level D-1, in key order: the mc children of
+// a flagged cell, else one where the cell is the first of its leaf.
+struct LeafOp {
+  CellLevels cl;
+  const unsigned char* flag;
+  int* base;        // exclusive leaf count; total at [cells(D-1)]
+  uint32_t* table;  // flagged: base | 2^31, else the ordinal of the cell's leaf
+  __device__ int value(long long i) const {
+    const int L = cl.D - 1;
+    if (flag[cl.off(L) + i]) return 1 << cl.dim;
+    int l = 0;  // level of the leaf that holds the cell
+    while (l < L && flag[cl.off(l) + (i >> (cl.dim * (L - l)))]) l++;
+    return (i & ((1ll << (cl.dim * (L - l))) - 1)) == 0 ? 1 : 0;
+  }
+  __device__ void put(long long i, int ex, int v) const {
+    base[i] = ex;
+    table[i] = v > 1 ? ((uint32_t)ex | 0x80000000u) : (uint32_t)(ex + v - 1);
+  }
+  __device__ void total(int t) const { base[cl.cells(cl.D - 1)] = t; }
+};
+
+// Box tables: the children of every flagged cell (and the root); lref: the
+// reference box of every leaf by ordinal (itself, or its parent at level D-1,
+// the cut-off level).
+__global__ void k_dense_boxes(CellLevels cl, KeyParams kp, const unsigned char* __restrict__ flag,
+                              const int* __restrict__ rank, const int* __restrict__ base,
+                              uint64_t* __restrict__ key, int* __restrict__ level,
+                              int* __restrict__ nonleaf, int* __restrict__ parent,
+                              int* __restrict__ child0, double* __restrict__ center,
+                              int* __restrict__ lref, int nboxes, int nleaves) {
+  const int dim = cl.dim, mc = 1 << dim, L = cl.D - 1;
+  const long long T = cl.off(cl.D);
+  for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < T * mc + 1;
+       g += (long long)gridDim.x * blockDim.x) {
+    int b, l, par;
+    uint32_t k;
+    if (g == T * mc) {  // the root
+      b = 0;
+      l = 0;
+      k = 0;
+      par = -1;
+    } else {
+      const long long i = g / mc;
+      const int j = (int)(g - i * mc);
+      if (!flag[i]) continue;
+      int pl = 0;
+      while (pl < L && i >= cl.off(pl + 1)) pl++;
+      const uint32_t c = (uint32_t)(i - cl.off(pl));
+      b = 1 + mc * rank[i] + j;
+      l = pl + 1;
+      k = (c << dim) | (uint32_t)j;
+      par = pl == 0 ? 0 : 1 + mc * rank[cl.off(pl - 1) + (c >> dim)] + (int)(c & (mc - 1));
+    }
+    if (!FGT_DCHECK(b < nboxes, 503)) continue;
+    const bool nl = l <= L && flag[cl.off(l) + k];
+    key[b] = k;
+    level[b] = l;
+    nonleaf[b] = nl ? 1 : 0;
+    parent[b] = par;
+    child0[b] = nl ? 1 + mc * rank[cl.off(l) + k] : -1;
+    double c[FGT_MAXDIM];
+    for (int d = 0; d < dim; d++) c[d] = kp.cen0[d];
+    for (int j = 0; j < l; j++) {
+      const int dig = (int)((k >> (dim * (l - 1 - j))) & (uint32_t)(mc - 1));
+      for (int d = 0; d < dim; d++) c[d] = c[d] + (((dig >> d) & 1) ? kp.bsh[j] : -kp.bsh[j]);
+    }
+    for (int d = 0; d < dim; d++) center[(size_t)b * dim + d] = c[d];
+    if (!nl) {
+      const int o = l <= L ? base[(long long)k << (dim * (L - l))] : base[k >> dim] + (int)(k & (mc - 1));
+      if (FGT_DCHECK(o < nleaves, 504)) lref[o] = l <= L ? b : par;
+    }
+  }
+}
+
+// Leaf ordinal of every point of both sets.
+__global__ void k_dense_ordinals(int dim, const uint32_t* __restrict__ ks, int ns,
+                                 const uint32_t* __restrict__ kt, int nt,
+                                 const uint32_t* __restrict__ table, uint32_t* __restrict__ os,
+                                 uint32_t* __restrict__ is, uint32_t* __restrict__ ot,
+                                 uint32_t* __restrict__ it) {
+  const long long n = (long long)ns + nt;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (long long)gridDim.x * blockDim.x) {
+    const bool src = i < ns;
+    const uint32_t j = (uint32_t)(src ? i : i - ns), k = src ? ks[j] : kt[j], t = table[k >> dim];
+    const uint32_t o = (t >> 31) ? (t & 0x7fffffffu) + (k & ((1u << dim) - 1)) : t;
+    (src ? os : ot)[j] = o;
+    (src ? is : it)[j] = j;
+  }
+}
+// First sorted point of every leaf, both sets (k_leaf_point_lo), and the
+// reference box of every sorted point (k_point_ref).
+__global__ void k_dense_leaf_points(const uint32_t* __restrict__ os, int ns,
+                                    const uint32_t* __restrict__ ot, int nt, int nl,
+                                    const int* __restrict__ lref, int* __restrict__ slo,
+                                    int* __restrict__ tlo, int* __restrict__ sref,
+                                    int* __restrict__ tref) {
+  const long long np = (long long)ns + nt, n = np + 2 * ((long long)nl + 1);
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (long long)gridDim.x * blockDim.x) {
+    if (i < np) {
+      if (i < ns) sref[i] = lref[os[i]];
+      else tref[i - ns] = lref[ot[i - ns]];
+      continue;
+    }
+    const bool src = i - np <= nl;
+    const uint32_t o = (uint32_t)(src ? i - np : i - np - nl - 1);
+    const uint32_t* ord = src ? os : ot;
+    int a = 0, b = src ? ns : nt;
+    while (a < b) {
+      const int m = (a + b) >> 1;
+      if (ord[m] < o) a = m + 1; else b = m;
+    }
+    (src ? slo : tlo)[o] = a;
+  }
+}
+__global__ void k_dense_ranges(CellLevels cl, int nboxes, const uint64_t* __restrict__ key,
+                               const int* __restrict__ level, const int* __restrict__ base,
+                               const int* __restrict__ slo, const int* __restrict__ tlo,
+                               int* __restrict__ s0, int* __restrict__ s1, int* __restrict__ t0,
+                               int* __restrict__ t1) {
+  const int L = cl.D - 1;
+  for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nboxes; b += gridDim.x * blockDim.x) {
+    const int l = level[b];
+    const long long k = (long long)key[b];
+    int a, c;
+    if (l <= L) {
+      const int sh = cl.dim * (L - l);
+      a = base[k << sh];
+      c = base[(k + 1) << sh];
+    } else {
+      a = base[k >> cl.dim] + (int)(k & ((1 << cl.dim) - 1));
+      c = a + 1;
+    }
+    s0[b] = slo[a];
+    s1[b] = slo[c];
+    t0[b] = tlo[a];
+    t1[b] = tlo[c];
+  }
+}
+
+// The dense tables hold 2^(dim (D-1)) cells at the finest level they cover:
+// taken when clearing and scanning them (about 20 bytes a cell) stays small
+// against the points; up to 2^21 cells (~20 us) always.  Bound by launches
+// for few points and by HBM for many.  Tree phase against sorted keys, level
+// by level with a read-back each: uniform N = 1e5 (D = 6) 0.64 -> 0.27 ms,
+// N = 3e3 (D = 5) 0.43 -> 0.22 ms, clusters N + M = 4e6 (D = 8) 1.76 -> 0.83
+// ms, 2D periodic N = 1e7 2.14 -> 1.07 ms.  FGT_TREE_SORTED=1 takes the sorted
+// keys, to compare the two.
+bool dense_tree_takes(int dim, int D, int ns, int nt) {
+  if (D < 1 || dim * (D - 1) > 24 || ns < 1) return false;
+  const char* e = getenv("FGT_TREE_SORTED");
+  if (e && e[0] == '1') return false;
+  return (1ll << (dim * (D - 1))) <= 4 * ((long long)ns + nt) + (1ll << 21);
+}
+
+void tree_build_dense(Tree& t, const KeyParams& kp, const double* d_src, const double* d_trg,
+                      cudaStream_t s) {
+  const int dim = t.dim, D = t.D, mc = t.mc, ns = t.ns, nt = t.nt;
+  const CellLevels cl{dim, D};
+  const long long C1 = cl.cells(D - 1), T = cl.off(D), np = (long long)ns + nt;
+  DBuf<uint32_t> ks(ns, s), kt(std::max(nt, 1), s), table((size_t)C1, s);
+  DBuf<int> cnt((size_t)T, s), rank((size_t)T, s), base((size_t)C1 + 1, s), lev(D + 1, s);
+  DBuf<unsigned char> flag((size_t)T, s);
+  // 1. keys and source counts of the cells
+  int* hist = cnt.get() + cl.off(D - 1);
+  FGT_CUDA(cudaMemsetAsync(hist, 0, sizeof(int) * C1, s));
+  auto keys = [&](auto d) {
+    constexpr int DIM = decltype(d)::value;
+    if (C1 <= HIST_SMEM)
+      k_keys_hist<DIM, true><<<grid_for(np, 256, 8), 256, 0, s>>>(d_src, ns, d_trg, nt, kp, ks, kt,
+                                                                  hist, (int)C1);
+    else
+      k_keys_hist<DIM, false><<<grid_for(np, 256), 256, 0, s>>>(d_src, ns, d_trg, nt, kp, ks, kt,
+                                                               hist, (int)C1);
+    FGT_LAUNCH_CHECK();
+  };
+  if (dim == 1) keys(std::integral_constant<int, 1>{});
+  else if (dim == 2) keys(std::integral_constant<int, 2>{});
+  else keys(std::integral_constant<int, 3>{});
+  // 2. refinement on source counts (pts_tree_build, pts_tree_nd.f:520-590)
+  for (int lhi = D - 1;;) {
+    const int q = std::min(lhi, 12 / dim);
+    k_pyramid<<<(unsigned)cl.cells(lhi - q), 256, 0, s>>>(cl, lhi, q, t.ndiv, cnt, flag);
+    FGT_LAUNCH_CHECK();
+    lhi -= q;
+    if (lhi == 0) break;
+  }
+  // 3. level restriction (minimal 2:1 balanced refinement)
+  int l = D - 1;
+  for (; l >= 2 && cl.cells(l) > 16384; l--) {
+    k_restrict<<<grid_for(cl.cells(l), 256), 256, 0, s>>>(cl, l, flag);
+    FGT_LAUNCH_CHECK();
+  }
+  if (l >= 2) {
+    k_restrict_rest<<<1, 1024, 0, s>>>(cl, l, flag);
+    FGT_LAUNCH_CHECK();
+  }
+  // 4. box numbers and leaf ordinals
+  auto scan = [&](const auto& op, long long n) {
+    const int nb = ceil_div(n, CS_TILE);
+    DBuf<int> part(nb, s);
+    k_cells_sum<<<nb, CS_T, 0, s>>>(op, n, part.get());
+    FGT_LAUNCH_CHECK();
+    k_cells_scan<<<nb, CS_T, 0, s>>>(op, n, part.get());
+    FGT_LAUNCH_CHECK();
+  };
+  scan(RankOp{cl, flag, rank, lev}, T);
+  scan(LeafOp{cl, flag, base, table}, C1);
+  DBuf<uint32_t> os(ns, s), ot(std::max(nt, 1), s);
+  t.isrc.alloc(ns, s);
+  t.itrg.alloc(std::max(nt, 1), s);
+  k_dense_ordinals<<<grid_for(np, 256), 256, 0, s>>>(dim, ks, ns, kt, nt, table, os, t.isrc, ot,
+                                                     t.itrg);
+  FGT_LAUNCH_CHECK();
+  int h[66];
+  fetch_span(lev, D + 1, h, s);
+  int nlevels = 0;
+  while (nlevels < D && h[nlevels + 1] > h[nlevels]) nlevels++;
+  t.nlevels = nlevels;
+  t.lev_start.assign(nlevels + 2, 0);
+  t.lev_start[1] = 1;
+  for (int k = 1; k <= nlevels; k++) t.lev_start[k + 1] = 1 + mc * h[k];
+  const int nboxes = t.nboxes = 1 + mc * h[D], nl = t.nleaves = nboxes - h[D];
+  t.boxsize.resize(nlevels + 1);
+  t.boxsize[0] = t.bs0;
+  for (int k = 1; k <= nlevels; k++) t.boxsize[k] = t.boxsize[k - 1] / 2;
+  // 5. box tables
+  t.key.alloc(nboxes, s);
+  t.level.alloc(nboxes, s);
+  t.nonleaf.alloc(nboxes, s);
+  t.parent.alloc(nboxes, s);
+  t.child0.alloc(nboxes, s);
+  t.center.alloc((size_t)nboxes * dim, s);
+  DBuf<int> lref(nl, s), slo(nl + 1, s), tlo(nl + 1, s);
+  k_dense_boxes<<<grid_for(T * mc + 1, 256), 256, 0, s>>>(cl, kp, flag, rank, base, t.key, t.level,
+                                                         t.nonleaf, t.parent, t.child0, t.center,
+                                                         lref, nboxes, nl);
+  FGT_LAUNCH_CHECK();
+  // 6. leaf order of the points (stable by original index)
+  const int obits = bits_for(nl);
+  DBuf<uint32_t> otmp(std::max(ns, nt), s), vtmp(std::max(ns, nt), s);
+  radix_sort_u32(os, t.isrc, otmp, vtmp, ns, obits, s);
+  if (nt > 0) radix_sort_u32(ot, t.itrg, otmp, vtmp, nt, obits, s);
+  t.src_ref.alloc(ns, s);
+  t.trg_ref.alloc(std::max(nt, 1), s);
+  k_dense_leaf_points<<<grid_for(np + 2 * ((long long)nl + 1), 256), 256, 0, s>>>(
+      os, ns, ot, nt, nl, lref, slo, tlo, t.src_ref, t.trg_ref);
+  FGT_LAUNCH_CHECK();
+  t.src_lo.alloc(nboxes, s);
+  t.src_hi.alloc(nboxes, s);
+  t.trg_lo.alloc(nboxes, s);
+  t.trg_hi.alloc(nboxes, s);
+  k_dense_ranges<<<grid_for(nboxes, 256), 256, 0, s>>>(cl, nboxes, t.key, t.level, base, slo, tlo,
+                                                      t.src_lo, t.src_hi, t.trg_lo, t.trg_hi);
+  FGT_LAUNCH_CHECK();
+}
+
+}  // namespace
+
+namespace {
 __global__ void k_fill_int(int* __restrict__ a, int n, int v) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) a[i] = v;
 }
@@ -391,34 +837,19 @@ void tree_build(Tree& t, int dim, int iperiod, int npwlevel, int ndiv, double bs
       bs = bsc;
     }
   }
+  if (dense_tree_takes(dim, D, ns, nt)) {
+    tree_build_dense(t, kp, d_src, d_trg, s);
+    return;
+  }
   // 1. full keys of sources and targets
   DBuf<uint64_t> skey(ns, s), tkey(nt, s), ksorted, ktmp(std::max(ns, nt), s);
   if (ns > 0) launch_point_keys(dim, d_src, ns, kp, skey, s);
   if (nt > 0) launch_point_keys(dim, d_trg, nt, kp, tkey, s);
-  // Source counts per box come from a dense histogram of the full keys
-  // (prefix sums over the 2^(dim*D) finest cells) when the key space is
-  // small, and not much larger than the point set (clearing and scanning
-  // 2^24 cells costs ~0.3 ms, far more than sorting a few thousand keys),
-  // else from binary searches in the sorted keys.
-  const bool dense =
-      dim * D <= 24 && (1ll << (dim * D)) <= 4ll * ((long long)ns + nt) + (1ll << 18);
-  DBuf<int> cellsum;
-  if (dense) {
-    const int ncell = 1 << (dim * D);
-    cellsum.alloc((size_t)ncell + 1, s);
-    cellsum.zero();
-    if (ns > 0) {
-      k_cell_hist<<<grid_for(ns, 256), 256, 0, s>>>(skey, ns, cellsum);
-      FGT_LAUNCH_CHECK();
-    }
-    exclusive_scan_i32(cellsum, cellsum, ncell + 1, nullptr, s);
-  } else {
-    ksorted.alloc(std::max(ns, 1), s);
-    if (ns > 0)
-      FGT_CUDA(cudaMemcpyAsync(ksorted.get(), skey.get(), sizeof(uint64_t) * ns,
-                               cudaMemcpyDeviceToDevice, s));
-    radix_sort(ksorted, nullptr, ktmp, nullptr, ns, dim * D, s);
-  }
+  ksorted.alloc(std::max(ns, 1), s);
+  if (ns > 0)
+    FGT_CUDA(cudaMemcpyAsync(ksorted.get(), skey.get(), sizeof(uint64_t) * ns,
+                             cudaMemcpyDeviceToDevice, s));
+  radix_sort(ksorted, nullptr, ktmp, nullptr, ns, dim * D, s);
 
   // 2. refinement on source counts (pts_tree_build, pts_tree_nd.f:520-590)
   std::vector<DBuf<uint64_t>> lk;   // keys of each level
@@ -431,10 +862,7 @@ void tree_build(Tree& t, int dim, int iperiod, int npwlevel, int ndiv, double bs
   for (int l = 0; l < D; l++) {
     int nb = nlk[l];
     DBuf<int> cnt(nb, s), flag(nb, s), pos(nb, s), tot(1, s);
-    if (dense)
-      k_box_counts_dense<<<grid_for(nb, 256), 256, 0, s>>>(lk[l], nb, dim * (D - l), cellsum, cnt);
-    else
-      k_box_counts<<<grid_for(nb, 256), 256, 0, s>>>(lk[l], nb, dim * (D - l), ksorted, ns, cnt);
+    k_box_counts<<<grid_for(nb, 256), 256, 0, s>>>(lk[l], nb, dim * (D - l), ksorted, ns, cnt);
     FGT_LAUNCH_CHECK();
     k_flag_gt<<<grid_for(nb, 256), 256, 0, s>>>(cnt, nb, ndiv, flag);
     FGT_LAUNCH_CHECK();
@@ -548,18 +976,8 @@ void tree_build(Tree& t, int dim, int iperiod, int npwlevel, int ndiv, double bs
     DBuf<uint32_t> vtmp(std::max(std::max(ns, nt), 1), s);
     uint32_t* otmp = reinterpret_cast<uint32_t*>(ktmp.get());  // >= max(ns, nt) u32
     t.isrc.alloc(std::max(ns, 1), s);
-    DBuf<uint32_t> table;
-    if (dense && nl > 0) {  // leaf ordinals by table lookup instead of binary search
-      const long long ncell = 1ll << (dim * D);
-      table.alloc((size_t)ncell, s);
-      k_cell_leaf<<<std::min(nl, kSMs * 16), 256, 0, s>>>(ls, nl, ncell, table);
-      FGT_LAUNCH_CHECK();
-    }
     auto point_leaf = [&](const uint64_t* keys, int n, uint32_t* o, uint32_t* idx) {
-      if (table.p)
-        k_point_leaf_dense<<<grid_for(n, 256), 256, 0, s>>>(keys, n, table, o, idx);
-      else
-        k_point_leaf<<<grid_for(n, 256), 256, 0, s>>>(keys, n, ls, nl, o, idx);
+      k_point_leaf<<<grid_for(n, 256), 256, 0, s>>>(keys, n, ls, nl, o, idx);
       FGT_LAUNCH_CHECK();
     };
     if (ns > 0) {

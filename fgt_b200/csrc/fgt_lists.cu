@@ -169,7 +169,7 @@ __device__ __forceinline__ int colleague_of(const TV& tv, int b, int periodic, i
 
 template <int DIM, bool FILL>
 __global__ void k_list1_warp(TV tv, int nboxes, int* __restrict__ cnt, const int* __restrict__ ptr,
-                             int* __restrict__ out) {
+                             int* __restrict__ out, int* __restrict__ trg) {
   constexpr int MC = 1 << DIM;
   const int lane = threadIdx.x & 31;
   const int nw = (gridDim.x * blockDim.x) >> 5;
@@ -179,7 +179,10 @@ __global__ void k_list1_warp(TV tv, int nboxes, int* __restrict__ cnt, const int
     int n = 0;
     auto emit = [&](bool keep, int S) {
       const unsigned m = __ballot_sync(0xffffffffu, keep);
-      if (FILL && keep) out[base + n + __popc(m & lt)] = S;
+      if (FILL && keep) {
+        out[base + n + __popc(m & lt)] = S;
+        trg[base + n + __popc(m & lt)] = T;
+      }
       n += __popc(m);
     };
     const int l = tv.level[T];
@@ -234,11 +237,12 @@ __global__ void k_list1_warp(TV tv, int nboxes, int* __restrict__ cnt, const int
 }
 
 template <bool FILL>
-void launch_list1(const TV& tv, int nb, int* cnt, const int* ptr, int* out, cudaStream_t s) {
+void launch_list1(const TV& tv, int nb, int* cnt, const int* ptr, int* out, int* trg,
+                  cudaStream_t s) {
   const int grid = grid_for((long long)nb * 32, 256);
-  if (tv.dim == 1) k_list1_warp<1, FILL><<<grid, 256, 0, s>>>(tv, nb, cnt, ptr, out);
-  else if (tv.dim == 2) k_list1_warp<2, FILL><<<grid, 256, 0, s>>>(tv, nb, cnt, ptr, out);
-  else k_list1_warp<3, FILL><<<grid, 256, 0, s>>>(tv, nb, cnt, ptr, out);
+  if (tv.dim == 1) k_list1_warp<1, FILL><<<grid, 256, 0, s>>>(tv, nb, cnt, ptr, out, trg);
+  else if (tv.dim == 2) k_list1_warp<2, FILL><<<grid, 256, 0, s>>>(tv, nb, cnt, ptr, out, trg);
+  else k_list1_warp<3, FILL><<<grid, 256, 0, s>>>(tv, nb, cnt, ptr, out, trg);
   FGT_LAUNCH_CHECK();
 }
 
@@ -349,7 +353,7 @@ void build_lists(const Tree& t, int npwlevel, int iperiod0, int nlevend, bool do
   // before the one read-back of all three totals
   L.l1_ptr.alloc(nb + 1, s);
   DBuf<int> cnt1(nb, s);
-  launch_list1<false>(tv, nb, cnt1, nullptr, nullptr, s);
+  launch_list1<false>(tv, nb, cnt1, nullptr, nullptr, nullptr, s);
   exclusive_scan_i32(cnt1, L.l1_ptr, nb, L.l1_ptr.get() + nb, s);
   L.n_form = L.n_eval = L.n_trans = 0;
   const int lo = do_pw ? t.lev_start[t.ncutoff] : 0;
@@ -377,7 +381,8 @@ void build_lists(const Tree& t, int npwlevel, int iperiod0, int nlevend, bool do
     L.n_eval = h[2];
   }
   L.l1_src.alloc(std::max(L.n_l1, 1), s);
-  launch_list1<true>(tv, nb, nullptr, L.l1_ptr, L.l1_src, s);
+  L.l1_trg.alloc(std::max(L.n_l1, 1), s);
+  launch_list1<true>(tv, nb, nullptr, L.l1_ptr, L.l1_src, L.l1_trg, s);
   if (!do_pw) return;
   L.form_box.alloc(std::max(L.n_form, 1), s);
   L.eval_box.alloc(std::max(L.n_eval, 1), s);

@@ -16,6 +16,7 @@ struct Lists {
   DBuf<int> trans_w;     // shift-table index 0..3^dim-1
   // direct part: CSR over all boxes (targets), sources are box ids
   DBuf<int> l1_ptr, l1_src;
+  DBuf<int> l1_trg;  // target box of every list entry
   int n_l1 = 0;
 };
 

@@ -231,31 +231,37 @@ __global__ void k_scan_apply(const int* in, int* out, int n, const int* __restri
 
 // ---------------------------------------------------------------- radix sort
 constexpr int RS_THREADS = 256;
-constexpr int RS_ITEMS = 16;
-constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
+// Items per thread (template RSI): 16, and 4 up to 2^17 items, where tiles of
+// 4096 leave most SMs without a block (N = 1e5: 25 blocks, 29 us a pass).
 constexpr int RS_WARPS = RS_THREADS / 32;
 
-template <typename K>
+template <typename K, int RSI>
 __global__ void __launch_bounds__(RS_THREADS) k_radix_hist(const K* __restrict__ keys, int n,
                                                            int shift, int* __restrict__ hist,
                                                            int nblocks) {
   __shared__ int h[256];
   h[threadIdx.x] = 0;
   __syncthreads();
-  int base = blockIdx.x * RS_TILE;
-  for (int r = 0; r < RS_ITEMS; r++) {
+  int base = blockIdx.x * RS_THREADS * RSI;
+  K k[RSI];
+#pragma unroll
+  for (int r = 0; r < RSI; r++) {
     int i = base + r * RS_THREADS + threadIdx.x;
-    if (i < n) atomicAdd(&h[(int)((keys[i] >> shift) & K(255))], 1);
+    k[r] = i < n ? keys[i] : K(0);
   }
+#pragma unroll
+  for (int r = 0; r < RSI; r++)
+    if (base + r * RS_THREADS + (int)threadIdx.x < n)
+      atomicAdd(&h[(int)((k[r] >> shift) & K(255))], 1);
   __syncthreads();
   hist[threadIdx.x * nblocks + blockIdx.x] = h[threadIdx.x];
 }
 
 // Global start of this block's items of digit threadIdx.x.  offs: the scanned
 // counts, or (raw) the counts themselves, [digit][block]: with few blocks
-// every block sums them itself, which saves the scan's launches (up to 64
-// blocks, 2^18 items: 64 KB read from L2 per block).
-constexpr int RS_RAW = 64;
+// every block sums them itself, which saves the scan's launches (up to 128
+// blocks: 128 KB read from L2 per block).
+constexpr int RS_RAW = 128;
 __device__ __forceinline__ int radix_start(const int* __restrict__ offs, int nblocks, int raw) {
   if (!raw) return offs[threadIdx.x * nblocks + blockIdx.x];
   __shared__ int ws[RS_WARPS];
@@ -280,7 +286,7 @@ __device__ __forceinline__ int radix_start(const int* __restrict__ offs, int nbl
   return r;
 }
 
-template <typename K>
+template <typename K, int RSI>
 __global__ void __launch_bounds__(RS_THREADS)
     k_radix_scatter(const K* __restrict__ kin, const uint32_t* __restrict__ vin,
                     K* __restrict__ kout, uint32_t* __restrict__ vout, int n, int shift,
@@ -290,9 +296,9 @@ __global__ void __launch_bounds__(RS_THREADS)
   int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   base[tid] = radix_start(offs, nblocks, raw);
   unsigned lt = (1u << lane) - 1u;
-  int tbase = blockIdx.x * RS_TILE;
+  int tbase = blockIdx.x * RS_THREADS * RSI;
   __syncthreads();
-  for (int r = 0; r < RS_ITEMS; r++) {
+  for (int r = 0; r < RSI; r++) {
     int i = tbase + r * RS_THREADS + tid;
     bool valid = i < n;
     K k = valid ? kin[i] : K(0);
@@ -332,10 +338,12 @@ __global__ void __launch_bounds__(RS_THREADS)
 // written out by consecutive threads, so each digit's run of the tile goes
 // to consecutive global positions (whole sectors) instead of one scattered
 // 4-byte store per item.  Same output as k_radix_scatter.
+template <int RSI>
 __global__ void __launch_bounds__(RS_THREADS)
     k_radix_scatter_tile(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
                          uint32_t* __restrict__ kout, uint32_t* __restrict__ vout, int n,
                          int shift, const int* __restrict__ offs, int nblocks, int raw) {
+  constexpr int RS_TILE = RS_THREADS * RSI;
   __shared__ uint32_t sk[RS_TILE];
   __shared__ uint32_t sv[RS_TILE];
   __shared__ int run[256];    // running count per digit, then the tile's digit start
@@ -348,10 +356,10 @@ __global__ void __launch_bounds__(RS_THREADS)
   const int tn = min(RS_TILE, n - tbase);
   run[tid] = 0;
   gbase[tid] = radix_start(offs, nblocks, raw);
-  uint32_t key[RS_ITEMS], val[RS_ITEMS];
-  int rk[RS_ITEMS];
+  uint32_t key[RSI], val[RSI];
+  int rk[RSI];
 #pragma unroll
-  for (int r = 0; r < RS_ITEMS; r++) {
+  for (int r = 0; r < RSI; r++) {
     const int i = tbase + r * RS_THREADS + tid;
     const bool valid = i < n;
     key[r] = valid ? kin[i] : 0u;
@@ -360,7 +368,7 @@ __global__ void __launch_bounds__(RS_THREADS)
   __syncthreads();
   // stable rank of every item among the tile's items of its digit
 #pragma unroll
-  for (int r = 0; r < RS_ITEMS; r++) {
+  for (int r = 0; r < RSI; r++) {
     const bool valid = tbase + r * RS_THREADS + tid < n;
     const int d = valid ? (int)((key[r] >> shift) & 255u) : 256;
     const unsigned peers = __match_any_sync(0xffffffffu, d);
@@ -402,7 +410,7 @@ __global__ void __launch_bounds__(RS_THREADS)
   }
   __syncthreads();
 #pragma unroll
-  for (int r = 0; r < RS_ITEMS; r++) {
+  for (int r = 0; r < RSI; r++) {
     if (tbase + r * RS_THREADS + tid < n) {
       const int d = (int)((key[r] >> shift) & 255u);
       const int slot = run[d] + rk[r];
@@ -458,24 +466,23 @@ void exclusive_scan_i32(const int* in, int* out, int n, int* total, cudaStream_t
 }
 
 namespace {
-template <typename K>
-void radix_sort_t(K* keys, uint32_t* vals, K* ktmp, uint32_t* vtmp, int n, int bits,
+template <typename K, int RSI>
+void radix_passes(K* keys, uint32_t* vals, K* ktmp, uint32_t* vtmp, int n, int bits,
                   cudaStream_t s) {
-  if (n <= 1 || bits <= 0) return;
-  int nb = ceil_div(n, RS_TILE);
+  const int nb = ceil_div(n, RS_THREADS * RSI);
   DBuf<int> hist((size_t)256 * nb, s);
   K *ka = keys, *kb = ktmp;
   uint32_t *va = vals, *vb = vtmp;
   int passes = 0;
+  const int raw = nb <= RS_RAW ? 1 : 0;
   for (int shift = 0; shift < bits; shift += 8) {
-    k_radix_hist<K><<<nb, RS_THREADS, 0, s>>>(ka, n, shift, hist, nb);
+    k_radix_hist<K, RSI><<<nb, RS_THREADS, 0, s>>>(ka, n, shift, hist, nb);
     FGT_LAUNCH_CHECK();
-    const int raw = nb <= RS_RAW ? 1 : 0;
     if (!raw) exclusive_scan_i32(hist, hist, 256 * nb, nullptr, s);
     if constexpr (sizeof(K) == 4)
-      k_radix_scatter_tile<<<nb, RS_THREADS, 0, s>>>(ka, va, kb, vb, n, shift, hist, nb, raw);
+      k_radix_scatter_tile<RSI><<<nb, RS_THREADS, 0, s>>>(ka, va, kb, vb, n, shift, hist, nb, raw);
     else
-      k_radix_scatter<K><<<nb, RS_THREADS, 0, s>>>(ka, va, kb, vb, n, shift, hist, nb, raw);
+      k_radix_scatter<K, RSI><<<nb, RS_THREADS, 0, s>>>(ka, va, kb, vb, n, shift, hist, nb, raw);
     FGT_LAUNCH_CHECK();
     std::swap(ka, kb);
     std::swap(va, vb);
@@ -485,6 +492,13 @@ void radix_sort_t(K* keys, uint32_t* vals, K* ktmp, uint32_t* vtmp, int n, int b
     FGT_CUDA(cudaMemcpyAsync(keys, ka, sizeof(K) * n, cudaMemcpyDeviceToDevice, s));
     if (vals) FGT_CUDA(cudaMemcpyAsync(vals, va, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s));
   }
+}
+template <typename K>
+void radix_sort_t(K* keys, uint32_t* vals, K* ktmp, uint32_t* vtmp, int n, int bits,
+                  cudaStream_t s) {
+  if (n <= 1 || bits <= 0) return;
+  if (n <= (1 << 17)) radix_passes<K, 4>(keys, vals, ktmp, vtmp, n, bits, s);
+  else radix_passes<K, 16>(keys, vals, ktmp, vtmp, n, bits, s);
 }
 }  // namespace
 

@@ -18,39 +18,63 @@ struct KeyParams {
   double bsh[64];  // bsh[l] = boxsize(l+1)/2: child-centre offset below level l
 };
 
+// Bounding box of both point sets: block partials [block][lo, hi][DIM], the
+// last block to finish (ticket, zero at launch) reduces them into out[lo, hi].
 template <int DIM>
-__global__ void k_bbox(const double* __restrict__ x, int n, double* __restrict__ part) {
+__global__ void __launch_bounds__(256)
+    k_bbox(const double* __restrict__ xs, int ns, const double* __restrict__ xt, int nt,
+           double* __restrict__ part, unsigned* __restrict__ ticket, double* __restrict__ out) {
   double lo[DIM], hi[DIM];
 #pragma unroll
   for (int k = 0; k < DIM; k++) { lo[k] = INFINITY; hi[k] = -INFINITY; }
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+  const long long n = (long long)ns + nt;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (long long)gridDim.x * blockDim.x) {
+    const double* x = i < ns ? xs + (size_t)i * DIM : xt + (size_t)(i - ns) * DIM;
 #pragma unroll
     for (int k = 0; k < DIM; k++) {
-      double v = x[(size_t)i * DIM + k];
-      lo[k] = fmin(lo[k], v);
-      hi[k] = fmax(hi[k], v);
+      lo[k] = fmin(lo[k], x[k]);
+      hi[k] = fmax(hi[k], x[k]);
     }
-  __shared__ double slo[DIM][32], shi[DIM][32];
-  int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-  for (int k = 0; k < DIM; k++) {
-    double a = lo[k], b = hi[k];
-    for (int o = 16; o; o >>= 1) {
-      a = fmin(a, __shfl_xor_sync(0xffffffffu, a, o));
-      b = fmax(b, __shfl_xor_sync(0xffffffffu, b, o));
-    }
-    if (lane == 0) { slo[k][w] = a; shi[k][w] = b; }
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
+  __shared__ double slo[DIM][8], shi[DIM][8];
+  __shared__ bool last;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  auto reduce = [&](double* o) {
 #pragma unroll
     for (int k = 0; k < DIM; k++) {
+      double a = lo[k], b = hi[k];
+      for (int q = 16; q; q >>= 1) {
+        a = fmin(a, __shfl_xor_sync(0xffffffffu, a, q));
+        b = fmax(b, __shfl_xor_sync(0xffffffffu, b, q));
+      }
+      if (lane == 0) { slo[k][w] = a; shi[k][w] = b; }
+    }
+    __syncthreads();
+    if (threadIdx.x < DIM) {
+      const int k = threadIdx.x;
       double a = INFINITY, b = -INFINITY;
-      for (int j = 0; j < (int)(blockDim.x >> 5); j++) { a = fmin(a, slo[k][j]); b = fmax(b, shi[k][j]); }
-      part[(size_t)blockIdx.x * 2 * DIM + k] = a;
-      part[(size_t)blockIdx.x * 2 * DIM + DIM + k] = b;
+      for (int q = 0; q < 8; q++) { a = fmin(a, slo[k][q]); b = fmax(b, shi[k][q]); }
+      o[k] = a;
+      o[DIM + k] = b;
     }
-  }
+  };
+  reduce(part + (size_t)blockIdx.x * 2 * DIM);
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+#pragma unroll
+  for (int k = 0; k < DIM; k++) { lo[k] = INFINITY; hi[k] = -INFINITY; }
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x)
+#pragma unroll
+    for (int k = 0; k < DIM; k++) {
+      lo[k] = fmin(lo[k], __ldcg(part + (size_t)b * 2 * DIM + k));
+      hi[k] = fmax(hi[k], __ldcg(part + (size_t)b * 2 * DIM + DIM + k));
+    }
+  reduce(out);
 }
 
 // Full path key of every point (D levels).  The centre recursion
@@ -87,13 +111,6 @@ void launch_point_keys(int dim, const double* x, int n, const KeyParams& p, uint
   else k_point_keys<3><<<grid_for(n, 256), 256, 0, s>>>(x, n, p, keys);
   FGT_LAUNCH_CHECK();
 }
-void launch_bbox(int dim, const double* x, int n, int gb, double* part, cudaStream_t s) {
-  if (dim == 1) k_bbox<1><<<gb, 256, 0, s>>>(x, n, part);
-  else if (dim == 2) k_bbox<2><<<gb, 256, 0, s>>>(x, n, part);
-  else k_bbox<3><<<gb, 256, 0, s>>>(x, n, part);
-  FGT_LAUNCH_CHECK();
-}
-
 // Source count of each box of level l from the sorted full keys.
 __global__ void k_box_counts(const uint64_t* __restrict__ bk, int nb, int shift,
                              const uint64_t* __restrict__ sk, int ns, int* __restrict__ cnt) {
@@ -287,21 +304,23 @@ void tree_setup_scalars(int dim, double delta, double eps, int iperiod, const do
                         int ns, const double* d_trg, int nt, int* levcut, double* bs0,
                         double* cen0, cudaStream_t s) {
   if (iperiod != 1) {
-    int gb = 4 * kSMs;
-    DBuf<double> part((size_t)2 * gb * 2 * dim, s);
-    launch_bbox(dim, d_src, ns, gb, part.get(), s);
-    launch_bbox(dim, d_trg, nt, gb, part.get() + (size_t)gb * 2 * dim, s);
-    std::vector<double> h((size_t)2 * gb * 2 * dim);
-    FGT_CUDA(cudaMemcpyAsync(h.data(), part.get(), sizeof(double) * h.size(),
-                             cudaMemcpyDeviceToHost, s));
-    FGT_CUDA(cudaStreamSynchronize(s));
+    const long long n = (long long)ns + nt;
+    const int gb = grid_for(n, 256, 4);
+    DBuf<double> part((size_t)(gb + 1) * 2 * dim, s);
+    DBuf<unsigned> ticket(1, s);
+    ticket.zero();
+    double* out = part.get() + (size_t)gb * 2 * dim;
+    if (dim == 1) k_bbox<1><<<gb, 256, 0, s>>>(d_src, ns, d_trg, nt, part, ticket, out);
+    else if (dim == 2) k_bbox<2><<<gb, 256, 0, s>>>(d_src, ns, d_trg, nt, part, ticket, out);
+    else k_bbox<3><<<gb, 256, 0, s>>>(d_src, ns, d_trg, nt, part, ticket, out);
+    FGT_LAUNCH_CHECK();
+    double h[2 * FGT_MAXDIM];
+    fetch_span(reinterpret_cast<const int*>(out), 4 * dim, reinterpret_cast<int*>(h), s);
     double lo[FGT_MAXDIM], hi[FGT_MAXDIM];
-    for (int k = 0; k < dim; k++) { lo[k] = INFINITY; hi[k] = -INFINITY; }
-    for (int b = 0; b < 2 * gb; b++)
-      for (int k = 0; k < dim; k++) {
-        lo[k] = std::min(lo[k], h[(size_t)b * 2 * dim + k]);
-        hi[k] = std::max(hi[k], h[(size_t)b * 2 * dim + dim + k]);
-      }
+    for (int k = 0; k < dim; k++) {
+      lo[k] = h[k];
+      hi[k] = h[dim + k];
+    }
     // pts_tree_nd.f:1390-1398
     *bs0 = hi[0] - lo[0];
     for (int k = 1; k < dim; k++)
@@ -393,38 +412,52 @@ __global__ void __launch_bounds__(256)
 
 // Counts and non-leaf flags of levels lhi .. lhi-q from the counts of level
 // lhi: one block per cell of level lhi-q sums its subtree in shared memory.
-constexpr int PYR_CELLS = 4096;
-__global__ void __launch_bounds__(256)
+constexpr int PYR_CELLS = 4096, PYR_T = 512;
+__global__ void __launch_bounds__(PYR_T)
     k_pyramid(CellLevels cl, int lhi, int q, int ndiv, int* __restrict__ cnt,
               unsigned char* __restrict__ flag) {
   __shared__ int sc[PYR_CELLS];
   int n = 1 << (cl.dim * q);
   {
     const long long o = cl.off(lhi) + (long long)blockIdx.x * n;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      const int c = cnt[o + i];
-      sc[i] = c;
-      flag[o + i] = c > ndiv ? 1 : 0;
+    int v[PYR_CELLS / PYR_T];
+#pragma unroll
+    for (int k = 0; k < PYR_CELLS / PYR_T; k++) {
+      const int i = threadIdx.x + k * PYR_T;
+      v[k] = i < n ? cnt[o + i] : 0;
+    }
+#pragma unroll
+    for (int k = 0; k < PYR_CELLS / PYR_T; k++) {
+      const int i = threadIdx.x + k * PYR_T;
+      if (i < n) {
+        sc[i] = v[k];
+        flag[o + i] = v[k] > ndiv ? 1 : 0;
+      }
     }
   }
   __syncthreads();
   const int mc = 1 << cl.dim;
   for (int l = lhi - 1; l >= lhi - q; l--) {
     const int m = n >> cl.dim;
-    int v[PYR_CELLS / 2 / 256];
-    int k = 0;
-    for (int i = threadIdx.x; i < m; i += blockDim.x, k++) {
+    int v[PYR_CELLS / 2 / PYR_T];
+#pragma unroll
+    for (int k = 0; k < PYR_CELLS / 2 / PYR_T; k++) {
+      const int i = threadIdx.x + k * PYR_T;
       int a = 0;
-      for (int j = 0; j < mc; j++) a += sc[i * mc + j];
+      if (i < m)
+        for (int j = 0; j < mc; j++) a += sc[i * mc + j];
       v[k] = a;
     }
     __syncthreads();
     const long long o = cl.off(l) + (long long)blockIdx.x * m;
-    k = 0;
-    for (int i = threadIdx.x; i < m; i += blockDim.x, k++) {
-      sc[i] = v[k];
-      flag[o + i] = v[k] > ndiv ? 1 : 0;
-      if (l == lhi - q) cnt[o + i] = v[k];
+#pragma unroll
+    for (int k = 0; k < PYR_CELLS / 2 / PYR_T; k++) {
+      const int i = threadIdx.x + k * PYR_T;
+      if (i < m) {
+        sc[i] = v[k];
+        flag[o + i] = v[k] > ndiv ? 1 : 0;
+        if (l == lhi - q) cnt[o + i] = v[k];
+      }
     }
     __syncthreads();
     n = m;
@@ -435,22 +468,22 @@ __global__ void __launch_bounds__(256)
 // cell whose closure touches a non-leaf cell of level l becomes non-leaf.
 __device__ __forceinline__ void touch_parents(const CellLevels& cl, int l, uint32_t cell,
                                               unsigned char* flag) {
+  // coordinate k of a key is its bits k, k + dim, ..: neighbours by adding
+  // and subtracting inside that bit field
   const int dim = cl.dim, mc = 1 << dim;
-  uint32_t c[FGT_MAXDIM];
-  key_to_coords(cell, l, dim, c);
-  const uint32_t lim = 1u << (l - 1);
+  const uint32_t par = cell >> dim, all = (uint32_t)(cl.cells(l - 1) - 1);
+  const uint32_t field = (dim == 1 ? 0xffffffffu : (dim == 2 ? 0x55555555u : 0x49249249u));
   const long long o = cl.off(l - 1);
+  uint32_t nb[FGT_MAXDIM];  // the other touching position of the coordinate, or its own
+  for (int k = 0; k < dim; k++) {
+    const uint32_t m = (field << k) & all, x = par & m;
+    if ((cell >> k) & 1u) nb[k] = x == m ? x : (((x | ~m) + (1u << k)) & m);
+    else nb[k] = x == 0 ? x : ((x - (1u << k)) & m);
+  }
   for (int j = 0; j < mc; j++) {
-    uint32_t q[FGT_MAXDIM];
-    for (int k = 0; k < dim; k++) {
-      const uint32_t m = c[k] >> 1;
-      q[k] = m;
-      if ((j >> k) & 1) {
-        const long long t = (c[k] & 1) ? (long long)m + 1 : (long long)m - 1;
-        if (t >= 0 && t < (long long)lim) q[k] = (uint32_t)t;
-      }
-    }
-    flag[o + (long long)coords_to_key(q, l - 1, dim)] = 1;
+    uint32_t q = 0;
+    for (int k = 0; k < dim; k++) q |= ((j >> k) & 1) ? nb[k] : (par & (field << k) & all);
+    flag[o + q] = 1;
   }
 }
 __global__ void k_restrict(CellLevels cl, int l, unsigned char* __restrict__ flag) {
@@ -471,10 +504,12 @@ __global__ void __launch_bounds__(1024)
   }
 }
 
-// Exclusive scans over cells in two launches: block sums of 4096 cells, then
-// every block adds the sums before it and writes its cells.  OP gives a
-// cell's value and takes its exclusive prefix.
-constexpr int CS_T = 256, CS_I = 16, CS_TILE = CS_T * CS_I;
+// Exclusive scans over cells in two launches: block sums, then every block
+// adds the sums before it and writes its cells.  OP gives a cell's value
+// (value() from the tables, stored() what the first launch kept of it) and
+// takes its exclusive prefix.  CI cells per thread: 4, to have many blocks in
+// flight on small tables, 16 where the sums of that many blocks would cost.
+constexpr int CS_T = 256;
 __device__ __forceinline__ int block_sum(int v, int* ws) {
 #pragma unroll
   for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -486,27 +521,28 @@ __device__ __forceinline__ int block_sum(int v, int* ws) {
   __syncthreads();
   return r;
 }
-template <class OP>
+template <int CI, class OP>
 __global__ void __launch_bounds__(CS_T) k_cells_sum(OP op, long long n, int* __restrict__ part) {
   __shared__ int ws[CS_T / 32];
-  const long long b = (long long)blockIdx.x * CS_TILE + threadIdx.x * CS_I;
+  const long long b = (long long)blockIdx.x * CS_T * CI + threadIdx.x;
   int v = 0;
-  for (int j = 0; j < CS_I; j++)
-    if (b + j < n) v += op.value(b + j);
+#pragma unroll
+  for (int j = 0; j < CI; j++)
+    if (b + j * CS_T < n) v += op.value(b + j * CS_T);
   v = block_sum(v, ws);
   if (threadIdx.x == 0) part[blockIdx.x] = v;
 }
-template <class OP>
+template <int CI, class OP>
 __global__ void __launch_bounds__(CS_T) k_cells_scan(OP op, long long n, const int* __restrict__ part) {
   __shared__ int ws[CS_T / 32];
   int before = 0;
   for (int i = threadIdx.x; i < (int)blockIdx.x; i += CS_T) before += part[i];
   before = block_sum(before, ws);
-  const long long b = (long long)blockIdx.x * CS_TILE + threadIdx.x * CS_I;
-  int v[CS_I], s = 0;
+  const long long b = (long long)blockIdx.x * CS_T * CI + threadIdx.x * CI;
+  int v[CI], s = 0;
 #pragma unroll
-  for (int j = 0; j < CS_I; j++) {
-    v[j] = b + j < n ? op.value(b + j) : 0;
+  for (int j = 0; j < CI; j++) {
+    v[j] = b + j < n ? op.stored(b + j) : 0;
     s += v[j];
   }
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -522,7 +558,7 @@ __global__ void __launch_bounds__(CS_T) k_cells_scan(OP op, long long n, const i
 #pragma unroll
   for (int k = 0; k < CS_T / 32; k++) ex += k < w ? ws[k] : 0;
 #pragma unroll
-  for (int j = 0; j < CS_I; j++) {
+  for (int j = 0; j < CI; j++) {
     if (b + j < n) op.put(b + j, ex, v[j]);
     ex += v[j];
     if (b + j == n - 1) op.total(ex);
@@ -535,10 +571,15 @@ struct RankOp {
   const unsigned char* flag;
   int *rank, *lev;  // lev: D+1 entries, the last is the total
   __device__ int value(long long i) const { return flag[i]; }
+  __device__ int stored(long long i) const { return flag[i]; }
   __device__ void put(long long i, int ex, int) const {
     rank[i] = ex;
-    for (int l = 0; l < cl.D; l++)
-      if (i == cl.off(l)) lev[l] = ex;
+    // starts of levels: i = (2^(dim l) - 1) / (2^dim - 1)
+    const unsigned long long c = (unsigned long long)i * ((1 << cl.dim) - 1) + 1;
+    if ((c & (c - 1)) == 0) {
+      const int b = 63 - __clzll((long long)c);
+      if (b % cl.dim == 0 && b / cl.dim < cl.D) lev[b / cl.dim] = ex;
+    }
   }
   __device__ void total(int t) const { lev[cl.D] = t; }
 };
@@ -551,11 +592,17 @@ struct LeafOp {
   uint32_t* table;  // flagged: base | 2^31, else the ordinal of the cell's leaf
   __device__ int value(long long i) const {
     const int L = cl.D - 1;
-    if (flag[cl.off(L) + i]) return 1 << cl.dim;
-    int l = 0;  // level of the leaf that holds the cell
-    while (l < L && flag[cl.off(l) + (i >> (cl.dim * (L - l)))]) l++;
-    return (i & ((1ll << (cl.dim * (L - l))) - 1)) == 0 ? 1 : 0;
+    // a flag implies those above it: the level of the cell's leaf is the
+    // number of flags on its path (independent loads)
+    int l = 0;
+    for (int k = 0; k < L; k++) l += flag[cl.off(k) + (i >> (cl.dim * (L - k)))];
+    const int v = flag[cl.off(L) + i]
+                      ? 1 << cl.dim
+                      : ((i & ((1ll << (cl.dim * (L - l))) - 1)) == 0 ? 1 : 0);
+    base[i] = v;
+    return v;
   }
+  __device__ int stored(long long i) const { return base[i]; }
   __device__ void put(long long i, int ex, int v) const {
     base[i] = ex;
     table[i] = v > 1 ? ((uint32_t)ex | 0x80000000u) : (uint32_t)(ex + v - 1);
@@ -725,14 +772,14 @@ void tree_build_dense(Tree& t, const KeyParams& kp, const double* d_src, const d
   // 2. refinement on source counts (pts_tree_build, pts_tree_nd.f:520-590)
   for (int lhi = D - 1;;) {
     const int q = std::min(lhi, 12 / dim);
-    k_pyramid<<<(unsigned)cl.cells(lhi - q), 256, 0, s>>>(cl, lhi, q, t.ndiv, cnt, flag);
+    k_pyramid<<<(unsigned)cl.cells(lhi - q), PYR_T, 0, s>>>(cl, lhi, q, t.ndiv, cnt, flag);
     FGT_LAUNCH_CHECK();
     lhi -= q;
     if (lhi == 0) break;
   }
   // 3. level restriction (minimal 2:1 balanced refinement)
   int l = D - 1;
-  for (; l >= 2 && cl.cells(l) > 16384; l--) {
+  for (; l >= 2 && cl.cells(l) > 1024; l--) {
     k_restrict<<<grid_for(cl.cells(l), 256), 256, 0, s>>>(cl, l, flag);
     FGT_LAUNCH_CHECK();
   }
@@ -742,12 +789,17 @@ void tree_build_dense(Tree& t, const KeyParams& kp, const double* d_src, const d
   }
   // 4. box numbers and leaf ordinals
   auto scan = [&](const auto& op, long long n) {
-    const int nb = ceil_div(n, CS_TILE);
-    DBuf<int> part(nb, s);
-    k_cells_sum<<<nb, CS_T, 0, s>>>(op, n, part.get());
-    FGT_LAUNCH_CHECK();
-    k_cells_scan<<<nb, CS_T, 0, s>>>(op, n, part.get());
-    FGT_LAUNCH_CHECK();
+    auto go = [&](auto cells) {
+      constexpr int CI = decltype(cells)::value;
+      const int nb = ceil_div(n, CS_T * CI);
+      DBuf<int> part(nb, s);
+      k_cells_sum<CI><<<nb, CS_T, 0, s>>>(op, n, part.get());
+      FGT_LAUNCH_CHECK();
+      k_cells_scan<CI><<<nb, CS_T, 0, s>>>(op, n, part.get());
+      FGT_LAUNCH_CHECK();
+    };
+    if (n <= (1ll << 20)) go(std::integral_constant<int, 4>{});
+    else go(std::integral_constant<int, 16>{});
   };
   scan(RankOp{cl, flag, rank, lev}, T);
   scan(LeafOp{cl, flag, base, table}, C1);

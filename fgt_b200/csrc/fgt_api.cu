@@ -350,14 +350,14 @@ struct Setup {
   Lists L;
   DBuf<double> soff, toff;
   DBuf<uint32_t> inv_s, inv_t;
-  // packed list-1 sources of the FP32 charge path: record count (-1: not
+  // packed list-1 sources of the charge path: record count (-1: not
   // built) and the positions of every list entry's records
   long long near_total = -1;
   DBuf<int> near_pos;
   int launches = 0;
 };
 
-// Records of the packed list-1 sources are 64 bytes; above this count (16 GiB,
+// Records of the packed list-1 sources are 64 bytes (FP64: 32); above this count (16 GiB,
 // and at most an eighth of the device's memory) the near field walks the
 // list instead.  The cap depends only on the device, so repeated calls take
 // the same path and reuse the same workspace.  FGT_NEAR_PACK_MAX (a record
@@ -408,8 +408,8 @@ DirectGeom direct_geom(const Setup& u) {
   return g;
 }
 
-// near_lists: build the positions of the packed list-1 sources (FP32, one
-// density; used by executions with charges only and pgh <= 2).
+// near_lists: build the positions of the packed list-1 sources (one density;
+// used by executions with charges only and pgh <= 2).
 void setup_geometry(Setup& u, const Call& c, double* bs0_io, double* cen0_io, const fgt_opts& o,
                     bool near_lists, cudaStream_t s, Timer& tm) {
   const int dim = c.dim;
@@ -604,15 +604,13 @@ void execute(const Setup& u, const Call& c, const fgt_opts& o, fgt_stats* st, cu
   double pairs = 0;
   NearPacked packed;
   DBuf<float4> near_rec;
-  if constexpr (sizeof(T) == 4) {
-    if (u.near_total > 0 && nd == 1 && c.ifcharge && !c.ifdipole && c.ifpgh <= 2 &&
-        c.ifpghtarg <= 2) {
-      near_rec.alloc((size_t)u.near_total * 4, s);
-      near_lists_fill(g, L, src, t.trg_lo, t.trg_hi, u.near_pos, near_rec, s);
-      launches++;
-      packed.pos = u.near_pos;
-      packed.rec = near_rec;
-    }
+  if (u.near_total > 0 && nd == 1 && c.ifcharge && !c.ifdipole && c.ifpgh <= 2 &&
+      c.ifpghtarg <= 2) {
+    near_rec.alloc((size_t)u.near_total * (sizeof(T) == 4 ? 4 : 2), s);
+    near_lists_fill<T>(g, L, src, t.trg_lo, t.trg_hi, u.near_pos, near_rec.get(), s);
+    launches++;
+    packed.pos = u.near_pos;
+    packed.rec = near_rec.get();
   }
   if (c.sources_done) {
     // sources first, then signal; the targets follow
@@ -749,8 +747,8 @@ template <typename T>
 void run_pfgt(const Call& c, double* bs0_io, double* cen0_io, const fgt_opts& o, fgt_stats* st,
               cudaStream_t s, Timer& tm) {
   Setup u;
-  // the packed near-field path: FP32, one density, charges only, pgh <= 2
-  const bool near = sizeof(T) == 4 && c.nd == 1 && c.ifcharge && !c.ifdipole && c.ifpgh <= 2 &&
+  // the packed near-field path: one density, charges only, pgh <= 2
+  const bool near = c.nd == 1 && c.ifcharge && !c.ifdipole && c.ifpgh <= 2 &&
                     c.ifpghtarg <= 2;
   setup_geometry(u, c, bs0_io, cen0_io, o, near, s, tm);
   fgt_opts oo = o;
@@ -1051,7 +1049,7 @@ fgt_plan* plan_create_impl(const fgt_opts* opts_in, int nd, int dim, double delt
       }
     }
     Timer tm(false, s);
-    setup_geometry(pl->u, c, bs0, cen0, o, pl->prec != FGT_PREC_FP64 && nd == 1, s, tm);
+    setup_geometry(pl->u, c, bs0, cen0, o, nd == 1, s, tm);
     FGT_CUDA(cudaStreamSynchronize(s));
   } catch (...) {
     cudaStreamSynchronize(s);

@@ -67,44 +67,138 @@ struct HessIdx<3> {  // xx, yy, zz, xy, xz, yz
   static __device__ __forceinline__ int b(int m) { return m < 3 ? m : (m == 3 ? 1 : 2); }
 };
 
-template <typename T, int DIM, int PGH, bool CHG, bool DIP, int NDC>
-__global__ void __launch_bounds__(DW * 32) k_direct(DArgs<T> a) {
+// exp(-u) for u = t ln2 / 64 >= 0 by a table of 2^(-i/64) and a polynomial in
+// the rest (table-driven exponential, Tang 1989): t = i + f, |f| <= 1/2, and
+// the fifth-order series of 2^(-f/64) is exact to 4e-17.  Valid up to the
+// exponent range; a pair beyond the cut-off is dropped whatever comes out.
+struct ExpTab {
+  double v[64];
+};
+__device__ __forceinline__ double exp_tab(const ExpTab& tab, double t) {
+  constexpr double L = 0.69314718055994530942 / 64;
+  constexpr double M = 6755399441055744.0;  // 1.5 * 2^52: the sum's low bits are rint(t)
+  const double s = t + M;
+  const int i = __double2loint(s);
+  const double f = t - (s - M);
+  double p = fma(f, -L * L * L * L * L / 120, L * L * L * L / 24);
+  p = fma(f, p, -L * L * L / 6);
+  p = fma(f, p, L * L / 2);
+  p = fma(f, p, -L);
+  p = fma(f, p, 1.0);
+  const double r = tab.v[i & 63] * p;
+  return __hiloint2double(__double2hiint(r) - ((i >> 6) << 20), __double2loint(r));
+}
+
+// FP64 near field (dipoles, hessians, several densities, or too many
+// records): one evaluation point per lane in registers.  The sources
+// of the list-1 boxes that can reach the target box are packed, across list
+// entries, into batches of 32 in shared memory and read as broadcasts.  An
+// item of at most 16, 8 or 4 points gives 2, 4 or 8 groups of lanes, each
+// with every 2nd, 4th or 8th source.  Bound by the FP64 pipe (26 instructions
+// a pair with the gradient): 2.5e9 listed pairs of config-2 clusters 6.9 ->
+// NEARMS ms against unpacked batches with the library exponential and a branch
+// on the cut-off.
+template <int DIM, int PGH, bool CHG, bool DIP, int NDC>
+__global__ void __launch_bounds__(DW * 32) k_direct(DArgs<double> a) {
   constexpr int NH = DIM * (DIM + 1) / 2;
   constexpr int NC = 1 + (PGH >= 2 ? DIM : 0) + (PGH >= 3 ? NH : 0);
-  constexpr bool SPLIT = sizeof(T) == 4;  // FP32: pair differences from hi/lo parts
-  __shared__ T sx[DW][DIM][32];
-  __shared__ T sxl[DW][SPLIT ? DIM : 1][32];
-  __shared__ T sq[DW][CHG ? NDC : 1][32];
-  __shared__ T sd[DW][DIP ? NDC : 1][32];
-  __shared__ T sn[DW][DIP ? DIM : 1][32];
+  __shared__ ExpTab tab;
+  __shared__ double sx[DW][DIM][64];
+  __shared__ double sq[DW][CHG ? NDC : 1][64];
+  __shared__ double sd[DW][DIP ? NDC : 1][64];
+  __shared__ double sn[DW][DIP ? DIM : 1][64];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x < 64) tab.v[threadIdx.x] = exp2(-(double)threadIdx.x / 64);
+  __syncthreads();
   const int ndc = min(NDC, a.nd - a.d0);
   const int n_items = *a.n_items_dev;
+  const double tscale = a.dinv * (64 * 1.4426950408889634074);
   for (int it = blockIdx.x * DW + warp; it < n_items; it += gridDim.x * DW) {
     const int tb = a.item_box[it];
-    const int p = a.item_lo[it] + lane;
-    const bool act = p < a.e_hi[tb];
-    T tx[DIM], txl[DIM];
+    const int np = min(32, a.e_hi[tb] - a.item_lo[it]);
+    const int wd = np > 16 ? 32 : (np > 8 ? 16 : (np > 4 ? 8 : 4));  // lanes of a group
+    const int nsub = 32 / wd, sub = lane / wd, q = lane & (wd - 1);
+    const int p = a.item_lo[it] + q;
+    const bool act = q < np;
+    double tx[DIM], acc[NDC][NC];
 #pragma unroll
-    for (int k = 0; k < DIM; k++) {
-      const double v = act ? a.eoff[(size_t)k * a.ne + p] : 0.0;
-      tx[k] = (T)v;
-      txl[k] = SPLIT ? (T)(v - (double)tx[k]) : T(0);
-    }
-    // T sums over one staged batch of 32 sources, FP64 sums over batches
-    T acc[NDC][NC];
-    double accd[NDC][NC];
+    for (int k = 0; k < DIM; k++) tx[k] = act ? a.eoff[(size_t)k * a.ne + p] : 0.0;
 #pragma unroll
     for (int i = 0; i < NDC; i++)
 #pragma unroll
-      for (int c = 0; c < NC; c++) {
-        acc[i][c] = T(0);
-        accd[i][c] = 0.0;
+      for (int c = 0; c < NC; c++) acc[i][c] = 0.0;
+    auto sum = [&](int cnt) {
+#pragma unroll(DIP || PGH >= 3 ? 1 : 2)
+      for (int j0 = 0; j0 < cnt; j0 += nsub) {
+        const int jj = min(j0 + sub, cnt - 1);
+        double dr[DIM], rr = 0.0;
+#pragma unroll
+        for (int k = 0; k < DIM; k++) {
+          dr[k] = tx[k] - sx[warp][k][jj];
+          rr = fma(dr[k], dr[k], rr);
+        }
+        const bool in = rr < a.dmax && j0 + sub < cnt;
+        // 60+ instructions a pair: a source out of every lane's reach is left out
+        if ((DIP || PGH >= 3) && !__any_sync(0xffffffffu, in)) continue;
+        const double e = exp_tab(tab, rr * tscale);
+        if (CHG) {
+          // gnd_directc{p,g,h}, src/pfgt/pfgt_direct.f:47-196
+#pragma unroll
+          for (int i = 0; i < NDC; i++) {
+            if (i >= ndc) break;
+            const double r = in ? e * sq[warp][i][jj] : 0.0;
+            acc[i][0] += r;
+            if (PGH >= 2) {
+              const double rg = -a.rfac * r;
+#pragma unroll
+              for (int k = 0; k < DIM; k++) acc[i][1 + k] = fma(dr[k], rg, acc[i][1 + k]);
+              if (PGH >= 3)
+#pragma unroll
+                for (int m = 0; m < NH; m++) {
+                  const int ka = HessIdx<DIM>::a(m), kb = HessIdx<DIM>::b(m);
+                  const double h = a.rfac * dr[ka] * dr[kb] - (ka == kb ? 1.0 : 0.0);
+                  acc[i][1 + DIM + m] = fma(-rg, h, acc[i][1 + DIM + m]);
+                }
+            }
+          }
+        }
+        if (DIP) {
+          // gnd_directd{p,g,h}, src/pfgt/pfgt_direct.f:204-384
+          double d[DIM], rn[DIM], rinc = 0.0;
+#pragma unroll
+          for (int k = 0; k < DIM; k++) {
+            d[k] = a.rfac * dr[k];
+            rn[k] = sn[warp][DIP ? k : 0][jj];
+            rinc = fma(d[k], rn[k], rinc);
+          }
+          double rg[DIM];
+#pragma unroll
+          for (int k = 0; k < DIM; k++) rg[k] = rn[k] * a.rfac - rinc * d[k];
+#pragma unroll
+          for (int i = 0; i < NDC; i++) {
+            if (i >= ndc) break;
+            const double r = in ? e * sd[warp][i][jj] : 0.0;
+            acc[i][0] = fma(rinc, r, acc[i][0]);
+            if (PGH >= 2)
+#pragma unroll
+              for (int k = 0; k < DIM; k++) acc[i][1 + k] = fma(rg[k], r, acc[i][1 + k]);
+            if (PGH >= 3)
+#pragma unroll
+              for (int m = 0; m < NH; m++) {
+                const int ka = HessIdx<DIM>::a(m), kb = HessIdx<DIM>::b(m);
+                const double h = (ka == kb) ? (-a.rfac * (d[ka] * rn[ka] + rinc) - rg[ka] * d[ka])
+                                            : (-a.rfac * d[ka] * rn[kb] - rg[ka] * d[kb]);
+                acc[i][1 + DIM + m] = fma(h, r, acc[i][1 + DIM + m]);
+              }
+          }
+        }
       }
+    };
     double cT[DIM];
 #pragma unroll
     for (int k = 0; k < DIM; k++) cT[k] = a.center[(size_t)tb * DIM + k];
-    const int lT = a.level[tb];
+    const double hT = 0.5 * a.bs0 * ldexp(1.0, -a.level[tb]);
+    int fill = 0;  // packed sources in the buffer
     for (int li = a.l1_ptr[tb]; li < a.l1_ptr[tb + 1]; li++) {
       const int sb = a.l1_src[li];
       if (!FGT_DCHECK(sb >= 0 && sb < a.nboxes, 401)) continue;
@@ -120,117 +214,70 @@ __global__ void __launch_bounds__(DW * 32) k_direct(DArgs<T> a) {
         }
         dc[k] = (cs + sh) - cT[k];
       }
-      if (box_beyond_cutoff<DIM>(dc, 0.5 * a.bs0 * (ldexp(1.0, -lT) + ldexp(1.0, -a.level[sb])),
-                                 a.dmax_d))
-        continue;
+      if (box_beyond_cutoff<DIM>(dc, hT + 0.5 * a.bs0 * ldexp(1.0, -a.level[sb]), a.dmax_d)) continue;
       const int s0 = a.s_lo[sb], s1 = a.s_hi[sb];
       for (int base = s0; base < s1; base += 32) {
         const int j = base + lane;
-        __syncwarp();
+        double v[DIM];
+        bool keep = false;
         if (j < s1) {
 #pragma unroll
-          for (int k = 0; k < DIM; k++) {
-            const double v = a.soff[(size_t)k * a.ns + j] + dc[k];
-            const T hi = (T)v;
-            sx[warp][k][lane] = hi;
-            if (SPLIT) sxl[warp][k][lane] = (T)(v - (double)hi);
-          }
+          for (int k = 0; k < DIM; k++) v[k] = a.soff[(size_t)k * a.ns + j] + dc[k];
+          keep = !box_beyond_cutoff<DIM>(v, hT, a.dmax_d);
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, keep);
+        if (keep) {
+          const int o = fill + __popc(m & ((1u << lane) - 1u));  // < 64
+#pragma unroll
+          for (int k = 0; k < DIM; k++) sx[warp][k][o] = v[k];
           if (CHG)
 #pragma unroll
             for (int i = 0; i < NDC; i++)
-              if (i < ndc) sq[warp][i][lane] = a.q[(size_t)(a.d0 + i) * a.ns + j];
+              if (i < ndc) sq[warp][i][o] = a.q[(size_t)(a.d0 + i) * a.ns + j];
           if (DIP) {
 #pragma unroll
             for (int i = 0; i < NDC; i++)
-              if (i < ndc) sd[warp][i][lane] = a.ds[(size_t)(a.d0 + i) * a.ns + j];
+              if (i < ndc) sd[warp][i][o] = a.ds[(size_t)(a.d0 + i) * a.ns + j];
 #pragma unroll
-            for (int k = 0; k < DIM; k++) sn[warp][k][lane] = a.rn[(size_t)k * a.ns + j];
+            for (int k = 0; k < DIM; k++) sn[warp][DIP ? k : 0][o] = a.rn[(size_t)k * a.ns + j];
           }
         }
+        fill += __popc(m);
         __syncwarp();
-        const int cnt = min(32, s1 - base);
-#pragma unroll 1
-        for (int jj = 0; jj < cnt; jj++) {
-          T dr[DIM], rr = T(0);
+        if (fill >= 32) {
+          sum(32);
+          __syncwarp();
+          fill -= 32;
+          if (lane < fill) {  // the rest to the front
 #pragma unroll
-          for (int k = 0; k < DIM; k++) {
-            dr[k] = SPLIT ? (tx[k] - sx[warp][k][jj]) + (txl[k] - sxl[warp][k][jj])
-                          : tx[k] - sx[warp][k][jj];
-            rr += dr[k] * dr[k];
-          }
-          if (!(rr < a.dmax)) continue;
-          const T e = Real<T>::expm(rr * a.dinv);
-          if (CHG) {
-            // gnd_directc{p,g,h}, src/pfgt/pfgt_direct.f:47-196
-            T dg[DIM];
+            for (int k = 0; k < DIM; k++) sx[warp][k][lane] = sx[warp][k][32 + lane];
+            if (CHG)
 #pragma unroll
-            for (int k = 0; k < DIM; k++) dg[k] = -a.rfac * dr[k];
+              for (int i = 0; i < NDC; i++) sq[warp][i][lane] = sq[warp][i][32 + lane];
+            if (DIP) {
 #pragma unroll
-            for (int i = 0; i < NDC; i++) {
-              if (i >= ndc) break;
-              const T r = e * sq[warp][i][jj];
-              acc[i][0] += r;
-              if (PGH >= 2)
+              for (int i = 0; i < NDC; i++) sd[warp][i][lane] = sd[warp][i][32 + lane];
 #pragma unroll
-                for (int k = 0; k < DIM; k++) acc[i][1 + k] += dg[k] * r;
-              if (PGH >= 3)
-#pragma unroll
-                for (int m = 0; m < NH; m++) {
-                  const int ka = HessIdx<DIM>::a(m), kb = HessIdx<DIM>::b(m);
-                  const T h = dg[ka] * dg[kb] + (ka == kb ? -a.rfac : T(0));
-                  acc[i][1 + DIM + m] += h * r;
-                }
+              for (int k = 0; k < DIM; k++) sn[warp][DIP ? k : 0][lane] = sn[warp][DIP ? k : 0][32 + lane];
             }
           }
-          if (DIP) {
-            // gnd_directd{p,g,h}, src/pfgt/pfgt_direct.f:204-384
-            T d[DIM], rn[DIM], rinc = T(0);
-#pragma unroll
-            for (int k = 0; k < DIM; k++) {
-              d[k] = a.rfac * dr[k];
-              rn[k] = sn[warp][k][jj];
-              rinc += d[k] * rn[k];
-            }
-            T rg[DIM];
-#pragma unroll
-            for (int k = 0; k < DIM; k++) rg[k] = rn[k] * a.rfac - rinc * d[k];
-#pragma unroll
-            for (int i = 0; i < NDC; i++) {
-              if (i >= ndc) break;
-              const T r = e * sd[warp][i][jj];
-              acc[i][0] += rinc * r;
-              if (PGH >= 2)
-#pragma unroll
-                for (int k = 0; k < DIM; k++) acc[i][1 + k] += rg[k] * r;
-              if (PGH >= 3)
-#pragma unroll
-                for (int m = 0; m < NH; m++) {
-                  const int ka = HessIdx<DIM>::a(m), kb = HessIdx<DIM>::b(m);
-                  T h = (ka == kb) ? (-a.rfac * (d[ka] * rn[ka] + rinc) - rg[ka] * d[ka])
-                                   : (-a.rfac * d[ka] * rn[kb] - rg[ka] * d[kb]);
-                  acc[i][1 + DIM + m] += h * r;
-                }
-            }
-          }
+          __syncwarp();
         }
-#pragma unroll
-        for (int i = 0; i < NDC; i++)
-#pragma unroll
-          for (int c = 0; c < NC; c++) {
-            accd[i][c] += (double)acc[i][c];
-            acc[i][c] = T(0);
-          }
       }
     }
-    if (act) {
+    if (fill > 0) sum(fill);
+    __syncwarp();
+    for (int o = wd; o < 32; o <<= 1)
+#pragma unroll
+      for (int i = 0; i < NDC; i++)
+#pragma unroll
+        for (int c = 0; c < NC; c++) acc[i][c] += __shfl_xor_sync(0xffffffffu, acc[i][c], o);
+    if (act && sub == 0) {
 #pragma unroll
       for (int i = 0; i < NDC; i++) {
         if (i >= ndc) break;
 #pragma unroll
-        for (int c = 0; c < NC; c++) {
-          double* o = &a.out[((size_t)c * a.nd + a.d0 + i) * a.ne + p];
-          *o += accd[i][c] + (double)acc[i][c];
-        }
+        for (int c = 0; c < NC; c++) a.out[((size_t)c * a.nd + a.d0 + i) * a.ne + p] += acc[i][c];
       }
     }
   }
@@ -561,16 +608,16 @@ struct NearArgs {
   double bs0, dmax;
   const int *l1_trg, *l1_src, *s_lo, *s_hi, *t_lo, *t_hi, *level;
   const double *center, *soff;
-  const float* q;                 // FILL: charges of density 0
+  const void* q;                  // FILL: charges of density 0 (float, or double for FP64 records)
   int* cnt;                       // COUNT: kept sources per list entry
   unsigned long long* total;      // COUNT: sum of cnt
   const int* pos;                 // FILL: first record of every list entry
-  float4* rec;                    // FILL: 4 float4 per kept source
+  void* rec;                      // FILL: 4 float4, or 2 double2 (x, y), (z, q), per kept source
 };
 
 // One warp per list entry (a box's ~27 entries one after the other left the
 // SMs to latency: uniform N = 1e5, 41 + 55 us for count and fill).
-template <int DIM, bool FILL>
+template <typename T, int DIM, bool FILL>
 __global__ void k_near_lists(NearArgs n) {
   const int lane = threadIdx.x & 31;
   const int nw = (gridDim.x * blockDim.x) >> 5;
@@ -609,18 +656,25 @@ __global__ void k_near_lists(NearArgs n) {
           }
           const unsigned m = __ballot_sync(0xffffffffu, keep);
           if (FILL && keep) {
-            float h[3] = {0.f, 0.f, 0.f}, l[3] = {0.f, 0.f, 0.f};
+            const size_t o = (size_t)(out + kept + __popc(m & ((1u << lane) - 1u)));
+            if constexpr (sizeof(T) == 4) {
+              float h[3] = {0.f, 0.f, 0.f}, l[3] = {0.f, 0.f, 0.f};
 #pragma unroll
-            for (int k = 0; k < DIM; k++) {
-              h[k] = (float)v[k];
-              l[k] = (float)(v[k] - (double)h[k]);
+              for (int k = 0; k < DIM; k++) {
+                h[k] = (float)v[k];
+                l[k] = (float)(v[k] - (double)h[k]);
+              }
+              const float qv = static_cast<const float*>(n.q)[j];
+              float4* r = static_cast<float4*>(n.rec) + 4 * o;
+              r[0] = make_float4(-h[0], -h[0], -h[1], -h[1]);
+              r[1] = make_float4(-h[2], -h[2], qv, qv);
+              r[2] = make_float4(-l[0], -l[0], -l[1], -l[1]);
+              r[3] = make_float4(-l[2], -l[2], 0.f, 0.f);
+            } else {
+              double2* r = static_cast<double2*>(n.rec) + 2 * o;
+              r[0] = make_double2(v[0], DIM > 1 ? v[DIM > 1 ? 1 : 0] : 0.0);
+              r[1] = make_double2(DIM > 2 ? v[DIM > 2 ? 2 : 0] : 0.0, static_cast<const double*>(n.q)[j]);
             }
-            const float qv = n.q[j];
-            float4* r = n.rec + 4 * (size_t)(out + kept + __popc(m & ((1u << lane) - 1u)));
-            r[0] = make_float4(-h[0], -h[0], -h[1], -h[1]);
-            r[1] = make_float4(-h[2], -h[2], qv, qv);
-            r[2] = make_float4(-l[0], -l[0], -l[1], -l[1]);
-            r[3] = make_float4(-l[2], -l[2], 0.f, 0.f);
           }
           kept += __popc(m);
         }
@@ -637,6 +691,95 @@ __global__ void k_near_lists(NearArgs n) {
       for (int w = 1; w < 8; w++) tot += sum[w];
       if (tot) atomicAdd(n.total, tot);
     }
+  }
+}
+
+// FP64 near field on packed list-1 sources (charges, one density, potential
+// or potential + gradient): one evaluation point per lane, the box's records
+// in batches of 32 through shared memory (the next batch in registers), items
+// of 32 points from a device counter.  An item of at most 16, 8 or 4 points
+// gives 2, 4 or 8 groups of lanes, each with every 2nd, 4th or 8th record.
+// Bound by the FP64 pipe (22 instructions a pair with the gradient, ~45 with
+// the library exponential).  Against the list walk with unpacked batches:
+// clusters, N = M = 2e6 (2.5e9 listed pairs, eps = 1e-9) 6.9 -> 4.1 ms plus
+// 0.2 for the records' positions, sphere, N = M = 2e6, eps = 1e-6 3.2 -> 2.3.
+template <int DIM, int PGH>
+__global__ void __launch_bounds__(DW * 32) k_direct64p(DArgs<double> a, const int* __restrict__ pos,
+                                                       const double2* __restrict__ rec,
+                                                       int* __restrict__ next) {
+  constexpr int NC = 1 + (PGH >= 2 ? DIM : 0);
+  __shared__ ExpTab tab;
+  __shared__ double2 stage[DW][2][32][2];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x < 64) tab.v[threadIdx.x] = exp2(-(double)threadIdx.x / 64);
+  __syncthreads();
+  const double tscale = a.dinv * (64 * 1.4426950408889634074);
+  const int n_items = *a.n_items_dev;
+  int it = 0;
+  if (lane == 0) it = atomicAdd(next, 1);
+  it = __shfl_sync(0xffffffffu, it, 0);
+  while (it < n_items) {
+    int nxt = 0;
+    if (lane == 0) nxt = atomicAdd(next, 1);
+    const int tb = a.item_box[it];
+    const int c0 = pos[a.l1_ptr[tb]], c1 = pos[a.l1_ptr[tb + 1]];
+    double2 r0 = make_double2(0.0, 0.0), r1 = r0;
+    if (c0 + lane < c1) {
+      r0 = rec[2 * (size_t)(c0 + lane)];
+      r1 = rec[2 * (size_t)(c0 + lane) + 1];
+    }
+    const int np = min(32, a.e_hi[tb] - a.item_lo[it]);
+    const int wd = np > 16 ? 32 : (np > 8 ? 16 : (np > 4 ? 8 : 4));  // lanes of a group
+    const int nsub = 32 / wd, sub = lane / wd, q = lane & (wd - 1);
+    const int p = a.item_lo[it] + q;
+    const bool act = q < np;
+    double tx[3] = {0.0, 0.0, 0.0}, acc[NC];
+#pragma unroll
+    for (int k = 0; k < DIM; k++) tx[k] = act ? a.eoff[(size_t)k * a.ne + p] : 0.0;
+#pragma unroll
+    for (int c = 0; c < NC; c++) acc[c] = 0.0;
+    int buf = 0;
+    for (int base = c0; base < c1; base += 32, buf ^= 1) {
+      double2(*S)[2] = stage[warp][buf];
+      S[lane][0] = r0;
+      S[lane][1] = r1;
+      if (base + 32 + lane < c1) {
+        r0 = rec[2 * (size_t)(base + 32 + lane)];
+        r1 = rec[2 * (size_t)(base + 32 + lane) + 1];
+      }
+      __syncwarp();
+      const int cnt = min(32, c1 - base);
+#pragma unroll 4
+      for (int j0 = 0; j0 < cnt; j0 += nsub) {
+        const int jj = min(j0 + sub, cnt - 1);
+        const double2 A = S[jj][0], Bq = S[jj][1];
+        const double sx[3] = {A.x, A.y, Bq.x};
+        double dr[DIM], rr = 0.0;
+#pragma unroll
+        for (int k = 0; k < DIM; k++) {
+          dr[k] = tx[k] - sx[k];
+          rr = fma(dr[k], dr[k], rr);
+        }
+        const bool in = rr < a.dmax && j0 + sub < cnt;
+        const double e = exp_tab(tab, rr * tscale);
+        // gnd_directc{p,g}, src/pfgt/pfgt_direct.f:47-140; the factor -2/delta
+        // of the gradient is applied to the sum
+        const double r = in ? e * Bq.y : 0.0;
+        acc[0] += r;
+        if (PGH >= 2)
+#pragma unroll
+          for (int k = 0; k < DIM; k++) acc[1 + k] = fma(dr[k], r, acc[1 + k]);
+      }
+    }
+    for (int o = wd; o < 32; o <<= 1)
+#pragma unroll
+      for (int c = 0; c < NC; c++) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+    if (act && sub == 0) {
+#pragma unroll
+      for (int c = 0; c < NC; c++)
+        a.out[((size_t)c * a.nd + a.d0) * a.ne + p] += c ? -a.rfac * acc[c] : acc[c];
+    }
+    it = __shfl_sync(0xffffffffu, nxt, 0);
   }
 }
 
@@ -857,7 +1000,7 @@ void launch_direct(const DArgs<T>& a, cudaStream_t s) {
   if constexpr (sizeof(T) == 4)
     k_direct32<DIM, PGH, CHG, DIP, NDC><<<grid, DW * 32, 0, s>>>(a);
   else
-    k_direct<T, DIM, PGH, CHG, DIP, NDC><<<grid, DW * 32, 0, s>>>(a);
+    k_direct<DIM, PGH, CHG, DIP, NDC><<<grid, DW * 32, 0, s>>>(a);
   FGT_LAUNCH_CHECK();
 }
 
@@ -903,12 +1046,12 @@ NearArgs near_args(const DirectGeom& g, const Lists& L, const int* s_lo, const i
   n.soff = soff;
   return n;
 }
-template <bool FILL>
+template <typename T, bool FILL>
 void launch_near_lists(int dim, const NearArgs& n, cudaStream_t s) {
   const int grid = grid_for((long long)n.n_l1 * 32, 256);
-  if (dim == 1) k_near_lists<1, FILL><<<grid, 256, 0, s>>>(n);
-  else if (dim == 2) k_near_lists<2, FILL><<<grid, 256, 0, s>>>(n);
-  else k_near_lists<3, FILL><<<grid, 256, 0, s>>>(n);
+  if (dim == 1) k_near_lists<T, 1, FILL><<<grid, 256, 0, s>>>(n);
+  else if (dim == 2) k_near_lists<T, 2, FILL><<<grid, 256, 0, s>>>(n);
+  else k_near_lists<T, 3, FILL><<<grid, 256, 0, s>>>(n);
   FGT_LAUNCH_CHECK();
 }
 }  // namespace
@@ -923,7 +1066,7 @@ long long near_lists_count(const DirectGeom& g, const Lists& L, const int* s_lo,
   tot.zero();
   n.cnt = cnt;
   n.total = tot;
-  launch_near_lists<false>(g.dim, n, s);
+  launch_near_lists<float, false>(g.dim, n, s);
   unsigned long long h = 0;
   FGT_CUDA(cudaMemcpyAsync(&h, tot.get(), sizeof(h), cudaMemcpyDeviceToHost, s));
   FGT_CUDA(cudaStreamSynchronize(s));
@@ -943,15 +1086,20 @@ int near_wait_status(cudaStream_t s) {
   return v;
 }
 
-void near_lists_fill(const DirectGeom& g, const Lists& L, const SourceSet<float>& src,
-                     const int* t_lo, const int* t_hi, const int* pos, float4* rec,
+template <typename T>
+void near_lists_fill(const DirectGeom& g, const Lists& L, const SourceSet<T>& src,
+                     const int* t_lo, const int* t_hi, const int* pos, void* rec,
                      cudaStream_t s) {
   NearArgs n = near_args(g, L, src.lo, src.hi, t_lo, t_hi, src.off, src.n);
   n.q = src.q;
   n.pos = pos;
   n.rec = rec;
-  launch_near_lists<true>(g.dim, n, s);
+  launch_near_lists<T, true>(g.dim, n, s);
 }
+template void near_lists_fill<float>(const DirectGeom&, const Lists&, const SourceSet<float>&,
+                                     const int*, const int*, const int*, void*, cudaStream_t);
+template void near_lists_fill<double>(const DirectGeom&, const Lists&, const SourceSet<double>&,
+                                      const int*, const int*, const int*, void*, cudaStream_t);
 
 namespace {
 // Blocks of k_direct32x2p resident on the device at once (the grid of the
@@ -984,7 +1132,8 @@ template <int DIM, int PGH>
 void launch_packed(const DArgs<float>& a, const NearPacked& p, int* next, cudaStream_t s) {
   t_packed_launched = true;
   const int grid = std::max(1, std::min(ceil_div(a.n_items, DW), resident_blocks_p<DIM, PGH>()));
-  k_direct32x2p<DIM, PGH><<<grid, DW * 32, 0, s>>>(a, p.pos, p.rec, next, near_stall_test());
+  k_direct32x2p<DIM, PGH><<<grid, DW * 32, 0, s>>>(a, p.pos, static_cast<const float4*>(p.rec), next,
+                                               near_stall_test());
   FGT_LAUNCH_CHECK();
 }
 }  // namespace
@@ -1047,6 +1196,22 @@ int direct_near_field(const DirectGeom& g, const Lists& L, const SourceSet<T>& s
   a.level = g.level;
   a.dmax_d = g.dmax;
   a.out = e.out;
+  if constexpr (sizeof(T) == 8) {
+    if (packed && packed->rec && chg && !dip && e.pgh <= 2 && g.nd == 1) {
+      a.d0 = 0;
+      DBuf<int> next(1, s);
+      next.zero();
+      auto go = [&](auto kern) {
+        kern<<<std::max(1, std::min(ceil_div(n_items, DW), kSMs * 8)), DW * 32, 0, s>>>(
+            a, packed->pos, static_cast<const double2*>(packed->rec), next);
+        FGT_LAUNCH_CHECK();
+      };
+      if (g.dim == 1) e.pgh == 1 ? go(k_direct64p<1, 1>) : go(k_direct64p<1, 2>);
+      else if (g.dim == 2) e.pgh == 1 ? go(k_direct64p<2, 1>) : go(k_direct64p<2, 2>);
+      else e.pgh == 1 ? go(k_direct64p<3, 1>) : go(k_direct64p<3, 2>);
+      return launches + 1;
+    }
+  }
   if constexpr (sizeof(T) == 4) {
     if (paired && packed && packed->rec) {
       a.d0 = 0;

@@ -40,7 +40,7 @@ struct DirectGeom {
 // target box, as hi/lo FP32 offsets from the target box centre and charges.
 struct NearPacked {
   const int* pos = nullptr;    // n_l1 + 1
-  const float4* rec = nullptr;
+  const void* rec = nullptr;   // 64-byte FP32 or 32-byte FP64 records
 };
 
 // Counts the packed records (geometry only: boxes, offsets, cut-off) and
@@ -52,8 +52,9 @@ long long near_lists_count(const DirectGeom& g, const Lists& L, const int* s_lo,
                            long long max_records, DBuf<int>& pos, cudaStream_t s);
 // Writes the records (charges of density 0) for positions from near_lists_count
 // with the same geometry.
-void near_lists_fill(const DirectGeom& g, const Lists& L, const SourceSet<float>& src,
-                     const int* t_lo, const int* t_hi, const int* pos, float4* rec,
+template <typename T>
+void near_lists_fill(const DirectGeom& g, const Lists& L, const SourceSet<T>& src,
+                     const int* t_lo, const int* t_hi, const int* pos, void* rec,
                      cudaStream_t s);
 
 // Status of the bounded waits of the packed near-field kernel since the last
@@ -63,7 +64,7 @@ int near_wait_status(cudaStream_t s);
 
 // Adds the list-1 interactions onto every point of `e`.  Returns the number
 // of kernel launches; *pairs receives the near-field pair count if not null.
-// With packed records (FP32, charges, one density, pgh <= 2) the near field
+// With packed records (charges, one density, pgh <= 2) the near field
 // streams them instead of walking the list.
 template <typename T>
 int direct_near_field(const DirectGeom& g, const Lists& L, const SourceSet<T>& src,

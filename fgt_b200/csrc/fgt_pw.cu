@@ -48,24 +48,14 @@ constexpr int TB = 4;           // block edge (base cells)
 constexpr int NBLK_MAX = 1024;  // blocks per box
 constexpr int PB = 8;           // points per warp batch
 constexpr int TP = 12;          // padded kernel row (TILE <= TP - 1)
-// points sorted per round: FP32 8192; FP64 2048 (its ~200 KB grid leaves
-// little shared memory)
-template <typename T>
-__host__ __device__ constexpr int fch() {
-  return sizeof(T) == 4 ? 8192 : 2048;
-}
-
-constexpr int RD = 10;  // FP64 kernel row: one tile row (TILE <= RD - 1) + a zero
+constexpr int FCH = 8192;       // points sorted per round
 
 // byte offset of the grid buffer in the tiled form kernel; every part is a
-// multiple of 16 bytes, so the kernel-row buffer is float4 aligned.  The
-// FP64 variant's row buffer holds three rows of RD doubles per warp.
+// multiple of 16 bytes, so the kernel-row buffer is float4 aligned.
 template <typename T>
 __host__ __device__ constexpr size_t tiled_offset(int G, int K) {
-  return tw_bytes16<T>(G, K) + sizeof(int) * (2 * NBLK_MAX + 32) + sizeof(int) * fch<T>() +
-         sizeof(unsigned short) * fch<T>() +
-         (sizeof(T) == 4 ? sizeof(float) * (PW_THREADS / 32) * PB * 3 * TP
-                         : sizeof(double) * (PW_THREADS / 32) * 3 * RD);
+  return tw_bytes16<T>(G, K) + sizeof(int) * (2 * NBLK_MAX + 32) + sizeof(int) * FCH +
+         sizeof(unsigned short) * FCH + sizeof(float) * (PW_THREADS / 32) * PB * 3 * TP;
 }
 
 // Exclusive scan of cnt[0..n) into off[0..n) for n <= 2 * blockDim.x;
@@ -223,116 +213,6 @@ __device__ void spread_tiled(const PWArgs<T>& a, T* B, const double* __restrict_
   __syncthreads();
 }
 
-// FP64 block-tiled spreading (3D, eps >= ~1e-6): as spread_tiled, with
-// blocks of TBD^3 base cells and a register tile of (TBD+W-1)^3 FP64 cells
-// (lane l owns the tile columns l, l+32, ... with all TILE z cells).  Per
-// point, lane t < 3 RD writes entry t % RD of the point's kernel row t / RD
-// in tile coordinates (zero outside the stencil, the x row times the
-// strength) to the warp's row buffer, and every lane reads its values as
-// broadcasts: no shuffles and no edge selects.  The flush adds every
-// non-zero tile cell with one atomic: ~TILE^3/(points per block) atomics
-// per point instead of W^3.
-template <int W, int TBD>
-__device__ void spread_tiled_d(const PWArgs<double>& a, double* B, const double* __restrict__ off,
-                               int ns, const double* __restrict__ sq,
-                               const double* __restrict__ sr, bool is_q, int c0, int n, int* cnt,
-                               int* boff, int* misc, int* tmp, unsigned short* perm,
-                               double* rows) {
-  constexpr int TILE = TBD + W - 1, NCOL = (TILE * TILE + 31) / 32;
-  static_assert(TILE <= RD - 1 && 3 * RD <= 32, "one row entry per lane, a zero at RD - 1");
-  const Geo& g = a.g;
-  const int nbd = (g.G - W + 1 + TBD - 1) / TBD, nblk = nbd * nbd * nbd;
-  for (int i = threadIdx.x; i < nblk; i += blockDim.x) cnt[i] = 0;
-  if (threadIdx.x == 0) misc[0] = 0;
-  __syncthreads();
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    int blk = 0;
-#pragma unroll
-    for (int d = 0; d < 3; d++)
-      blk = blk * nbd + base_cell<double, W>(a, off[(size_t)d * ns + c0 + i] * a.scale_d) / TBD;
-    const int r = atomicAdd(&cnt[blk], 1);
-    tmp[i] = (r << 10) | blk;
-  }
-  __syncthreads();
-  block_scan(cnt, boff, nblk, misc + 1);
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const int v = tmp[i];
-    perm[boff[v & (NBLK_MAX - 1)] + (v >> 10)] = (unsigned short)i;
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  double* R = rows + (threadIdx.x >> 5) * 3 * RD;
-  // slots past the tile read entry RD - 1 of the rows, which stays zero
-  int cx[NCOL], cy[NCOL];
-#pragma unroll
-  for (int j = 0; j < NCOL; j++) {
-    const int c = lane + 32 * j;
-    cx[j] = c < TILE * TILE ? c / TILE : RD - 1;
-    cy[j] = c < TILE * TILE ? c % TILE : RD - 1;
-  }
-  const int kd = lane / RD, kq = lane - kd * RD;  // this lane's row entry
-  for (;;) {
-    int bi = 0;
-    if (lane == 0) bi = atomicAdd(&misc[0], 1);
-    bi = __shfl_sync(0xffffffffu, bi, 0);
-    if (bi >= nblk) break;
-    const int nb = cnt[bi];
-    if (nb == 0) continue;
-    const int start = boff[bi];
-    int org[3];
-    org[2] = (bi % nbd) * TBD;
-    org[1] = ((bi / nbd) % nbd) * TBD;
-    org[0] = (bi / (nbd * nbd)) * TBD;
-    double acc[NCOL][TILE];
-#pragma unroll
-    for (int j = 0; j < NCOL; j++)
-#pragma unroll
-      for (int t = 0; t < TILE; t++) acc[j][t] = 0.0;
-    for (int k = 0; k < nb; k++) {
-      const int pt = c0 + perm[start + k];
-      // this lane's row entry: kernel value at stencil offset kq - o[kd] of
-      // dimension kd (zero outside the stencil; the x row carries the strength)
-      double v = 0.0;
-      if (lane < 3 * RD) {
-        const double x = off[(size_t)kd * ns + pt] * a.scale_d;
-        double f0;
-        int b = kernel_start<double>(a, x, f0) - g.l0;
-        b = b < 0 ? 0 : (b > g.G - W ? g.G - W : b);
-        int j = kq - (b - (kd == 0 ? org[0] : (kd == 1 ? org[1] : org[2])));
-        if (!FGT_DCHECK(kq != RD - 1 || j >= W, 208)) j = W;  // entry RD - 1 stays zero
-        if (j >= 0 && j < W) {
-          v = es_kernel<double>((f0 + (double)j) * a.inv_hw, a.beta);
-          if (kd == 0) v *= is_q ? sq[pt] : sq[pt] * sr[pt];
-        }
-        R[lane] = v;
-      }
-      __syncwarp();
-      double pz[TILE];
-#pragma unroll
-      for (int t = 0; t < TILE; t++) pz[t] = R[2 * RD + t];
-#pragma unroll
-      for (int j = 0; j < NCOL; j++) {
-        const double pxy = R[cx[j]] * R[RD + cy[j]];
-#pragma unroll
-        for (int t = 0; t < TILE; t++) acc[j][t] = fma(pxy, pz[t], acc[j][t]);
-      }
-      __syncwarp();
-    }
-#pragma unroll
-    for (int j = 0; j < NCOL; j++) {
-      const int x = org[0] + cx[j], y = org[1] + cy[j];
-      if (lane + 32 * j < TILE * TILE && x < g.G && y < g.G) {
-        double* col = B + x * g.str[0] + y * g.str[1] + org[2];
-#pragma unroll
-        for (int t = 0; t < TILE; t++)
-          if (org[2] + t < g.G && acc[j][t] != 0.0) atomicAdd(col + t, acc[j][t]);
-      }
-    }
-  }
-  __syncthreads();
-}
-constexpr int TB_D = 2;  // FP64 block edge (register tile of 3 x 9 columns, no spills)
-
 template <typename T, int DIM, int W, bool GB, bool TILED>
 __global__ void __launch_bounds__(PW_THREADS) k_form(PWArgs<T> a, FormIO io, FormPtrs<T> p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -351,9 +231,9 @@ __global__ void __launch_bounds__(PW_THREADS) k_form(PWArgs<T> a, FormIO io, For
   int* tcnt = reinterpret_cast<int*>(smem_raw + tw_bytes16<T>(G, K));  // NBLK_MAX
   int* toff = tcnt + NBLK_MAX;                             // NBLK_MAX
   int* tmisc = toff + NBLK_MAX;                            // 32
-  int* ttmp = tmisc + 32;                                  // fch
-  unsigned short* tperm = reinterpret_cast<unsigned short*>(ttmp + fch<T>());  // fch
-  T* trows = reinterpret_cast<T*>(tperm + fch<T>());  // FP32: warps * PB * 3 * TP
+  int* ttmp = tmisc + 32;                                  // FCH
+  unsigned short* tperm = reinterpret_cast<unsigned short*>(ttmp + FCH);  // FCH
+  T* trows = reinterpret_cast<T*>(tperm + FCH);  // FP32: warps * PB * 3 * TP
   T* B = GB ? a.gscratch + (size_t)blockIdx.x * g.bufsz
             : reinterpret_cast<T*>(smem_raw + (TILED ? tiled_offset<T>(G, K)
                                                      : order_offset<T>(G, K)));
@@ -388,13 +268,9 @@ __global__ void __launch_bounds__(PW_THREADS) k_form(PWArgs<T> a, FormIO io, For
         if constexpr (TILED) {
           const T* sq = is_q ? p.q + (size_t)id * io.ns : p.ds + (size_t)id * io.ns;
           const T* sr = is_q ? nullptr : p.rn + (size_t)dd * io.ns;
-          for (int c0 = p0; c0 < p1; c0 += fch<T>()) {
-            if constexpr (std::is_same<T, double>::value)
-              spread_tiled_d<W, TB_D>(a, B, p.off, io.ns, sq, sr, is_q, c0, min(fch<T>(), p1 - c0),
-                                      tcnt, toff, tmisc, ttmp, tperm, trows);
-            else
-              spread_tiled<T, W>(a, B, p.off, io.ns, sq, sr, is_q, c0, min(fch<T>(), p1 - c0),
-                                 tcnt, toff, tmisc, ttmp, tperm, trows);
+          for (int c0 = p0; c0 < p1; c0 += FCH) {
+            spread_tiled<T, W>(a, B, p.off, io.ns, sq, sr, is_q, c0, min(FCH, p1 - c0), tcnt, toff,
+                               tmisc, ttmp, tperm, trows);
           }
         } else {
           for (int c0 = p0; c0 < p1; c0 += ORDER_CHUNK) {
@@ -847,31 +723,6 @@ __global__ void k_count_points(int n, const int* __restrict__ box, const int* __
 
 template <typename T, int DIM, int W>
 int launch_form(PWArgs<T>& a, const FormIO& io, const FormPtrs<T>& fp, DBuf<T>& gs, cudaStream_t s) {
-  size_t fix = fixed_smem(a, W, 1);
-  size_t need = fix + sizeof(T) * (size_t)a.g.bufsz;
-  int grid = std::max(1, std::min(io.max_items, kSMs));
-  if constexpr (std::is_same<T, float>::value && DIM == 3 && TB + W - 1 <= TP - 1) {
-    const int nbd = (a.g.G - W + 1 + TB - 1) / TB;
-    const size_t tneed = tiled_offset<T>(a.g.G, a.g.K) + sizeof(T) * (size_t)a.g.bufsz;
-    if (!a.g.wrap && nbd * nbd * nbd <= NBLK_MAX && tneed <= (size_t)MAXSMEM) {
-      auto k = k_form<T, DIM, W, false, true>;
-      set_smem(k, tneed);
-      k<<<grid, PW_THREADS, tneed, s>>>(a, io, fp);
-      FGT_LAUNCH_CHECK();
-      return 1;
-    }
-  }
-  if constexpr (std::is_same<T, double>::value && DIM == 3 && W <= 8) {
-    const int nbd = (a.g.G - W + 1 + TB_D - 1) / TB_D;
-    const size_t tneed = tiled_offset<T>(a.g.G, a.g.K) + sizeof(T) * (size_t)a.g.bufsz;
-    if (!a.g.wrap && nbd * nbd * nbd <= NBLK_MAX && tneed <= (size_t)MAXSMEM) {
-      auto k = k_form<T, DIM, W, false, true>;
-      set_smem(k, tneed);
-      k<<<grid, PW_THREADS, tneed, s>>>(a, io, fp);
-      FGT_LAUNCH_CHECK();
-      return 1;
-    }
-  }
   if constexpr (std::is_same<T, double>::value && DIM == 3) {
     if (io.f64) {
       Form64 f;
@@ -895,16 +746,35 @@ int launch_form(PWArgs<T>& a, const FormIO& io, const FormPtrs<T>& fp, DBuf<T>& 
       return form64_launch(W, &a, f, s);
     }
   }
+  size_t fix = fixed_smem(a, W, 1);
+  size_t need = fix + sizeof(T) * (size_t)a.g.bufsz;
+  int grid = std::max(1, std::min(io.max_items, kSMs));
+  if constexpr (std::is_same<T, float>::value && DIM == 3 && TB + W - 1 <= TP - 1) {
+    const int nbd = (a.g.G - W + 1 + TB - 1) / TB;
+    const size_t tneed = tiled_offset<T>(a.g.G, a.g.K) + sizeof(T) * (size_t)a.g.bufsz;
+    if (!a.g.wrap && nbd * nbd * nbd <= NBLK_MAX && tneed <= (size_t)MAXSMEM) {
+      auto k = k_form<T, DIM, W, false, true>;
+      set_smem(k, tneed);
+      k<<<grid, PW_THREADS, tneed, s>>>(a, io, fp);
+      FGT_LAUNCH_CHECK();
+      return 1;
+    }
+  }
+  if constexpr (std::is_same<T, float>::value && DIM == 3) {
+    if (io.nslab > 1) {
+      // x-slab grids (the expansions were zeroed by the caller)
+      const size_t sm = fix + sizeof(T) * (size_t)a.g.str[0] * io.slab;
+      auto k = k_form_slab<T, W>;
+      set_smem(k, sm);
+      k<<<grid, PW_THREADS, sm, s>>>(a, io, fp);
+      FGT_LAUNCH_CHECK();
+      return 1;
+    }
+  }
   if (need <= (size_t)MAXSMEM) {
     auto k = k_form<T, DIM, W, false, false>;
     set_smem(k, need);
     k<<<grid, PW_THREADS, need, s>>>(a, io, fp);
-  } else if (DIM == 3 && io.nslab > 1) {
-    // x-slab grids (the expansions were zeroed by the caller)
-    const size_t sm = fix + sizeof(T) * (size_t)a.g.str[0] * io.slab;
-    auto k = k_form_slab<T, W>;
-    set_smem(k, sm);
-    k<<<grid, PW_THREADS, sm, s>>>(a, io, fp);
   } else {
     gs.alloc((size_t)grid * a.g.bufsz, s);
     a.gscratch = gs;
@@ -1152,13 +1022,11 @@ int pw_form(const PWParams& P, const Tree& t, const Lists& L, const SourceSet<T>
     sp = slab_plan(a.g, sizeof(T), order_offset<T>(a.g.G, a.g.K));
   if (sp.nslab > 1) D.mp.zero();
   if (work) work->slabs_form = sp.nslab;
-  // FP64 grids that do not fit in shared memory: the matrix instructions
-  io.f64 = sizeof(T) == 8 && P.dim == 3 &&
-           sizeof(T) * (size_t)a.g.bufsz + order_offset<T>(a.g.G, a.g.K) > (size_t)MAXSMEM &&
-           form64_takes(P.w, P.K, P.G, P.wrap);
+  // FP64 3D: the matrix instructions
+  io.f64 = sizeof(T) == 8 && P.dim == 3 && form64_takes(P.w, P.K, P.G, P.wrap);
   ItemList il;
   build_items(il, L.n_form, small2 ? first.get() : nullptr, oval, L.form_box, src.lo, src.hi,
-              nullptr, nullptr, src.n, thr, !io.f64, s, sp.nslab, io.f64);
+              nullptr, nullptr, src.n, io.f64 ? split_threshold64(L.n_form, src.n) : thr, !io.f64, s, sp.nslab, io.f64);
   io.items = il.items;
   io.n_items = il.n_items;
   io.item_off = il.ioff;

@@ -17,7 +17,10 @@
 // 1e-12: 33.7 -> 2.1 and 21.1 -> 6.6 ms.  One fused kernel per direction
 // (spreading and transforms of a box in one 256-thread CTA) took 4.9 and
 // 15.6 ms: the transforms want the 16 warps of two CTAs to hide their loads,
-// the spreading and the interpolation 200+ registers per thread.
+// the spreading and the interpolation 200+ registers per thread.  Grids that
+// fit in shared memory gain too (N = M = 2e6, eps = 1e-6: form 3.2 -> 2.0,
+// evaluation 7.8 -> 4.0 ms against a 200 KB grid and a SIMT stencil per CTA;
+// N = 1e5, eps = 1e-3: 0.43 -> 0.22 and 0.37 -> 0.17).
 #include <stdlib.h>
 
 #include "fgt_pw64.cuh"
@@ -512,6 +515,8 @@ __global__ void __launch_bounds__(TT64, 2)
 template <int W>
 struct Tile64;
 template <>
+struct Tile64<6> { static constexpr int TBX = 3, TBY = 3, TBZ = 3; };
+template <>
 struct Tile64<8> { static constexpr int TBX = 3, TBY = 1, TBZ = 5; };
 template <>
 struct Tile64<10> { static constexpr int TBX = 3, TBY = 7, TBZ = 3; };
@@ -529,7 +534,7 @@ struct EvalSmem64 {
   using TL = Tile64<W>;
   static constexpr int TX = W + TL::TBX - 1, TY = W + TL::TBY - 1, TZ = W + TL::TBZ - 1;
   static constexpr int MY = TY / 8, KZ = TZ / 4, ND = DERIV ? 2 : 1;
-  static constexpr int YS = TY == 8 ? 10 : 18, ZS = TZ == 16 ? 20 : TZ;  // row strides
+  static constexpr int YS = TY == 8 ? 10 : 18, ZS = TZ % 8 == 4 ? TZ : TZ + 4;  // row strides
   static_assert(TY % 8 == 0 && TZ % 4 == 0 && ZS % 8 == 4, "whole matrix tiles");
   struct alignas(16) Rows {  // values (0) and derivatives (1) of a unit's kernel rows
     double x[ND][TX][EUP64];
@@ -538,6 +543,9 @@ struct EvalSmem64 {
   };
   Sort64<ECH64, EUP64> s;
   Rows rows[W64];
+  // a unit's kernel and derivative sums and its points' cells in the tile
+  double ksum[W64][ND == 2 ? EUP64 : 1][3][2];
+  int cell[W64][ND == 2 ? EUP64 : 1][3];
   int item;
 };
 
@@ -881,10 +889,20 @@ __global__ void __launch_bounds__(T64, 1)
           double f0;
           o = cell64<W>(a, off[pt], f0) - (d == 0 ? org[0] : (d == 1 ? org[1] : org[2]));
           if (!FGT_DCHECK(o >= 0 && o + W <= TD, 607)) o = 0;
+          double ks = 0.0, kd = 0.0;
           es64_row<W, DERIV>(a, es, f0, [&](int j, double f, double df) {
             w[(o + j) * st] = f;
-            if constexpr (DERIV) w[dv + (o + j) * st] = df;
+            if constexpr (DERIV) {
+              w[dv + (o + j) * st] = df;
+              ks += f;
+              kd += df;
+            }
           });
+          if constexpr (DERIV) {
+            sm.ksum[warp][pi][d][0] = ks;
+            sm.ksum[warp][pi][d][1] = kd;
+            sm.cell[warp][pi][d] = o;
+          }
         }
         // zero outside the stencil, and rows of no point
         for (int k = pi < cnt ? W : 0; k < TD; k++) {
@@ -914,8 +932,19 @@ __global__ void __launch_bounds__(T64, 1)
             const int q = st ? q0[1] + ii - m[0] : q0[0] + ii;
             const int comp = DERIV ? k : c;
             if (comp >= (st ? p.ncomp[1] : p.ncomp[0])) continue;
-            const double r = k == 0 ? v[nt][i][0]
-                                    : (k == 1 ? v[nt][i][1] : (k == 2 ? v[nt][i][2] : v[nt][i][3]));
+            double r = k == 0 ? v[nt][i][0]
+                              : (k == 1 ? v[nt][i][1] : (k == 2 ? v[nt][i][2] : v[nt][i][3]));
+            if constexpr (DERIV) {
+              if (p.drop_ref && k > 0) {
+                const auto& S = sm.ksum[warp][pj];
+                const int* o = sm.cell[warp][pj];
+                const int x = org[0] + o[0] + W / 2, y = org[1] + o[1] + W / 2,
+                          z = org[2] + o[2] + W / 2;
+                if (FGT_DCHECK(x >= 0 && x < G && y >= 0 && y < G && z >= 0 && z < G, 612))
+                  r -= B[(size_t)x * lay.planep + y * lay.rowp + z] *
+                       (S[0][k == 1] * S[1][k == 2] * S[2][k == 3]);
+              }
+            }
             double* out = st ? p.out[1] : p.out[0];
             atomicAdd(out + ((size_t)comp * p.nd + id) * (st ? p.n[1] : p.n[0]) + q, r);
           }
@@ -1067,7 +1096,7 @@ __global__ void __launch_bounds__(T64, 1)
 }  // namespace
 
 bool form64_takes(int w, int K, int G, bool wrap) {
-  if (wrap || (w != 10 && w != 12 && w != 14) || K > 31 || G > 64) return false;
+  if (wrap || w < 6 || w > 14 || (w & 1) || K > 31 || G > 64) return false;
   const int tb = 17 - w, nbd = (G - w + tb) / tb;
   return nbd * nbd * nbd <= NBLK64;
 }
@@ -1080,6 +1109,7 @@ static bool eval_blocks_fit(int G) {
 bool eval64_takes(int w, int K, int G, bool wrap) {
   if (wrap || K > 31 || G > 64) return false;
   switch (w) {
+    case 6: return eval_blocks_fit<6>(G);
     case 8: return eval_blocks_fit<8>(G);
     case 10: return eval_blocks_fit<10>(G);
     case 12: return eval_blocks_fit<12>(G);
@@ -1179,6 +1209,8 @@ static int launch_form64(const PWArgs<double>& a, const Form64& io, cudaStream_t
 int form64_launch(int w, const void* av, const Form64& io, cudaStream_t s) {
   const PWArgs<double>& a = *static_cast<const PWArgs<double>*>(av);
   switch (w) {
+    case 6: return launch_form64<6>(a, io, s);
+    case 8: return launch_form64<8>(a, io, s);
     case 10: return launch_form64<10>(a, io, s);
     case 12: return launch_form64<12>(a, io, s);
     case 14: return launch_form64<14>(a, io, s);
@@ -1231,6 +1263,9 @@ int eval64_launch(int w, bool deriv, const void* av, const Eval64& io, cudaStrea
   case WW:                                                         \
     return deriv ? launch_eval64<WW, true>(a, io, s) : launch_eval64<WW, false>(a, io, s);
   switch (w) {
+    case 6:
+      FGT_REQUIRE(!deriv, FGT_ERR_UNSUPPORTED, "derivative evaluation needs a kernel width >= 7");
+      return launch_eval64<6, false>(a, io, s);
     FGT_E64(8) FGT_E64(10) FGT_E64(12) FGT_E64(14) FGT_E64(16)
     default: FGT_REQUIRE(false, FGT_ERR_UNSUPPORTED, "no FP64 evaluation kernel for this width");
   }

@@ -29,6 +29,9 @@ struct Eval64 {
   double* out[2];
   int n[2], ncomp[2];
   int nd, ncomp_max;
+  // gradients without the terms of the stencil's centre cell (as
+  // interp_grad_cells, which the grids that fit in shared memory had)
+  int drop_ref;
 };
 
 // x-planes of a grid transformed by one CTA.

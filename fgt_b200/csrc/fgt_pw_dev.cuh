@@ -1032,6 +1032,13 @@ inline int form_split_threshold(long long n) {
 inline int eval_split_threshold(long long n) {
   return (int)std::max<long long>(8192, (n + 2 * kSMs - 1) / (2 * kSMs));
 }
+// The FP64 matrix-instruction kernels build a box's grid once, whatever its
+// parts: with too few boxes for the SMs, parts of 1/8 of an SM's share, 512
+// points at least (below that the parts' blocks hold too few points each).
+inline int split_threshold64(int nbox, long long n) {
+  if (nbox >= 4 * kSMs) return eval_split_threshold(n);
+  return (int)std::min<long long>(8192, std::max<long long>(512, n / (8 * kSMs)));
+}
 
 // Work items of a sorted slot list (host side, all sizes stay on the device).
 // n: list length bound; count: actual length on the device (or null = n);

@@ -38,6 +38,7 @@ struct EvalPtrs {
   int cell_bins;  // base cells of the sub-grid for the cell order, 0: bank-class order
   int slab, nslab;  // x-slab grids: planes per slab and slabs per box (1: whole grids)
   const int* item_off;  // first item of every box (e64)
+  int drop_ref;         // e64: see Eval64
   int e64;  // FP64 3D grids on the matrix instructions (fgt_pw64.cu)
 };
 
@@ -934,6 +935,7 @@ inline Eval64 eval64_args(const EvalPtrs<double>& ep) {
   }
   io.nd = ep.nd;
   io.ncomp_max = ep.ncomp_max;
+  io.drop_ref = ep.drop_ref;
   return io;
 }
 
@@ -1066,12 +1068,6 @@ int eval_dim(int dim, int w, PWArgs<T>& a, const EvalPtrs<T>& ep, bool deriv, DB
 
 }  // namespace
 
-// FP64 grids that do not fit in shared memory.
-template <typename T>
-static bool e64_wanted(const Geo& g) {
-  return eval_offset<T>(g.G, g.K) + sizeof(T) * (size_t)g.bufsz > (size_t)MAXSMEM;
-}
-
 template <typename T>
 int pw_eval(const PWParams& P, const Tree& t, const Lists& L, const PWData<T>& D,
             const EvalSet<T>& e0, const EvalSet<T>& e1, int small_eval, PWWork* work,
@@ -1144,17 +1140,17 @@ int pw_eval(const PWParams& P, const Tree& t, const Lists& L, const PWData<T>& D
   ep.items = nullptr;
   ep.n_items = nullptr;
   ep.max_items = 0;
-  // grids too large for shared memory (3D without wrap-around): FP64 on the
-  // matrix instructions, else x-slabs
+  // FP64 3D without wrap-around: the matrix instructions; else x-slabs for
+  // grids too large for shared memory
   SlabPlan sp;
-  ep.e64 = sizeof(T) == 8 && P.dim == 3 && e64_wanted<T>(a.g) &&
-           eval64_takes(Pe.w, P.K, Pe.G, Pe.wrap);
-  if (!ep.e64 &&
-      eval_offset<T>(a.g.G, a.g.K) + sizeof(T) * (size_t)a.g.bufsz > (size_t)MAXSMEM)
+  const bool beyond = eval_offset<T>(a.g.G, a.g.K) + sizeof(T) * (size_t)a.g.bufsz > (size_t)MAXSMEM;
+  ep.e64 = sizeof(T) == 8 && P.dim == 3 && eval64_takes(Pe.w, P.K, Pe.G, Pe.wrap);
+  ep.drop_ref = !beyond;
+  if (!ep.e64 && beyond)
     sp = slab_plan(a.g, sizeof(T), order_offset<T>(a.g.G, a.g.K));
   ep.slab = sp.planes;
   ep.nslab = sp.nslab;
-  if (work) work->slabs_eval = ep.e64 ? ceil_div(Pe.G, SLAB64) : sp.nslab;
+  if (work) work->slabs_eval = ep.e64 && beyond ? ceil_div(Pe.G, SLAB64) : sp.nslab;
   ItemList il;
   DBuf<int> first2(1, s), next2(1, s);
   DBuf<T> gs;
@@ -1189,7 +1185,8 @@ int pw_eval(const PWParams& P, const Tree& t, const Lists& L, const PWData<T>& D
     build_items(il, L.n_eval, small2 ? first2.get() : counts.get(),
                 reinterpret_cast<const uint32_t*>(lbig.get()),
                 L.eval_box, u0 ? e0.lo : e1.lo, u0 ? e0.hi : e1.hi, (u0 && u1) ? e1.lo : nullptr,
-                (u0 && u1) ? e1.hi : nullptr, npts, eval_split_threshold(npts), false, s,
+                (u0 && u1) ? e1.hi : nullptr, npts,
+                ep.e64 ? split_threshold64(L.n_eval, npts) : eval_split_threshold(npts), false, s,
                 sp.nslab, ep.e64);
     ep.items = il.items;
     ep.item_off = il.ioff;

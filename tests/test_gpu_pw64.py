@@ -1,6 +1,6 @@
 """FP64 3D form, evaluation and modal sums on the matrix instructions
 (fgt_pw64.cu) against the oracle's exact plane-wave sums, at the edges of
-their tiles: kernel widths 10-16, blocks with 1, 8, 9, 16, 17, 64, 65 and
+their tiles: kernel widths 6-16, blocks with 1, 8, 9, 16, 17, 64, 65 and
 more than 8192 points (several sort chunks), several densities, dipoles,
 hessians, boxes below the modal threshold, several runs over the boxes.
 
@@ -28,6 +28,11 @@ def points(seed, big):
 
 
 @pytest.mark.parametrize("eps,pgh,nd,dip,big", [
+    (1e-3, 1, 1, False, 400),
+    (1e-3, 2, 1, False, 9001),
+    (1e-4, 3, 1, True, 400),
+    (1e-6, 1, 2, False, 400),
+    (1e-6, 2, 1, True, 400),
     (1e-8, 1, 1, False, 400),
     (1e-8, 2, 2, False, 400),
     (1e-9, 2, 1, False, 9001),

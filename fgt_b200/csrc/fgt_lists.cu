@@ -16,60 +16,6 @@ struct TV {
   int lev_start[66];
 };
 
-__device__ __forceinline__ void coords_of(const TV& tv, int b, uint32_t* c) {
-  int l = tv.level[b];
-  uint64_t key = tv.key[b];
-  for (int k = 0; k < tv.dim; k++) c[k] = 0;
-  for (int j = 0; j < l; j++) {
-    int dig = (int)((key >> (tv.dim * (l - 1 - j))) & ((1u << tv.dim) - 1));
-    for (int k = 0; k < tv.dim; k++) c[k] = (c[k] << 1) | ((dig >> k) & 1);
-  }
-}
-
-__device__ __forceinline__ int find_box(const TV& tv, int l, const uint32_t* c) {
-  uint64_t key = 0;
-  for (int j = 0; j < l; j++) {
-    int dig = 0;
-    for (int k = 0; k < tv.dim; k++) dig |= ((c[k] >> (l - 1 - j)) & 1) << k;
-    key = (key << tv.dim) | (uint64_t)dig;
-  }
-  int lo = tv.lev_start[l], n = tv.lev_start[l + 1] - lo;
-  int i = dev_find(tv.key + lo, n, key);
-  return i < 0 ? -1 : lo + i;
-}
-
-// Colleagues (same level, closures touching, self included), as computecoll
-// (src/common/tree_routs_nd.f:106-242): periodic wrap when `periodic`.
-template <typename F>
-__device__ __forceinline__ void for_colleagues(const TV& tv, int b, int periodic, F f) {
-  int l = tv.level[b];
-  uint32_t c[FGT_MAXDIM];
-  coords_of(tv, b, c);
-  long long n = 1ll << l;
-  long long vals[FGT_MAXDIM][3];
-  int nv[FGT_MAXDIM];
-  for (int k = 0; k < tv.dim; k++) {
-    nv[k] = 0;
-    for (int o = -1; o <= 1; o++) {
-      long long q = (long long)c[k] + o;
-      if (periodic) q = ((q % n) + n) % n;
-      else if (q < 0 || q >= n) continue;
-      bool dup = false;
-      for (int j = 0; j < nv[k]; j++) dup |= (vals[k][j] == q);
-      if (!dup) vals[k][nv[k]++] = q;
-    }
-  }
-  int tot = 1;
-  for (int k = 0; k < tv.dim; k++) tot *= nv[k];
-  for (int i = 0; i < tot; i++) {
-    uint32_t q[FGT_MAXDIM];
-    int r = i;
-    for (int k = 0; k < tv.dim; k++) { q[k] = (uint32_t)vals[k][r % nv[k]]; r /= nv[k]; }
-    int bb = find_box(tv, l, q);
-    if (bb >= 0) f(bb);
-  }
-}
-
 // ---- modified list 1 of every target box (pfgt_compute_modified_list1,
 // src/common/tree_routs_nd.f:1063-1257, restated from the target side):
 //   * same level: leaf colleagues (self included);
@@ -122,8 +68,10 @@ __device__ __forceinline__ bool touch_levels_d(const uint32_t* cf, int lf, const
   }
   return ok;
 }
-// Colleague `i` (in the candidate order of for_colleagues) of box b on this
-// lane: the box id, or -1 (no such box, or i >= *tot).
+// Colleague `i` of box b on this lane: the box id, or -1 (no such box, or
+// i >= *tot).  Colleagues are the boxes of the same level whose closures touch
+// (self included), as computecoll (src/common/tree_routs_nd.f:106-242), with
+// periodic wrap when `periodic`; the first coordinate runs fastest.
 template <int DIM>
 __device__ __forceinline__ int colleague_of(const TV& tv, int b, int periodic, int i, int* tot) {
   const int l = tv.level[b];
@@ -247,19 +195,32 @@ void launch_list1(const TV& tv, int nb, int* cnt, const int* ptr, int* out, int*
 }
 
 // Plane-wave flags at the cutoff level: form (npts > ndiv, pfgt.f:779) and
-// ifpwexp (pfgt_find_pwexp_boxes, src/common/tree_routs_nd.f:1373-1460).
+// ifpwexp (pfgt_find_pwexp_boxes, src/common/tree_routs_nd.f:1373-1460).  One
+// group of lanes per box, one colleague's key search per lane (a thread's 27
+// searches one after the other took 53-68 us whatever the box count).
+template <int DIM>
+__host__ __device__ constexpr int coll_lanes() {  // >= 3^DIM
+  return DIM == 3 ? 32 : (DIM == 2 ? 16 : 4);
+}
+template <int DIM>
 __global__ void k_pw_flags(TV tv, int ndiv, int* __restrict__ fform, int* __restrict__ feval) {
-  int lo = tv.lev_start[tv.ncutoff], n = tv.lev_start[tv.ncutoff + 1] - lo;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    int b = lo + i;
-    fform[i] = (tv.src_hi[b] - tv.src_lo[b] > ndiv) ? 1 : 0;
-    int e = 0;
-    if (tv.npwlevel <= 0) {
-      e = (b == 0);
-    } else {
-      for_colleagues(tv, b, tv.iperiod0, [&](int J) { e |= tv.nonleaf[J]; });
+  const int lo = tv.lev_start[tv.ncutoff], n = tv.lev_start[tv.ncutoff + 1] - lo;
+  constexpr int GL = coll_lanes<DIM>();
+  const int gl = threadIdx.x & (GL - 1), ng = gridDim.x * blockDim.x / GL;
+  const int g0 = (blockIdx.x * blockDim.x + threadIdx.x) / GL;
+  for (int i0 = g0 - g0 % (32 / GL); i0 < n; i0 += ng) {  // whole warps
+    const int i = i0 + g0 % (32 / GL), b = lo + min(i, n - 1);
+    bool e = b == 0;
+    if (tv.npwlevel > 0) {
+      int tot;
+      const int J = colleague_of<DIM>(tv, b, tv.iperiod0, gl, &tot);
+      const unsigned m = __ballot_sync(0xffffffffu, J >= 0 && tv.nonleaf[J]);
+      e = (m >> (threadIdx.x & (32 - GL))) & ((1ull << GL) - 1);
     }
-    feval[i] = e;
+    if (gl == 0 && i < n) {
+      fform[i] = (tv.src_hi[b] - tv.src_lo[b] > ndiv) ? 1 : 0;
+      feval[i] = e ? 1 : 0;
+    }
   }
 }
 
@@ -276,40 +237,55 @@ __device__ __forceinline__ int fnint(double x) { return (int)round(x); }
 // PW list of each eval box: non-leaf colleagues other than itself
 // (pfgt_compute_listpw, src/common/tree_routs_nd.f:1487-1555) with their
 // shift-table index (gnd_find_pwshift_ind, src/bfgt/bfgt_pwrouts.f:1592-1636).
-template <bool FILL>
+// One group of lanes per box, one colleague per lane, kept in colleague order.
+template <int DIM, bool FILL>
 __global__ void k_trans(TV tv, const int* __restrict__ eval_box, int n_eval,
                         const int* __restrict__ form_slot, const int* __restrict__ ptr,
                         int* __restrict__ cnt, int* __restrict__ src, int* __restrict__ widx) {
-  int lo = tv.lev_start[tv.ncutoff];
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n_eval; e += gridDim.x * blockDim.x) {
-    int t = eval_box[e];
-    int c = 0, p = FILL ? ptr[e] : 0;
-    for_colleagues(tv, t, tv.iperiod0, [&](int s) {
-      if (s == t || !tv.nonleaf[s]) return;
-      int slot = form_slot[s - lo];
-      if (slot < 0) return;  // empty expansion contributes nothing
-      if (FILL) {
-        int ind = 0, inc = 1;
-        for (int d = 0; d < tv.dim; d++) {
-          double dx = tv.center[(size_t)t * tv.dim + d] - tv.center[(size_t)s * tv.dim + d];
-          int jx = fnint(dx / tv.xmin);
-          if (tv.iperiod0 == 1) {
-            int jxp1 = fnint((dx - tv.bs0) / tv.xmin);
-            int jxm1 = fnint((dx + tv.bs0) / tv.xmin);
-            if (abs(jx) > abs(jxp1)) jx = jxp1;
-            if (abs(jx) > abs(jxm1)) jx = jxm1;
-          }
-          ind += (jx + 1) * inc;
-          inc *= 3;
+  const int lo = tv.lev_start[tv.ncutoff];
+  constexpr int GL = coll_lanes<DIM>();
+  const int gl = threadIdx.x & (GL - 1), ng = gridDim.x * blockDim.x / GL;
+  const int g0 = (blockIdx.x * blockDim.x + threadIdx.x) / GL;
+  for (int e0 = g0 - g0 % (32 / GL); e0 < n_eval; e0 += ng) {  // whole warps
+    const int e = e0 + g0 % (32 / GL), t = eval_box[min(e, n_eval - 1)];
+    int tot, slot = -1;
+    const int s = colleague_of<DIM>(tv, t, tv.iperiod0, gl, &tot);
+    if (s >= 0 && s != t && tv.nonleaf[s]) slot = form_slot[s - lo];  // -1: empty expansion
+    const unsigned m = (unsigned)((__ballot_sync(0xffffffffu, slot >= 0) >> (threadIdx.x & (32 - GL))) &
+                                  ((1ull << GL) - 1));
+    if (!FILL) {
+      if (gl == 0 && e < n_eval) cnt[e] = __popc(m);
+    } else if (slot >= 0 && e < n_eval) {
+      int ind = 0, inc = 1;
+#pragma unroll
+      for (int d = 0; d < DIM; d++) {
+        const double dx = tv.center[(size_t)t * DIM + d] - tv.center[(size_t)s * DIM + d];
+        int jx = fnint(dx / tv.xmin);
+        if (tv.iperiod0 == 1) {
+          const int jxp1 = fnint((dx - tv.bs0) / tv.xmin), jxm1 = fnint((dx + tv.bs0) / tv.xmin);
+          if (abs(jx) > abs(jxp1)) jx = jxp1;
+          if (abs(jx) > abs(jxm1)) jx = jxm1;
         }
-        src[p] = slot;
-        widx[p] = ind;
-        p++;
+        ind += (jx + 1) * inc;
+        inc *= 3;
       }
-      c++;
-    });
-    if (!FILL) cnt[e] = c;
+      const int p = ptr[e] + __popc(m & ((1u << gl) - 1u));
+      src[p] = slot;
+      widx[p] = ind;
+    }
   }
+}
+template <bool FILL>
+void launch_trans(const TV& tv, const int* eval_box, int n_eval, const int* form_slot,
+                  const int* ptr, int* cnt, int* src, int* widx, cudaStream_t s) {
+  const int grid = grid_for((long long)n_eval * (tv.dim == 3 ? 32 : (tv.dim == 2 ? 16 : 4)), 256);
+  auto go = [&](auto kern) {
+    kern<<<grid, 256, 0, s>>>(tv, eval_box, n_eval, form_slot, ptr, cnt, src, widx);
+    FGT_LAUNCH_CHECK();
+  };
+  if (tv.dim == 1) go(k_trans<1, FILL>);
+  else if (tv.dim == 2) go(k_trans<2, FILL>);
+  else go(k_trans<3, FILL>);
 }
 
 TV make_tv(const Tree& t, int npwlevel, int iperiod0, int nlevend) {
@@ -367,7 +343,10 @@ void build_lists(const Tree& t, int npwlevel, int iperiod0, int nlevend, bool do
     tf.alloc(1, s);
     te.alloc(1, s);
     fslot.alloc(n, s);
-    k_pw_flags<<<grid_for(n, 128), 128, 0, s>>>(tv, t.ndiv, ff, fe);
+    const int grid = grid_for((long long)n * (tv.dim == 3 ? 32 : (tv.dim == 2 ? 16 : 4)), 256);
+    if (tv.dim == 1) k_pw_flags<1><<<grid, 256, 0, s>>>(tv, t.ndiv, ff, fe);
+    else if (tv.dim == 2) k_pw_flags<2><<<grid, 256, 0, s>>>(tv, t.ndiv, ff, fe);
+    else k_pw_flags<3><<<grid, 256, 0, s>>>(tv, t.ndiv, ff, fe);
     FGT_LAUNCH_CHECK();
     exclusive_scan_i32(ff, pf, n, tf, s);
     exclusive_scan_i32(fe, pe, n, te, s);
@@ -400,21 +379,15 @@ void build_lists(const Tree& t, int npwlevel, int iperiod0, int nlevend, bool do
   L.trans_ptr.alloc(L.n_eval + 1, s);
   {
     DBuf<int> cnt(std::max(L.n_eval, 1), s);
-    if (L.n_eval > 0) {
-      k_trans<false><<<grid_for(L.n_eval, 128), 128, 0, s>>>(tv, L.eval_box, L.n_eval, fslot,
-                                                             nullptr, cnt, nullptr, nullptr);
-      FGT_LAUNCH_CHECK();
-    }
+    if (L.n_eval > 0)
+      launch_trans<false>(tv, L.eval_box, L.n_eval, fslot, nullptr, cnt, nullptr, nullptr, s);
     exclusive_scan_i32(cnt, L.trans_ptr, L.n_eval, L.trans_ptr.get() + L.n_eval, s);
     L.n_trans = fetch_int(L.trans_ptr.get() + L.n_eval, s);
     L.trans_src.alloc(std::max(L.n_trans, 1), s);
     L.trans_w.alloc(std::max(L.n_trans, 1), s);
-    if (L.n_eval > 0) {
-      k_trans<true><<<grid_for(L.n_eval, 128), 128, 0, s>>>(tv, L.eval_box, L.n_eval, fslot,
-                                                            L.trans_ptr, nullptr, L.trans_src,
-                                                            L.trans_w);
-      FGT_LAUNCH_CHECK();
-    }
+    if (L.n_eval > 0)
+      launch_trans<true>(tv, L.eval_box, L.n_eval, fslot, L.trans_ptr, nullptr, L.trans_src,
+                         L.trans_w, s);
   }
 }
 

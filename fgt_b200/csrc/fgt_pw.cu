@@ -721,29 +721,34 @@ __global__ void k_count_points(int n, const int* __restrict__ box, const int* __
     atomicAdd(cnt, (unsigned long long)(hi[box[i]] - lo[box[i]]));
 }
 
+// The launch's arguments for the FP64 matrix-instruction kernels.
+Form64 form64_args(const FormIO& io, const FormPtrs<double>& fp) {
+  Form64 f;
+  f.form_box = io.form_box;
+  f.s_lo = io.s_lo;
+  f.s_hi = io.s_hi;
+  f.order = io.order;
+  f.items = io.items;
+  f.n_items = io.n_items;
+  f.item_off = io.item_off;
+  f.n_form = io.n_form;
+  f.ns = io.ns;
+  f.nd = io.nd;
+  f.ncomp = io.ncomp;
+  f.has_q = io.has_q;
+  f.off = fp.off;
+  f.q = fp.q;
+  f.ds = fp.ds;
+  f.rn = fp.rn;
+  f.mp = fp.mp;
+  return f;
+}
+
 template <typename T, int DIM, int W>
 int launch_form(PWArgs<T>& a, const FormIO& io, const FormPtrs<T>& fp, DBuf<T>& gs, cudaStream_t s) {
   if constexpr (std::is_same<T, double>::value && DIM == 3) {
     if (io.f64) {
-      Form64 f;
-      f.form_box = io.form_box;
-      f.s_lo = io.s_lo;
-      f.s_hi = io.s_hi;
-      f.order = io.order;
-      f.items = io.items;
-      f.n_items = io.n_items;
-      f.item_off = io.item_off;
-      f.n_form = io.n_form;
-      f.ns = io.ns;
-      f.nd = io.nd;
-      f.ncomp = io.ncomp;
-      f.has_q = io.has_q;
-      f.off = fp.off;
-      f.q = fp.q;
-      f.ds = fp.ds;
-      f.rn = fp.rn;
-      f.mp = fp.mp;
-      return form64_launch(W, &a, f, s);
+      return form64_launch(W, &a, form64_args(io, fp), s);
     }
   }
   size_t fix = fixed_smem(a, W, 1);
@@ -827,6 +832,10 @@ void launch_form_small2(PWArgs<T>& a, const FormIO& io, const FormPtrs<T>& fp,
 template <typename T>
 void form_small2_w(int w, PWArgs<T>& a, const FormIO& io, const FormPtrs<T>& fp,
                    const uint32_t* order, const int* first, int* next, cudaStream_t s) {
+  if constexpr (std::is_same<T, double>::value) {
+    if (small2d64_takes(w, a.g.K, a.g.G, a.g.wrap))
+      return form2d64_launch(w, &a, form64_args(io, fp), first, next, s);
+  }
   switch (w) {
     case 6: return launch_form_small2<T, 6>(a, io, fp, order, first, next, s);
     case 8: return launch_form_small2<T, 8>(a, io, fp, order, first, next, s);

@@ -49,4 +49,12 @@ int form64_launch(int w, const void* a, const Form64& io, cudaStream_t s);
 bool modal64_launch(const void* a, const Eval64& io, int pmax, size_t smem, cudaStream_t s);
 int eval64_launch(int w, bool deriv, const void* a, const Eval64& io, cudaStream_t s);
 
+// Small 2D boxes (fgt_pw64_2d.cu): the boxes from *first on of the order, one
+// warp per (box, density); next: work counter, zero.
+bool small2d64_takes(int w, int K, int G, bool wrap);
+void form2d64_launch(int w, const void* a, const Form64& io, const int* first, int* next,
+                     cudaStream_t s);
+void eval2d64_launch(int w, bool deriv, const void* a, const Eval64& io, const int* first,
+                     int* next, cudaStream_t s);
+
 }  // namespace fgt

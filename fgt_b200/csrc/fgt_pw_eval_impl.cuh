@@ -1015,6 +1015,10 @@ void launch_eval_small2(PWArgs<T>& a, const EvalPtrs<T>& ep, const int* first, i
 template <typename T>
 void eval_small2_w(int w, bool deriv, PWArgs<T>& a, const EvalPtrs<T>& ep, const int* first,
                    int* next, cudaStream_t s) {
+  if constexpr (std::is_same<T, double>::value) {
+    if (small2d64_takes(w, a.g.K, a.g.G, a.g.wrap))
+      return eval2d64_launch(w, deriv, &a, eval64_args(ep), first, next, s);
+  }
 #define FGT_S2(WW)                                                              \
   case WW:                                                                      \
     if (deriv) launch_eval_small2<T, WW, true>(a, ep, first, next, s);          \

@@ -57,6 +57,39 @@ def test_matrix_kernels_match_oracle(fgt, oracle, eps, pgh, nd, dip, big):
                 assert relerr(ro[f], r[f]) <= 0.3 * eps, (f, relerr(ro[f], r[f]))
 
 
+@pytest.mark.parametrize("eps,pgh,nd,dip,period", [
+    (1e-3, 1, 1, False, 0),
+    (1e-3, 2, 2, False, 1),
+    (1e-6, 2, 1, True, 0),
+    (1e-8, 1, 3, False, 0),
+    (1e-9, 2, 2, False, 0),
+    (1e-10, 1, 1, False, 1),
+    (1e-12, 2, 1, True, 0),
+    (1e-13, 1, 1, False, 0),
+])
+def test_2d_matrix_kernels_match_oracle(fgt, oracle, eps, pgh, nd, dip, period):
+    """Small 2D boxes: groups of 81 to 2,049 points (the last beyond the
+    warp-per-box kernels), counts off the batches of 16 and steps of 4."""
+    rng = np.random.default_rng(6)
+    groups = [rng.uniform(-0.4, 0.4, 2) + rng.uniform(-5e-3, 5e-3, (n, 2))
+              for n in (81, 82, 96, 97, 100, 2048, 2049)]
+    src = np.concatenate(groups + [rng.uniform(-0.5, 0.5, (700, 2))])
+    trg = rng.uniform(-0.5, 0.5, (333, 2))
+    n = src.shape[0]
+    kw = dict(nd=nd, dim=2, delta=2e-3, eps=eps, iperiod=period, sources=src, bs0=1.0,
+              cen0=[0.0, 0.0], charge=rng.standard_normal((n, nd)), ifpgh=pgh, targets=trg,
+              ifpghtarg=pgh)
+    if dip:
+        kw.update(dipstr=rng.standard_normal((n, nd)), rnormal=rng.standard_normal((n, 2)))
+    ro = oracle.pfgt(**kw)
+    for small_eval in (-1, 0):
+        r = fgt.pfgt(precision=fgt.PREC_FP64, small_eval=small_eval, stats=True, **kw)
+        assert r["stats"]["n_form_boxes"] > 0
+        for f in FIELDS:
+            if f in ro:
+                assert relerr(ro[f], r[f]) <= 0.3 * eps, (f, relerr(ro[f], r[f]))
+
+
 def test_several_runs_over_the_boxes(fgt, monkeypatch):
     """Grids of a few boxes held at a time give the sums of all at once (equal
     but for the order of the atomics)."""

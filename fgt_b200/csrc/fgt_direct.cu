@@ -970,28 +970,42 @@ __global__ void __launch_bounds__(DW * 32) k_direct32x2p(DArgs<float> a, const i
   }
 }
 
-__global__ void k_items_count(int nboxes, const int* __restrict__ l1_ptr, const int* __restrict__ lo,
-                              const int* __restrict__ hi, const int* __restrict__ s_lo,
-                              const int* __restrict__ s_hi, const int* __restrict__ l1_src,
-                              int tpi, int* __restrict__ cnt, double* __restrict__ pairs) {
-  for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nboxes; b += gridDim.x * blockDim.x) {
-    int ne = hi[b] - lo[b], nl = l1_ptr[b + 1] - l1_ptr[b];
-    cnt[b] = (ne > 0 && nl > 0) ? (ne + tpi - 1) / tpi : 0;
-    if (pairs && ne > 0 && nl > 0) {
-      double ns = 0;
-      for (int i = l1_ptr[b]; i < l1_ptr[b + 1]; i++) ns += s_hi[l1_src[i]] - s_lo[l1_src[i]];
-      atomicAdd(pairs, ns * ne);
+// Near-field items: up to tpi points of one box each.  A warp takes the items
+// of its 32 boxes from the counter at once; the items' order does not matter.
+__global__ void k_items(int nboxes, const int* __restrict__ l1_ptr, const int* __restrict__ lo,
+                        const int* __restrict__ hi, const int* __restrict__ s_lo,
+                        const int* __restrict__ s_hi, const int* __restrict__ l1_src, int tpi,
+                        int max_items, int* __restrict__ n_items, int* __restrict__ ibox,
+                        int* __restrict__ ilo, double* __restrict__ pairs) {
+  const int lane = threadIdx.x & 31;
+  for (int b0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31); b0 < nboxes;
+       b0 += gridDim.x * blockDim.x) {
+    const int b = b0 + lane;
+    int c = 0;
+    if (b < nboxes) {
+      const int ne = hi[b] - lo[b], nl = l1_ptr[b + 1] - l1_ptr[b];
+      c = (ne > 0 && nl > 0) ? (ne + tpi - 1) / tpi : 0;
+      if (pairs && c > 0) {
+        double ns = 0;
+        for (int i = l1_ptr[b]; i < l1_ptr[b + 1]; i++) ns += s_hi[l1_src[i]] - s_lo[l1_src[i]];
+        atomicAdd(pairs, ns * ne);
+      }
+    }
+    int inc = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += u;
+    }
+    int base = 0;
+    if (lane == 31 && inc) base = atomicAdd(n_items, inc);
+    base = __shfl_sync(0xffffffffu, base, 31) + inc - c;
+    for (int k = 0; k < c; k++) {
+      if (!FGT_DCHECK(base + k < max_items, 404)) break;
+      ibox[base + k] = b;
+      ilo[base + k] = lo[b] + tpi * k;
     }
   }
-}
-__global__ void k_items_fill(int nboxes, int tpi, const int* __restrict__ cnt,
-                             const int* __restrict__ pos, const int* __restrict__ lo,
-                             int* __restrict__ ibox, int* __restrict__ ilo) {
-  for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nboxes; b += gridDim.x * blockDim.x)
-    for (int c = 0; c < cnt[b]; c++) {
-      ibox[pos[b] + c] = b;
-      ilo[pos[b] + c] = lo[b] + tpi * c;
-    }
 }
 
 template <typename T, int DIM, int PGH, bool CHG, bool DIP, int NDC>
@@ -1062,8 +1076,8 @@ long long near_lists_count(const DirectGeom& g, const Lists& L, const int* s_lo,
   if (L.n_l1 <= 0) return -1;
   NearArgs n = near_args(g, L, s_lo, s_hi, t_lo, t_hi, soff, ns);
   DBuf<int> cnt(L.n_l1, s);
-  DBuf<unsigned long long> tot(1, s);
-  tot.zero();
+  DBuf<unsigned long long> tot;
+  tot.alloc_zeroed(1, s);
   n.cnt = cnt;
   n.total = tot;
   launch_near_lists<float, false>(g.dim, n, s);
@@ -1076,13 +1090,44 @@ long long near_lists_count(const DirectGeom& g, const Lists& L, const int* s_lo,
   return (long long)h;
 }
 
+namespace {
+struct PinnedInt {
+  int* p = nullptr;
+  bool queued = false;
+  ~PinnedInt() {
+    if (p) cudaFreeHost(p);
+  }
+};
+PinnedInt& near_status_buf() {
+  static thread_local PinnedInt b;
+  return b;
+}
+}  // namespace
+
+void near_status_fetch(cudaStream_t s) {
+  if (!t_packed_launched) return;
+  PinnedInt& b = near_status_buf();
+  if (!b.p) FGT_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&b.p), sizeof(int), cudaHostAllocPortable));
+  FGT_CUDA(cudaMemcpyFromSymbolAsync(b.p, g_near_status, sizeof(int), 0, cudaMemcpyDeviceToHost, s));
+  b.queued = true;
+}
+
 int near_wait_status(cudaStream_t s) {
   if (!t_packed_launched) return FGT_OK;
   t_packed_launched = false;
+  PinnedInt& b = near_status_buf();
   int v = 0, z = 0;
-  FGT_CUDA(cudaMemcpyFromSymbolAsync(&v, g_near_status, sizeof(v), 0, cudaMemcpyDeviceToHost, s));
-  FGT_CUDA(cudaStreamSynchronize(s));
-  if (v) FGT_CUDA(cudaMemcpyToSymbolAsync(g_near_status, &z, sizeof(z), 0, cudaMemcpyHostToDevice, s));
+  if (b.queued) {
+    v = *b.p;
+  } else {
+    FGT_CUDA(cudaMemcpyFromSymbolAsync(&v, g_near_status, sizeof(v), 0, cudaMemcpyDeviceToHost, s));
+    FGT_CUDA(cudaStreamSynchronize(s));
+  }
+  b.queued = false;
+  if (v) {
+    FGT_CUDA(cudaMemcpyToSymbolAsync(g_near_status, &z, sizeof(z), 0, cudaMemcpyHostToDevice, s));
+    FGT_CUDA(cudaStreamSynchronize(s));
+  }
   return v;
 }
 
@@ -1147,26 +1192,21 @@ int direct_near_field(const DirectGeom& g, const Lists& L, const SourceSet<T>& s
   // two evaluation points per lane: FP32, charges only, pot or pot + grad, one density
   const bool paired = sizeof(T) == 4 && chg && !dip && e.pgh <= 2 && g.nd == 1;
   const int tpi = paired ? 64 : 32;
-  DBuf<int> cnt(nb, s), pos(nb, s), tot(1, s);
-  DBuf<double> dpairs(1, s);
-  dpairs.zero();
-  k_items_count<<<grid_for(nb, 128), 128, 0, s>>>(nb, L.l1_ptr, e.lo, e.hi, src.lo, src.hi,
-                                                   L.l1_src, tpi, cnt,
-                                                   pairs ? dpairs.get() : nullptr);
+  // the item count stays on the device: sum_b ceil(ne_b / tpi) <= ne / tpi + nboxes
+  const int n_items = (int)std::min<long long>((long long)e.n / tpi + nb + 1, INT32_MAX);
+  DBuf<int> ibox(n_items, s), ilo(n_items, s), tot;
+  DBuf<double> dpairs;
+  tot.alloc_zeroed(1, s);
+  dpairs.alloc_zeroed(1, s);
+  k_items<<<grid_for(nb, 128), 128, 0, s>>>(nb, L.l1_ptr, e.lo, e.hi, src.lo, src.hi, L.l1_src, tpi,
+                                             n_items, tot, ibox, ilo, pairs ? dpairs.get() : nullptr);
   FGT_LAUNCH_CHECK();
-  exclusive_scan_i32(cnt, pos, nb, tot, s);
   if (pairs) {  // statistics only: the one read-back of this function
     double h = 0;
     FGT_CUDA(cudaMemcpyAsync(&h, dpairs.get(), sizeof(double), cudaMemcpyDeviceToHost, s));
     FGT_CUDA(cudaStreamSynchronize(s));
     *pairs += h;
   }
-  launches += 2;
-  // the item count stays on the device: sum_b ceil(ne_b / tpi) <= ne / tpi + nboxes
-  const int n_items = (int)std::min<long long>((long long)e.n / tpi + nb + 1, INT32_MAX);
-  DBuf<int> ibox(n_items, s), ilo(n_items, s);
-  k_items_fill<<<grid_for(nb, 128), 128, 0, s>>>(nb, tpi, cnt, pos, e.lo, ibox, ilo);
-  FGT_LAUNCH_CHECK();
   launches++;
   DArgs<T> a;
   a.n_items = n_items;
@@ -1199,8 +1239,8 @@ int direct_near_field(const DirectGeom& g, const Lists& L, const SourceSet<T>& s
   if constexpr (sizeof(T) == 8) {
     if (packed && packed->rec && chg && !dip && e.pgh <= 2 && g.nd == 1) {
       a.d0 = 0;
-      DBuf<int> next(1, s);
-      next.zero();
+      DBuf<int> next;
+      next.alloc_zeroed(1, s);
       auto go = [&](auto kern) {
         kern<<<std::max(1, std::min(ceil_div(n_items, DW), kSMs * 8)), DW * 32, 0, s>>>(
             a, packed->pos, static_cast<const double2*>(packed->rec), next);
@@ -1215,8 +1255,8 @@ int direct_near_field(const DirectGeom& g, const Lists& L, const SourceSet<T>& s
   if constexpr (sizeof(T) == 4) {
     if (paired && packed && packed->rec) {
       a.d0 = 0;
-      DBuf<int> next(1, s);
-      next.zero();
+      DBuf<int> next;
+      next.alloc_zeroed(1, s);
       const DArgs<float>& af = a;
       if (g.dim == 1) {
         if (e.pgh == 1) launch_packed<1, 1>(af, *packed, next, s);

@@ -61,6 +61,9 @@ void near_lists_fill(const DirectGeom& g, const Lists& L, const SourceSet<T>& sr
 // read: FGT_OK, or FGT_ERR_TIMEOUT when a wait ran out (the kernel stopped
 // early and the results are incomplete).  Clears it; synchronises the stream.
 int near_wait_status(cudaStream_t s);
+// Queues the status's copy to the host before a call's last synchronisation,
+// which then covers it.
+void near_status_fetch(cudaStream_t s);
 
 // Adds the list-1 interactions onto every point of `e`.  Returns the number
 // of kernel launches; *pairs receives the near-field pair count if not null.

@@ -113,7 +113,24 @@ void* Arena::alloc(size_t bytes) {
   return p;
 }
 
+void* Arena::alloc_zeroed(size_t bytes, cudaStream_t s) {
+  bytes = (bytes + 15) & ~size_t(15);
+  if (bytes > zero_left) {
+    constexpr size_t kBlock = 4096;
+    const size_t want = std::max(bytes, kBlock);
+    zero_p = static_cast<char*>(alloc(want));
+    zero_left = want;
+    FGT_CUDA(cudaMemsetAsync(zero_p, 0, want, s));
+  }
+  char* p = zero_p;
+  zero_p += bytes;
+  zero_left -= bytes;
+  return p;
+}
+
 void Arena::reset(cudaStream_t s) {
+  zero_p = nullptr;
+  zero_left = 0;
   if (chunks.size() > 1) {
     // consolidate into one chunk of the high-water size for the next call
     cudaStreamSynchronize(s);
@@ -136,11 +153,15 @@ std::vector<size_t> Arena::mark() const {
 }
 
 void Arena::rewind(const std::vector<size_t>& m) {
+  zero_p = nullptr;  // may lie past the mark
+  zero_left = 0;
   for (size_t i = 0; i < chunks.size(); i++) chunks[i].off = i + 1 < m.size() ? m[i] : 0;
   used = m.empty() ? 0 : m.back();
 }
 
 void Arena::release_all() {
+  zero_p = nullptr;
+  zero_left = 0;
   for (auto& c : chunks) cudaFree(c.p);
   chunks.clear();
   used = high = 0;
@@ -168,6 +189,8 @@ namespace {
 constexpr int SCAN_THREADS = 256;
 constexpr int SCAN_ITEMS = 4;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
+constexpr int SCAN_ONE = 16384;   // one block up to here
+constexpr int SCAN_TWO = 1 << 21; // two launches up to here (2,048 block sums)
 
 __device__ __forceinline__ int warp_incl_scan(int v) {
   int lane = threadIdx.x & 31;
@@ -227,6 +250,55 @@ __global__ void k_scan_apply(const int* in, int* out, int n, const int* __restri
     ex += v[j];
   }
   if (total && blockIdx.x == nblocks - 1 && threadIdx.x == SCAN_THREADS - 1) *total = ex;
+}
+
+// Scan of up to SCAN_ONE values by one block: a contiguous run per thread.
+__global__ void __launch_bounds__(1024) k_scan_one(const int* in, int* out, int n, int* total) {
+  constexpr int PER = SCAN_ONE / 1024;
+  __shared__ int ws[32];
+  const int per = (n + 1023) / 1024, b = threadIdx.x * per;
+  int v[PER], s = 0;
+#pragma unroll
+  for (int j = 0; j < PER; j++) {
+    v[j] = j < per && b + j < n ? in[b + j] : 0;
+    s += v[j];
+  }
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int inc = warp_incl_scan(s);
+  if (lane == 31) ws[w] = inc;
+  __syncthreads();
+  const int before = warp_incl_scan(ws[lane]) - ws[lane];
+  int ex = inc - s + __shfl_sync(0xffffffffu, before, w);
+#pragma unroll
+  for (int j = 0; j < PER; j++) {
+    if (j < per && b + j < n) out[b + j] = ex;
+    ex += v[j];
+  }
+  if (total && threadIdx.x == 1023) *total = ex;
+}
+
+// Second launch of a scan in two: every block adds the block sums before it.
+__global__ void __launch_bounds__(SCAN_THREADS)
+    k_scan_add(const int* in, int* out, int n, const int* __restrict__ part, int* total, int nblocks) {
+  int before = 0;
+  for (int i = threadIdx.x; i < (int)blockIdx.x; i += SCAN_THREADS) before += part[i];
+  int all;
+  block_excl_scan(before, &all);
+  const int base = blockIdx.x * SCAN_TILE;
+  int v[SCAN_ITEMS], s = 0;
+  for (int j = 0; j < SCAN_ITEMS; j++) {
+    const int i = base + threadIdx.x * SCAN_ITEMS + j;
+    v[j] = i < n ? in[i] : 0;
+    s += v[j];
+  }
+  int tot;
+  int ex = block_excl_scan(s, &tot) + all;
+  for (int j = 0; j < SCAN_ITEMS; j++) {
+    const int i = base + threadIdx.x * SCAN_ITEMS + j;
+    if (i < n) out[i] = ex;
+    ex += v[j];
+  }
+  if (total && (int)blockIdx.x == nblocks - 1 && threadIdx.x == SCAN_THREADS - 1) *total = ex;
 }
 
 // ---------------------------------------------------------------- radix sort
@@ -449,6 +521,20 @@ __global__ void k_unique_scatter(const uint64_t* __restrict__ a, int n, const in
 void exclusive_scan_i32(const int* in, int* out, int n, int* total, cudaStream_t s) {
   if (n <= 0) {
     if (total) FGT_CUDA(cudaMemsetAsync(total, 0, sizeof(int), s));
+    return;
+  }
+  if (n <= SCAN_ONE) {
+    k_scan_one<<<1, 1024, 0, s>>>(in, out, n, total);
+    FGT_LAUNCH_CHECK();
+    return;
+  }
+  if (n <= SCAN_TWO) {
+    const int nb = ceil_div(n, SCAN_TILE);
+    DBuf<int> part(nb, s);
+    k_scan_reduce<<<nb, SCAN_THREADS, 0, s>>>(in, n, part);
+    FGT_LAUNCH_CHECK();
+    k_scan_add<<<nb, SCAN_THREADS, 0, s>>>(in, out, n, part, total, nb);
+    FGT_LAUNCH_CHECK();
     return;
   }
   int nb = ceil_div(n, SCAN_TILE);

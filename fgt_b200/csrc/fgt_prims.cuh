@@ -19,7 +19,11 @@ struct Arena {
   };
   std::vector<Chunk> chunks;
   size_t used = 0, high = 0;
+  // zeroed bytes for small counters, cleared in blocks (one memset for many)
+  char* zero_p = nullptr;
+  size_t zero_left = 0;
   void* alloc(size_t bytes);
+  void* alloc_zeroed(size_t bytes, cudaStream_t s);
   void reset(cudaStream_t s);  // call end: all allocations are dead
   void release_all();
   // Allocation state, and a return to it: buffers allocated after the mark
@@ -70,6 +74,13 @@ struct DBuf {
     n = count;
     size_t bytes = (count ? count : 1) * sizeof(T);
     p = (T*)thread_arena()->alloc(bytes);
+  }
+  // a small zeroed buffer (counters)
+  void alloc_zeroed(size_t count, cudaStream_t st) {
+    release();
+    s = st;
+    n = count;
+    p = (T*)thread_arena()->alloc_zeroed((count ? count : 1) * sizeof(T), st);
   }
   void zero() {
     if (p) FGT_CUDA(cudaMemsetAsync(p, 0, (n ? n : 1) * sizeof(T), s));

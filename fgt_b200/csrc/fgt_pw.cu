@@ -1001,8 +1001,8 @@ int pw_form(const PWParams& P, const Tree& t, const Lists& L, const SourceSet<T>
   // split threshold are cut into parts of about thr sources.
   DBuf<uint64_t> okey(std::max(L.n_form, 1), s), otmp(std::max(L.n_form, 1), s);
   DBuf<uint32_t> oval(std::max(L.n_form, 1), s), vtmp(std::max(L.n_form, 1), s);
-  DBuf<int> next(1, s);
-  next.zero();
+  DBuf<int> next;
+  next.alloc_zeroed(1, s);
   if (L.n_form > 0) {
     k_lpt_keys<<<grid_for(L.n_form, 256), 256, 0, s>>>(L.n_form, nullptr, L.form_box, nullptr,
                                                        src.lo, src.hi, nullptr, nullptr, okey,
@@ -1015,9 +1015,9 @@ int pw_form(const PWParams& P, const Tree& t, const Lists& L, const SourceSet<T>
   // the warp-per-box kernel, the rest to the CTA kernel
   size_t sm2 = 0;
   const bool small2 = P.dim == 2 && !a.g.wrap && small2_warps<T>(a.g, sm2) > 0;
-  DBuf<int> first(1, s), next2(1, s);
+  DBuf<int> first(1, s), next2;
+  next2.alloc_zeroed(1, s);
   if (small2) {
-    next2.zero();
     k_first_at_most<<<1, 32, 0, s>>>(okey, L.n_form, SMALL2_MAX, first);
     FGT_LAUNCH_CHECK();
   }

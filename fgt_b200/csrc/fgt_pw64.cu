@@ -1062,8 +1062,8 @@ static int launch_form64(const PWArgs<double>& a, const Form64& io, cudaStream_t
   const Lay64 lay(G, K);
   const int held = grids_held(lay, G, io.n_form), runs = ceil_div(io.n_form, held) * io.nd * io.ncomp;
   DBuf<double> grids((size_t)held * lay.grid(G), s);
-  DBuf<int> next(runs, s);
-  next.zero();
+  DBuf<int> next;
+  next.alloc_zeroed(runs, s);
   Es64 es;
   es_polys(W, a, es);
   set_smem(k_spread64<W>, sizeof(FormSmem64));
@@ -1113,8 +1113,8 @@ static int launch_eval64(const PWArgs<double>& a, const Eval64& io, cudaStream_t
   const int nc = DERIV ? 1 : io.ncomp_max, held = grids_held(lay, G, io.nbox);
   const int runs = ceil_div(io.nbox, held) * io.nd * nc;
   DBuf<double> grids((size_t)held * lay.grid(G), s);
-  DBuf<int> next(runs, s);
-  next.zero();
+  DBuf<int> next;
+  next.alloc_zeroed(runs, s);
   const size_t sm = sizeof(EvalSmem64<W, DERIV>);
   static_assert(sizeof(EvalSmem64<W, DERIV>) <= MAXSMEM, "shared memory of a CTA");
   Es64 es;

@@ -1067,8 +1067,7 @@ inline void build_items(ItemList& il, int n, const int* count, const uint32_t* o
   il.items.alloc(std::max(il.max_items, 1), s);
   il.n_items.alloc(1, s);
   il.n_partial.alloc(1, s);
-  il.n_split.alloc(1, s);
-  il.n_split.zero();
+  il.n_split.alloc_zeroed(1, s);
   if (want_split) il.split.alloc(std::max(il.max_partial, 1), s);
   if (n <= 0) {
     il.n_items.zero();

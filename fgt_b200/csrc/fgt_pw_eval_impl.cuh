@@ -1109,8 +1109,8 @@ int pw_eval(const PWParams& P, const Tree& t, const Lists& L, const PWData<T>& D
   const int thr = std::min(small_eval >= 0 ? small_eval : (P.dim == 3 ? 48 : (P.dim == 2 ? 8 : 4)),
                            (int)((MAXSMEM - modal_fix) / modal_pt));
   DBuf<int> big(L.n_eval, s), pos(L.n_eval, s), tot(1, s);
-  DBuf<unsigned long long> cnt(2, s);
-  cnt.zero();
+  DBuf<unsigned long long> cnt;
+  cnt.alloc_zeroed(2, s);
   k_eval_split<<<grid_for(L.n_eval, 256), 256, 0, s>>>(
       L.n_eval, L.eval_box, u0 ? e0.lo : nullptr, u0 ? e0.hi : nullptr, u1 ? e1.lo : nullptr,
       u1 ? e1.hi : nullptr, thr, big, cnt);
@@ -1156,14 +1156,15 @@ int pw_eval(const PWParams& P, const Tree& t, const Lists& L, const PWData<T>& D
   ep.nslab = sp.nslab;
   if (work) work->slabs_eval = ep.e64 && beyond ? ceil_div(Pe.G, SLAB64) : sp.nslab;
   ItemList il;
-  DBuf<int> first2(1, s), next2(1, s);
+  DBuf<int> first2(1, s), next2;
+  next2.alloc_zeroed(1, s);
   DBuf<T> gs;
   {
     // longest-processing-time order of the grid boxes (by point count)
     DBuf<uint64_t> okey(L.n_eval, s), otmp(L.n_eval, s);
     DBuf<uint32_t> vtmp(L.n_eval, s);
-    DBuf<int> next(1, s);
-    next.zero();
+    DBuf<int> next;
+    next.alloc_zeroed(1, s);
     k_lpt_keys<<<grid_for(L.n_eval, 256), 256, 0, s>>>(
         L.n_eval, counts.get(), L.eval_box, lbig, u0 ? e0.lo : e1.lo, u0 ? e0.hi : e1.hi,
         (u0 && u1) ? e1.lo : nullptr, (u0 && u1) ? e1.hi : nullptr, okey,
@@ -1180,7 +1181,6 @@ int pw_eval(const PWParams& P, const Tree& t, const Lists& L, const PWData<T>& D
     const bool small2 = P.dim == 2 && !a.g.wrap && (deriv || ep.ncomp_max == 1) &&
                         small2_eval_warps<T>(a.g, sm2) > 0;
     if (small2) {
-      next2.zero();
       k_first_at_most_e<<<1, 32, 0, s>>>(okey, L.n_eval, SMALL2_MAX, first2);
       FGT_LAUNCH_CHECK();
     }

@@ -288,6 +288,59 @@ void launch_trans(const TV& tv, const int* eval_box, int n_eval, const int* form
   else go(k_trans<3, FILL>);
 }
 
+// Sibling groups of the translation: one warp per parent of cut-off-level
+// boxes, one of the 4^DIM positions around the children per lane.
+template <int DIM>
+__global__ void k_groups(TV tv, int n_grp, const int* __restrict__ form_slot,
+                         const int* __restrict__ eval_flag, const int* __restrict__ eval_pos,
+                         int* __restrict__ gsrc, int* __restrict__ gtrg) {
+  constexpr int NP = 1 << (2 * DIM), MC = 1 << DIM;
+  const int l = tv.ncutoff, lo = tv.lev_start[l];
+  const int lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
+  for (int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < n_grp; g += nw) {
+    const int c0 = lo + g * MC;  // the group's first child
+    const bool ev = lane < MC && eval_flag[g * MC + lane];
+    if (lane < MC) gtrg[g * MC + lane] = ev ? eval_pos[g * MC + lane] : -1;
+    const unsigned em = __ballot_sync(0xffffffffu, ev);
+    uint32_t c[DIM];
+    coords_of_d<DIM>(tv, c0, c);  // even coordinates
+    const long long n = 1ll << l;
+    int cnt = 0;
+    for (int p0 = 0; p0 < NP; p0 += 32) {
+      const int p = p0 + lane;
+      uint32_t q[DIM];
+      bool in = p < NP;
+#pragma unroll
+      for (int k = 0; k < DIM; k++) {
+        long long x = (long long)c[k] - 1 + ((p >> (2 * k)) & 3);
+        if (tv.iperiod0 == 1) x = ((x % n) + n) % n;
+        in = in && x >= 0 && x < n;
+        q[k] = (uint32_t)x;
+      }
+      bool used = false;  // by one of the group's targets
+#pragma unroll
+      for (int j = 0; j < MC; j++) {
+        bool near = (em >> j) & 1;
+#pragma unroll
+        for (int k = 0; k < DIM; k++)
+          near = near && abs(1 + ((j >> k) & 1) - ((p >> (2 * k)) & 3)) <= 1;
+        used = used || near;
+      }
+      in = in && used;
+      const int b = in ? find_box_d<DIM>(tv, l, q) : -1;
+      const int sl = b >= 0 ? form_slot[b - lo] : -1;
+      if (DIM < 3) {
+        if (p < NP) gsrc[(size_t)g * NP + p] = sl;
+      } else {
+        const unsigned m = __ballot_sync(0xffffffffu, sl >= 0);
+        if (sl >= 0) gsrc[(size_t)g * NP + cnt + __popc(m & ((1u << lane) - 1u))] = sl * 64 + p;
+        cnt += __popc(m);
+      }
+    }
+    if (DIM == 3 && lane == 0 && cnt < NP) gsrc[(size_t)g * NP + cnt] = -1;
+  }
+}
+
 TV make_tv(const Tree& t, int npwlevel, int iperiod0, int nlevend) {
   TV tv;
   tv.dim = t.dim;
@@ -375,6 +428,20 @@ void build_lists(const Tree& t, int npwlevel, int iperiod0, int nlevend, bool do
     k_eval_self<<<grid_for(L.n_eval, 256), 256, 0, s>>>(L.n_eval, L.eval_box, fslot, lo,
                                                          L.eval_self);
     FGT_LAUNCH_CHECK();
+  }
+  // levels of two boxes a side and up: no position around a group repeats
+  if (t.ncutoff >= 1 && (iperiod0 != 1 || t.ncutoff >= 2) && L.n_eval > 0 && L.n_form < (1 << 25)) {
+    L.n_grp = n / t.mc;
+    L.grp_src.alloc((size_t)L.n_grp << (2 * t.dim), s);
+    L.grp_trg.alloc((size_t)L.n_grp * t.mc, s);
+    const int grid = grid_for((long long)L.n_grp * 32, 256);
+    auto go = [&](auto kern) {
+      kern<<<grid, 256, 0, s>>>(tv, L.n_grp, fslot, fe, pe, L.grp_src, L.grp_trg);
+      FGT_LAUNCH_CHECK();
+    };
+    if (t.dim == 1) go(k_groups<1>);
+    else if (t.dim == 2) go(k_groups<2>);
+    else go(k_groups<3>);
   }
   L.trans_ptr.alloc(L.n_eval + 1, s);
   {

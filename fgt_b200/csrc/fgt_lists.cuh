@@ -14,6 +14,12 @@ struct Lists {
   DBuf<int> trans_ptr;   // per eval box: CSR offsets into trans_src/trans_w (n_eval+1)
   DBuf<int> trans_src;   // form slot of the source expansion
   DBuf<int> trans_w;     // shift-table index 0..3^dim-1
+  // translation by sibling groups: the 2^dim children of one parent at the
+  // cut-off level, their eval slots (-1: none) and the form slots (-1: none)
+  // of the 4^dim boxes around them, first coordinate fastest; in 3D only those
+  // present, as slot * 64 + position, closed by a -1 where there are fewer
+  int n_grp = 0;
+  DBuf<int> grp_src, grp_trg;
   // direct part: CSR over all boxes (targets), sources are box ids
   DBuf<int> l1_ptr, l1_src;
   DBuf<int> l1_trg;  // target box of every list entry

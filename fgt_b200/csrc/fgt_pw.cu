@@ -688,6 +688,254 @@ __global__ void k_translate(int n_eval, int n_form, int nsh, int nexp, int nd, i
   }
 }
 
+// The same sums by sibling groups: a thread holds one mode's 3^DIM shift
+// factors in registers and, for every group, the sums of its 2^DIM children;
+// each of the 4^DIM expansions around them is read once for all of them
+// instead of once per child, and the factors once for many groups.  In 1D and
+// 2D row by row with the next row in flight.  A child's own
+// expansion comes first, then its neighbours with the first coordinate
+// fastest: the order of its list.  With the roundings written out (left to
+// the compiler, they change with the code around them) the FP32 sums are
+// k_translate's bit for bit.
+__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+template <typename T, int DIM>
+__global__ void __launch_bounds__(128)
+    k_translate_groups(int n_grp, int n_form, int nexp, int nd, const int* __restrict__ gsrc,
+                       const int* __restrict__ gtrg, const T* __restrict__ mp,
+                       const T* __restrict__ wtab, T* __restrict__ loc) {
+  using V = typename std::conditional<sizeof(T) == 4, float2, double2>::type;
+  constexpr int MC = 1 << DIM, NP = 1 << (2 * DIM), NW = DIM == 3 ? 27 : (DIM == 2 ? 9 : 3);
+  constexpr int ROWS = NP / 4;
+  const V* mpv = reinterpret_cast<const V*>(mp);
+  V* lv = reinterpret_cast<V*>(loc);
+  const int m = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool ok = m < nexp;
+  V w[NW];
+#pragma unroll
+  for (int i = 0; i < NW; i++)
+    w[i] = reinterpret_cast<const V*>(wtab)[(size_t)i * nexp + (ok ? m : 0)];
+  for (int g = blockIdx.y; g < n_grp; g += gridDim.y) {
+    int et[MC];
+    bool any = false;
+#pragma unroll
+    for (int c = 0; c < MC; c++) {
+      et[c] = gtrg[(size_t)g * MC + c];
+      any = any || et[c] >= 0;
+    }
+    if (!any) continue;
+    const int* gs = gsrc + (size_t)g * NP;
+    for (int id = 0; id < nd; id++) {
+      auto load = [&](int p) {
+        const int sl = gs[p];
+        V v;
+        v.x = v.y = T(0);
+        if (sl >= 0 && ok && FGT_DCHECK(sl < n_form, 205))
+          v = __ldg(mpv + ((size_t)sl * nd + id) * nexp + m);
+        return v;
+      };
+      // position of child c: coordinate k is 1 + bit k
+      V acc[MC];
+#pragma unroll
+      for (int c = 0; c < MC; c++) {
+        int p = 0;
+#pragma unroll
+        for (int k = 0; k < DIM; k++) p |= (1 + ((c >> k) & 1)) << (2 * k);
+        acc[c] = load(p);
+      }
+      V nx[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) nx[i] = load(i);
+#pragma unroll
+      for (int r = 0; r < ROWS; r++) {
+        V cur[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          cur[i] = nx[i];
+          if (r + 1 < ROWS) nx[i] = load(4 * (r + 1) + i);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const int p = 4 * r + i;
+#pragma unroll
+          for (int c = 0; c < MC; c++) {
+            // shift index: sum_k (target - source + 1) 3^k
+            int ind = 0, inc = 1;
+            bool near = true, self = true;
+#pragma unroll
+            for (int k = 0; k < DIM; k++) {
+              const int d = 1 + ((c >> k) & 1) - ((p >> (2 * k)) & 3);
+              near = near && d >= -1 && d <= 1;
+              self = self && d == 0;
+              ind += (d + 1) * inc;
+              inc *= 3;
+            }
+            if (near && !self) {
+              const V a = cur[i], q = w[near ? ind : 0];
+              acc[c].x = add_rn(acc[c].x, fma(a.x, q.x, mul_rn(-a.y, q.y)));
+              acc[c].y = add_rn(acc[c].y, fma(a.x, q.y, mul_rn(a.y, q.x)));
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < MC; c++)
+        if (et[c] >= 0 && ok) lv[((size_t)et[c] * nd + id) * nexp + m] = acc[c];
+    }
+  }
+}
+
+// In 3D the sums are nested by dimension, shift factors being products of one
+// phase per dimension: a row of four expansions gives the sums of two children
+// in x, four rows those of two in y, four planes those of two in z; 112
+// complex products for the 8 children instead of 208, and 6 factors instead of
+// 27.  Most of the 64 positions around a group on a surface are empty: only the
+// present ones are listed, and fetched ahead by asynchronous copies, TG_RING - 1
+// of them in flight per thread, which reads back only what it copied itself (no
+// barrier).  The loop over them is a real one: unrolled over the positions, the
+// code does not fit the instruction cache, and waiting for it took half of the
+// time.  Bound by issue (59% of the slots, 1.9 TB/s DRAM).  Two modes a thread
+// need 168 registers and lose as much to occupancy: 1.11 against 1.01 ms.
+constexpr int TG_RING = 8, TG_THREADS = 128;
+template <typename V>
+__device__ __forceinline__ void cfma(V& acc, const V& a, const V& w) {
+  acc.x += a.x * w.x - a.y * w.y;
+  acc.y += a.x * w.y + a.y * w.x;
+}
+template <typename V>
+__device__ __forceinline__ void cadd(V& acc, const V& a) {
+  acc.x += a.x;
+  acc.y += a.y;
+}
+// adds position p's n values to the two children that see it: child c stands
+// at position 1 + c, wp shifts by +1 (from the position before), wm by -1
+template <int N, typename V>
+__device__ __forceinline__ void tg_add(int p, V* c0, V* c1, const V* v, const V& wp, const V& wm) {
+  if (p < 2) {
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+      if (p == 0) cfma(c0[i], v[i], wp);
+      else {
+        cadd(c0[i], v[i]);
+        cfma(c1[i], v[i], wp);
+      }
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+      if (p == 3) cfma(c1[i], v[i], wm);
+      else {
+        cfma(c0[i], v[i], wm);
+        cadd(c1[i], v[i]);
+      }
+    }
+  }
+}
+template <int N, typename V>
+__device__ __forceinline__ void vzero(V* v) {
+#pragma unroll
+  for (int i = 0; i < N; i++) v[i].x = v[i].y = 0;
+}
+template <typename T, int MODES = 1>
+__global__ void __launch_bounds__(TG_THREADS, 5)
+    k_translate_groups3(int n_grp, int n_form, int nexp, int nd, const int* __restrict__ gsrc,
+                        const int* __restrict__ gtrg, const T* __restrict__ mp,
+                        const T* __restrict__ wtab, T* __restrict__ loc) {
+  using V = typename std::conditional<sizeof(T) == 4, float2, double2>::type;
+  __shared__ V ring[TG_RING][MODES][TG_THREADS];
+  const V* mpv = reinterpret_cast<const V*>(mp);
+  V* lv = reinterpret_cast<V*>(loc);
+  const int lane = threadIdx.x & 31;
+  int m[MODES];          // idle lanes read a valid mode and write none
+  V wm[MODES][3], wp[MODES][3];  // shifts by -1 and +1 along each dimension
+#pragma unroll
+  for (int k = 0; k < MODES; k++) {
+    m[k] = (blockIdx.x * MODES + k) * TG_THREADS + threadIdx.x;
+    const int mc = min(m[k], nexp - 1);
+#pragma unroll
+    for (int d = 0, inc = 1; d < 3; d++, inc *= 3) {
+      wm[k][d] = reinterpret_cast<const V*>(wtab)[(size_t)(13 - inc) * nexp + mc];
+      wp[k][d] = reinterpret_cast<const V*>(wtab)[(size_t)(13 + inc) * nexp + mc];
+    }
+  }
+  const unsigned ring0 = (unsigned)__cvta_generic_to_shared(&ring[0][0][threadIdx.x]);
+  // a run of groups: neighbours in Morton order read the same expansions
+  const int g1 = (int)((long long)n_grp * (blockIdx.y + 1) / gridDim.y);
+  for (int g = (int)((long long)n_grp * blockIdx.y / gridDim.y); g < g1; g++) {
+    const int et = lane < 8 ? gtrg[(size_t)g * 8 + lane] : -1;
+    if (!__any_sync(0xffffffffu, et >= 0)) continue;
+    const int e0 = gsrc[(size_t)g * 64 + lane], e1 = gsrc[(size_t)g * 64 + 32 + lane];
+    const unsigned end0 = __ballot_sync(0xffffffffu, e0 < 0);
+    const unsigned end1 = __ballot_sync(0xffffffffu, e1 < 0);
+    // entries past the closing one are not set
+    const int n = end0 ? __ffs(end0) - 1 : 32 + (end1 ? __ffs(end1) - 1 : 32);
+    for (int id = 0; id < nd; id++) {
+      auto issue = [&](int j) {  // entry j, or an empty group of copies
+        if (j < n) {
+          const int sl = __shfl_sync(0xffffffffu, j < 32 ? e0 : e1, j & 31) >> 6;
+          if (FGT_DCHECK(sl < n_form, 205)) {
+            const V* p = mpv + ((size_t)sl * nd + id) * nexp;
+            const unsigned dst = ring0 + (j % TG_RING) * (unsigned)(MODES * TG_THREADS * sizeof(V));
+#pragma unroll
+            for (int k = 0; k < MODES; k++)
+              asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
+                               dst + k * (unsigned)(TG_THREADS * sizeof(V))),
+                           "l"(p + min(m[k], nexp - 1)), "n"(sizeof(V))
+                           : "memory");
+          }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+      };
+#pragma unroll 1
+      for (int j = 0; j < TG_RING - 1; j++) issue(j);
+      V acc[MODES][8], pl[MODES][4], rw[MODES][2];  // acc, pl: x fastest
+#pragma unroll
+      for (int k = 0; k < MODES; k++) {
+        vzero<8>(acc[k]);
+        vzero<4>(pl[k]);
+        vzero<2>(rw[k]);
+      }
+#pragma unroll 1
+      for (int j = 0; j < n; j++) {
+        issue(j + TG_RING - 1);
+        const int p = __shfl_sync(0xffffffffu, j < 32 ? e0 : e1, j & 31) & 63;
+        const int jn = j + 1;
+        const int pn = jn < n ? __shfl_sync(0xffffffffu, jn < 32 ? e0 : e1, jn & 31) & 63 : 64;
+        asm volatile("cp.async.wait_group %0;" ::"n"(TG_RING - 1) : "memory");
+#pragma unroll
+        for (int k = 0; k < MODES; k++) {
+          const V a = ring[j % TG_RING][k][threadIdx.x];
+          tg_add<1>(p & 3, &rw[k][0], &rw[k][1], &a, wp[k][0], wm[k][0]);
+        }
+        if (p >> 2 != pn >> 2) {  // the row's last
+#pragma unroll
+          for (int k = 0; k < MODES; k++) {
+            tg_add<2>((p >> 2) & 3, pl[k], pl[k] + 2, rw[k], wp[k][1], wm[k][1]);
+            vzero<2>(rw[k]);
+          }
+          if (p >> 4 != pn >> 4) {  // the plane's last
+#pragma unroll
+            for (int k = 0; k < MODES; k++) {
+              tg_add<4>(p >> 4, acc[k], acc[k] + 4, pl[k], wp[k][2], wm[k][2]);
+              vzero<4>(pl[k]);
+            }
+          }
+        }
+      }
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+      for (int c = 0; c < 8; c++) {
+        const int e = __shfl_sync(0xffffffffu, et, c);
+#pragma unroll
+        for (int k = 0; k < MODES; k++)
+          if (e >= 0 && m[k] < nexp) __stcs(lv + ((size_t)e * nd + id) * nexp + m[k], acc[k][c]);
+      }
+    }
+  }
+}
+
 // W[s][m] = prod_d exp(i ts(k_d) xmin s_d) (gnd_mk_full_translation_matrices,
 // src/pfgt/pfgt_nufftrouts.f:336-424), s_d = s/3^d % 3 - 1.
 template <typename T>
@@ -1022,9 +1270,7 @@ int pw_form(const PWParams& P, const Tree& t, const Lists& L, const SourceSet<T>
     FGT_LAUNCH_CHECK();
   }
   // FP32 grids too large for shared memory: x-slabs (3D without
-  // wrap-around).  FP64 keeps the global-memory grid: its shared-memory
-  // atomics are no faster than global ones (the slab form of the FP64
-  // eps = 1e-9 cell took 101 ms against 88 ms).
+  // wrap-around).  FP64 grids of that size take the matrix instructions below.
   SlabPlan sp;
   if (sizeof(T) == 4 &&
       sizeof(T) * (size_t)a.g.bufsz + order_offset<T>(a.g.G, a.g.K) > (size_t)MAXSMEM)
@@ -1100,6 +1346,24 @@ int pw_translate(const PWParams& P, const Lists& L, PWData<T>& D, PWWork* work, 
     work->bytes_translate = (double)sizeof(T) * 2 * P.nexp * P.nd *
                             ((double)L.n_trans + 2.0 * L.n_eval);
   if (L.n_eval == 0) return 1;
+  // FP64 and 2D read memory less often by groups: 10^7 points in a periodic
+  // square 2.1 -> 0.78 ms, spheres of 4e6 points at 1e-9 2.7 -> 1.9 and of 2e6
+  // at 1e-6 1.2 -> 1.0.  In FP32 3D the expansions fit the L2 and the kernel by
+  // lists is as fast (0.56 / 0.57 ms at 1e6 points, 0.74 / 0.71 at 10^7).
+  if (L.n_grp > 0 && (P.dim < 3 || sizeof(T) == 8)) {
+    // a few waves of blocks; a thread's factors serve all its groups
+    const int gx = ceil_div(P.nexp, TG_THREADS);
+    const dim3 grid(gx, std::max(1, std::min({L.n_grp, 65535, ceil_div(12 * kSMs, gx)})));
+    auto go = [&](auto kern) {
+      kern<<<grid, TG_THREADS, 0, s>>>(L.n_grp, L.n_form, P.nexp, P.nd, L.grp_src, L.grp_trg, D.mp, D.wtab,
+                                D.loc);
+      FGT_LAUNCH_CHECK();
+    };
+    if (P.dim == 1) go(k_translate_groups<T, 1>);
+    else if (P.dim == 2) go(k_translate_groups<T, 2>);
+    else if constexpr (sizeof(T) == 8) go(k_translate_groups3<T>);
+    return 2;
+  }
   // a thread runs TRANS_MPT modes of TGE consecutive eval boxes, which
   // share most of their source expansions: the repeated reads hit L1
   constexpr int TGE = 4;

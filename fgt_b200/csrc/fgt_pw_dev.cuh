@@ -15,6 +15,9 @@
 // stencil base cell (order_cells: a warp reads few distinct addresses);
 // thread-per-point spreading and the periodic full grids use a bank-balanced
 // order (order_chunk: 32 distinct banks per stencil offset).
+//
+// FP64 3D grids without wrap-around and small 2D boxes in FP64 have kernels of
+// their own on the matrix instructions (fgt_pw64.cu, fgt_pw64_2d.cu).
 #pragma once
 #include <math.h>
 

@@ -779,6 +779,9 @@ __global__ void __launch_bounds__(DW * 32) k_direct64p(DArgs<double> a, const in
       for (int c = 0; c < NC; c++)
         a.out[((size_t)c * a.nd + a.d0) * a.ne + p] += c ? -a.rfac * acc[c] : acc[c];
     }
+    // the next item's first batch goes into the buffer that the last one may
+    // still be read from: shuffles order no memory
+    __syncwarp();
     it = __shfl_sync(0xffffffffu, nxt, 0);
   }
 }

@@ -291,15 +291,16 @@ struct SideSync {
 // Pinned staging of a small call's host arrays, per host thread.  Copies from
 // and to pageable memory go through the driver one thread at a time (60
 // batched instances, 52 MB: about 9 ms whatever the number of workers); a
-// memcpy into pinned memory runs on the caller's core.  At most kMax bytes per
-// thread, freed with the thread; page-locked arrays and larger calls copy
-// directly (the driver overlaps its own staging with the transfer: 16 MB took
-// 5% longer through one memcpy each way).
+// memcpy into pinned memory runs on the caller's core.  Calls of at most kMax
+// bytes; the buffer (a power of two, 8 MB at most) is freed with the thread.
+// Page-locked arrays and larger calls copy directly (the driver overlaps its
+// own staging with the transfer: 16 MB took 5% longer through one memcpy each
+// way).  No call leaves copies from or to the buffer behind (CallSync).
 class HostStage {
  public:
   static constexpr size_t kMax = 4 << 20;
   // Whether a call whose arrays take `bytes` stages them.
-  bool begin(size_t bytes, const void* array, cudaStream_t s) {
+  bool begin(size_t bytes, const void* array) {
     if (bytes > kMax) return false;
     cudaPointerAttributes at;
     if (cudaPointerGetAttributes(&at, array) != cudaSuccess) {
@@ -307,7 +308,6 @@ class HostStage {
       return false;
     }
     if (at.type != cudaMemoryTypeUnregistered) return false;
-    if (open_) (void)cudaStreamSynchronize(s_);  // a call that failed half way
     out_.clear();
     used_ = 0;
     bytes += 1024;  // rounding of up to 11 arrays
@@ -324,25 +324,22 @@ class HostStage {
       }
       cap_ = want;
     }
-    open_ = true;
-    s_ = s;
     return true;
   }
-  void h2d(void* dev, const void* host, size_t bytes) {
+  void h2d(void* dev, const void* host, size_t bytes, cudaStream_t s) {
     char* p = take(bytes);
     memcpy(p, host, bytes);
-    FGT_CUDA(cudaMemcpyAsync(dev, p, bytes, cudaMemcpyHostToDevice, s_));
+    FGT_CUDA(cudaMemcpyAsync(dev, p, bytes, cudaMemcpyHostToDevice, s));
   }
-  void d2h(void* host, const void* dev, size_t bytes) {
+  void d2h(void* host, const void* dev, size_t bytes, cudaStream_t s) {
     char* p = take(bytes);
-    FGT_CUDA(cudaMemcpyAsync(p, dev, bytes, cudaMemcpyDeviceToHost, s_));
+    FGT_CUDA(cudaMemcpyAsync(p, dev, bytes, cudaMemcpyDeviceToHost, s));
     out_.push_back({host, p, bytes});
   }
   // After the stream has been synchronised: the results to the caller.
   void finish() {
     for (const Out& o : out_) memcpy(o.host, o.p, o.bytes);
     out_.clear();
-    open_ = false;
   }
   ~HostStage() {
     if (p_) cudaFreeHost(p_);
@@ -362,14 +359,23 @@ class HostStage {
   }
   char* p_ = nullptr;
   size_t cap_ = 0, used_ = 0;
-  bool open_ = false;
-  cudaStream_t s_ = nullptr;
   std::vector<Out> out_;
 };
 HostStage& host_stage() {
   static thread_local HostStage st;
   return st;
 }
+// Waits for a call's stream when the call leaves by an error: its stream is
+// the caller's, who may destroy it then, and its workspace and the staging
+// buffer are the next call's.
+struct CallSync {
+  cudaStream_t s;
+  bool done = false;
+  explicit CallSync(cudaStream_t st) : s(st) {}
+  ~CallSync() {
+    if (!done) (void)cudaStreamSynchronize(s);
+  }
+};
 
 // Phase names of fgt_stats.ms (slots 0..9).
 const char* const kPhaseName[10] = {"h2d",       "tree",  "sort_gather", "lists", "form",
@@ -985,12 +991,13 @@ int pfgt_impl(const fgt_opts* opts_in, int nd, int dim, double delta, double eps
       sizeof(double) * ((size_t)ns * (dim + (c.ifcharge ? nd : 0) + (c.ifdipole ? nd + dim : 0) +
                                       nd * ncomp(c.ifpgh)) +
                         (size_t)nt * (dim + nd * ncomp(c.ifpghtarg)));
+  CallSync call_sync(s);
   HostStage& stage = host_stage();
-  const bool staged = !o.device_ptrs && stage.begin(host_bytes, sources, s);
+  const bool staged = !o.device_ptrs && stage.begin(host_bytes, sources);
   auto h2d = [&](DBuf<double>& b, const double* h, size_t n) -> const double* {
     if (o.device_ptrs) return h;
     b.alloc(n, s);
-    if (staged) stage.h2d(b.get(), h, sizeof(double) * n);
+    if (staged) stage.h2d(b.get(), h, sizeof(double) * n, s);
     else FGT_CUDA(cudaMemcpyAsync(b.get(), h, sizeof(double) * n, cudaMemcpyHostToDevice, s));
     return b.get();
   };
@@ -1043,7 +1050,7 @@ int pfgt_impl(const fgt_opts* opts_in, int nd, int dim, double delta, double eps
     if (side_sync.s && c.sources_done) FGT_CUDA(cudaStreamWaitEvent(so, c.sources_done, 0));
     auto d2h = [&](double* h, const DBuf<double>& b, size_t n, cudaStream_t q) {
       if (!h || !b.p) return;
-      if (staged) stage.d2h(h, b.get(), sizeof(double) * n);
+      if (staged) stage.d2h(h, b.get(), sizeof(double) * n, q);
       else FGT_CUDA(cudaMemcpyAsync(h, b.get(), sizeof(double) * n, cudaMemcpyDeviceToHost, q));
     };
     if (ifpgh >= 1) d2h(pot, d_pot, (size_t)ns * nd, so);
@@ -1060,6 +1067,7 @@ int pfgt_impl(const fgt_opts* opts_in, int nd, int dim, double delta, double eps
   tm.mark(9);
   near_status_fetch(s);
   FGT_CUDA(cudaStreamSynchronize(s));
+  call_sync.done = true;
   raise_failed_checks(s);
   if (staged) stage.finish();
   if (st) {
@@ -1195,12 +1203,13 @@ int plan_execute_impl(fgt_plan* pl, int ifcharge, const double* charge, int ifdi
       sizeof(double) * ((size_t)ns * ((c.ifcharge ? nd : 0) + (c.ifdipole ? nd + dim : 0) +
                                       nd * ncomp(ifpgh)) +
                         (size_t)nt * nd * ncomp(pght));
+  CallSync call_sync(s);
   HostStage& stage = host_stage();
-  const bool staged = !o.device_ptrs && stage.begin(host_bytes, c.ifcharge ? charge : dipstr, s);
+  const bool staged = !o.device_ptrs && stage.begin(host_bytes, c.ifcharge ? charge : dipstr);
   auto h2d = [&](DBuf<double>& b, const double* h, size_t n) -> const double* {
     if (o.device_ptrs) return h;
     b.alloc(n, s);
-    if (staged) stage.h2d(b.get(), h, sizeof(double) * n);
+    if (staged) stage.h2d(b.get(), h, sizeof(double) * n, s);
     else FGT_CUDA(cudaMemcpyAsync(b.get(), h, sizeof(double) * n, cudaMemcpyHostToDevice, s));
     return b.get();
   };
@@ -1224,7 +1233,7 @@ int plan_execute_impl(fgt_plan* pl, int ifcharge, const double* charge, int ifdi
   if (!o.device_ptrs) {
     auto d2h = [&](double* h, const DBuf<double>& b, size_t n) {
       if (!h || !b.p) return;
-      if (staged) stage.d2h(h, b.get(), sizeof(double) * n);
+      if (staged) stage.d2h(h, b.get(), sizeof(double) * n, s);
       else FGT_CUDA(cudaMemcpyAsync(h, b.get(), sizeof(double) * n, cudaMemcpyDeviceToHost, s));
     };
     if (ifpgh >= 1) d2h(pot, d_pot, (size_t)ns * nd);
@@ -1236,6 +1245,7 @@ int plan_execute_impl(fgt_plan* pl, int ifcharge, const double* charge, int ifdi
   }
   near_status_fetch(s);
   FGT_CUDA(cudaStreamSynchronize(s));
+  call_sync.done = true;
   raise_failed_checks(s);
   if (staged) stage.finish();
   return FGT_OK;

@@ -1,0 +1,69 @@
+"""Small host-array calls and their pinned staging: after a call that failed
+half way on a stream of the caller's, which the caller then destroys, the
+thread's next small call gives the results of a call in a fresh thread.
+
+Tolerance: equal calls differ by the order of FP32 atomics only, as in
+test_gpu_failure.py (1e-6)."""
+import ctypes as C
+import threading
+
+import numpy as np
+import pytest
+
+from conftest import relerr
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs():
+    rng = np.random.default_rng(12)
+    src, trg = rng.uniform(-0.5, 0.5, (2, 2000, 3))
+    return src, trg, rng.standard_normal((2000, 1))
+
+
+def _call(fgt, delta, stream=0):
+    """pot and pottarg of the status call with host arrays on `stream`."""
+    L = fgt.lib()
+    src, trg, q = _inputs()
+    pot, pt = np.zeros((2, 2000, 1))
+    o = fgt.FgtOpts()
+    L.fgt_opts_default(C.byref(o))
+    o.stream = stream
+    b0, c0 = C.c_double(1.0), np.zeros(3)
+
+    def p(a):
+        return a.ctypes.data_as(C.c_void_p)
+
+    rc = L.fgt_pfgt_c(C.byref(o), 1, 3, delta, 1e-6, 0, C.byref(b0),
+                      c0.ctypes.data_as(C.POINTER(C.c_double)), 2000, p(src), 1, p(q), 0, None,
+                      None, 1, p(pot), None, None, 2000, p(trg), 1, p(pt), None, None)
+    return rc, pot, pt
+
+
+def _in_fresh_thread(f):
+    out = []
+    t = threading.Thread(target=lambda: out.append(f()))
+    t.start()
+    t.join()
+    return out[0]
+
+
+def test_call_after_a_failed_call_whose_stream_is_gone(fgt):
+    import torch
+    rt = torch.cuda.cudart()
+    rc, pot, pt = _in_fresh_thread(lambda: _call(fgt, 1e-3))
+    assert rc == fgt.FGT_OK
+
+    def failed_then_good():
+        torch.cuda.init()
+        s = C.c_void_p()
+        assert int(rt.cudaStreamCreate(C.addressof(s))) == 0
+        first = _call(fgt, 1e-16, s.value)[0]  # deeper than the path key holds
+        assert int(rt.cudaStreamDestroy(s.value)) == 0
+        return first, [_call(fgt, 1e-3) for _ in range(2)]
+
+    first, after = _in_fresh_thread(failed_then_good)
+    assert first == fgt.FGT_ERR_UNSUPPORTED
+    for rc, a, b in after:
+        assert rc == fgt.FGT_OK
+        assert relerr(pot, a) < 1e-6 and relerr(pt, b) < 1e-6

@@ -89,7 +89,18 @@ unsigned check_sites(cudaStream_t s) {
   return first;
 }
 
-void* Arena::alloc(size_t bytes) {
+namespace {
+// FGT_WORKSPACE_MAX (bytes; unset: no limit).
+size_t workspace_max() {
+  const char* e = getenv("FGT_WORKSPACE_MAX");
+  if (!e || !*e) return SIZE_MAX;
+  char* end = nullptr;
+  const unsigned long long v = strtoull(e, &end, 10);
+  return end == e ? SIZE_MAX : (size_t)v;
+}
+}  // namespace
+
+void* Arena::try_alloc(size_t bytes) {
   bytes = (bytes + 255) & ~size_t(255);
   for (auto& c : chunks)
     if (c.off + bytes <= c.cap) {
@@ -101,15 +112,36 @@ void* Arena::alloc(size_t bytes) {
     }
   size_t cap = std::max(bytes, (size_t)256 << 20);
   if (!chunks.empty()) cap = std::max(cap, chunks.back().cap);
-  char* p = nullptr;
-  if (cudaMalloc((void**)&p, cap) != cudaSuccess) {
+  // where memory is short: what is needed only, then without the last chunks
+  // that a rewind has emptied (those in front keep their place for the marks)
+  const size_t limit = workspace_max();
+  for (size_t want : {cap, bytes, bytes}) {
+    char* p = nullptr;
+    size_t held = 0;
+    for (const auto& c : chunks) held += c.cap;
+    if (held <= limit && want <= limit - held && cudaMalloc((void**)&p, want) == cudaSuccess) {
+      chunks.push_back({p, want, bytes});
+      used += bytes;
+      high = std::max(high, used);
+      return p;
+    }
     (void)cudaGetLastError();
+    if (want != bytes) continue;
+    if (chunks.empty() || chunks.back().off) break;
+    while (!chunks.empty() && chunks.back().off == 0) {
+      cudaFree(chunks.back().p);  // waits for the kernels that used it
+      chunks.pop_back();
+    }
+  }
+  return nullptr;
+}
+
+void* Arena::alloc(size_t bytes) {
+  void* p = try_alloc(bytes);
+  if (!p) {
     fgt_set_error_message("device workspace allocation failed", __FILE__, __LINE__);
     throw Error{FGT_ERR_NOMEM, "device workspace allocation failed"};
   }
-  chunks.push_back({p, cap, bytes});
-  used += bytes;
-  high = std::max(high, used);
   return p;
 }
 
@@ -137,6 +169,7 @@ void Arena::reset(cudaStream_t s) {
     for (auto& c : chunks) cudaFree(c.p);
     chunks.clear();
     size_t cap = ((size_t)(high * 1.05) + ((size_t)1 << 20)) & ~(((size_t)1 << 20) - 1);
+    cap = std::min(cap, workspace_max());
     char* p = nullptr;
     if (cudaMalloc((void**)&p, cap) == cudaSuccess) chunks.push_back({p, cap, 0});
     else (void)cudaGetLastError();
@@ -153,9 +186,15 @@ std::vector<size_t> Arena::mark() const {
 }
 
 void Arena::rewind(const std::vector<size_t>& m) {
-  zero_p = nullptr;  // may lie past the mark
-  zero_left = 0;
-  for (size_t i = 0; i < chunks.size(); i++) chunks[i].off = i + 1 < m.size() ? m[i] : 0;
+  bool keep = false;  // the zeroed bytes, unless they lie past the mark
+  for (size_t i = 0; i < chunks.size(); i++) {
+    chunks[i].off = i + 1 < m.size() ? m[i] : 0;
+    keep = keep || (zero_p >= chunks[i].p && zero_p + zero_left <= chunks[i].p + chunks[i].off);
+  }
+  if (!keep) {
+    zero_p = nullptr;
+    zero_left = 0;
+  }
   used = m.empty() ? 0 : m.back();
 }
 

@@ -12,6 +12,8 @@ namespace fgt {
 // across calls (reset at the end of every call; grown with cudaMalloc only
 // when a call needs more than any earlier one, then consolidated into one
 // chunk of the high-water size).  Removes allocation from the steady state.
+// FGT_WORKSPACE_MAX (bytes) bounds what one workspace may hold, to test what a
+// call does where memory is short.
 struct Arena {
   struct Chunk {
     char* p;
@@ -22,7 +24,8 @@ struct Arena {
   // zeroed bytes for small counters, cleared in blocks (one memset for many)
   char* zero_p = nullptr;
   size_t zero_left = 0;
-  void* alloc(size_t bytes);
+  void* alloc(size_t bytes);      // fails the call when there is no room
+  void* try_alloc(size_t bytes);  // null when there is no room
   void* alloc_zeroed(size_t bytes, cudaStream_t s);
   void reset(cudaStream_t s);  // call end: all allocations are dead
   void release_all();
@@ -74,6 +77,14 @@ struct DBuf {
     n = count;
     size_t bytes = (count ? count : 1) * sizeof(T);
     p = (T*)thread_arena()->alloc(bytes);
+  }
+  // false (and empty) when there is no room
+  bool try_alloc(size_t count, cudaStream_t st) {
+    release();
+    s = st;
+    p = (T*)thread_arena()->try_alloc((count ? count : 1) * sizeof(T));
+    n = p ? count : 0;
+    return p != nullptr;
   }
   // a small zeroed buffer (counters)
   void alloc_zeroed(size_t count, cudaStream_t st) {

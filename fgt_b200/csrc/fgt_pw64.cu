@@ -21,7 +21,10 @@
 // fit in shared memory gain too (N = M = 2e6, eps = 1e-6: form 3.2 -> 2.0,
 // evaluation 7.8 -> 4.0 ms against a 200 KB grid and a SIMT stencil per CTA;
 // N = 1e5, eps = 1e-3: 0.43 -> 0.22 and 0.37 -> 0.17).
+#include <limits.h>
 #include <stdlib.h>
+
+#include <mutex>
 
 #include "fgt_pw64.cuh"
 #include "fgt_pw64_dev.cuh"
@@ -1044,24 +1047,61 @@ bool eval64_takes(int w, int K, int G, bool wrap) {
   }
 }
 
-// Boxes whose grids are held at a time: 4 GB of them, one per SM at least.
+// Boxes whose grids may be held at a time: a 128th of the device's memory
+// (1.4 GB, 2,700 boxes at eps = 1e-9) of the thread's workspace, which the
+// form and the evaluations of a call use one after the other.  Fewer cost the
+// ends of the runs: 2,265 boxes of 64 clusters, N = M = 2e6, evaluation 9.6 ms
+// at once, 9.8 in runs of 1,184 and 2,000, 10.1 of 592, 13.6 of 148.
 // FGT_GRID64_BOXES (a box count) lowers it, to test the loop over the runs.
-static int grids_held(const Lay64& lay, int G, int nbox) {
-  const size_t fit = ((size_t)4 << 30) / (sizeof(double) * lay.grid(G));
-  size_t held = std::max<size_t>(fit, kSMs);
+static int grids_fit(const Lay64& lay, int G) {
+  static std::mutex mu;
+  static size_t budget[64] = {0};
+  int dev = 0;
+  FGT_CUDA(cudaGetDevice(&dev));
+  size_t bytes;
+  {
+    std::lock_guard<std::mutex> lk(mu);
+    size_t& b = budget[dev & 63];
+    if (b == 0) {
+      size_t free_b = 0, total_b = 0;
+      FGT_CUDA(cudaMemGetInfo(&free_b, &total_b));
+      b = total_b / 128;
+    }
+    bytes = b;
+  }
+  size_t held = std::max<size_t>(bytes / (sizeof(double) * lay.grid(G)), 1);
   if (const char* e = getenv("FGT_GRID64_BOXES")) {
     const long v = strtol(e, nullptr, 10);
     if (v > 0) held = std::min<size_t>(held, (size_t)v);
   }
-  return (int)std::min<size_t>((size_t)nbox, held);
+  return (int)std::min<size_t>(held, INT_MAX);
 }
+// Buffer of the grids of `nbox` boxes in as few runs as fit, all of one
+// length; shorter ones where the device has no room.  Returns their length.
+static int alloc_grids(DBuf<double>& grids, const Lay64& lay, int G, int nbox, cudaStream_t s) {
+  for (int fit = grids_fit(lay, G);; fit = (fit + 1) / 2) {
+    const int held = ceil_div(nbox, ceil_div(nbox, fit));
+    if (grids.try_alloc((size_t)held * lay.grid(G), s)) return held;
+    FGT_REQUIRE(held > 1, FGT_ERR_NOMEM, "device workspace allocation failed");
+  }
+}
+// The workspace a form or an evaluation takes is free again after it (its
+// kernels run before any later ones on the stream).
+struct ArenaMark {
+  Arena* a = thread_arena();
+  std::vector<size_t> m = a->mark();
+  ~ArenaMark() { a->rewind(m); }
+};
 
 template <int W>
 static int launch_form64(const PWArgs<double>& a, const Form64& io, cudaStream_t s) {
   const int G = a.g.G, K = a.g.K, NF = 2 * K + 1, ksg = (G + 3) / 4;
+  if (io.n_form <= 0) return 0;
   const Lay64 lay(G, K);
-  const int held = grids_held(lay, G, io.n_form), runs = ceil_div(io.n_form, held) * io.nd * io.ncomp;
-  DBuf<double> grids((size_t)held * lay.grid(G), s);
+  const ArenaMark mark;
+  DBuf<double> grids;
+  const int held = alloc_grids(grids, lay, G, io.n_form, s);
+  const int runs = ceil_div(io.n_form, held) * io.nd * io.ncomp;
   DBuf<int> next;
   next.alloc_zeroed(runs, s);
   Es64 es;
@@ -1110,9 +1150,15 @@ template <int W, bool DERIV>
 static int launch_eval64(const PWArgs<double>& a, const Eval64& io, cudaStream_t s) {
   const int G = a.g.G, K = a.g.K;
   const Lay64 lay(G, K);
-  const int nc = DERIV ? 1 : io.ncomp_max, held = grids_held(lay, G, io.nbox);
-  const int runs = ceil_div(io.nbox, held) * io.nd * nc;
-  DBuf<double> grids((size_t)held * lay.grid(G), s);
+  const ArenaMark mark;
+  // the count of boxes with a grid is read back only where the bound asks for
+  // several runs (~15 us against the empty ones and the memory)
+  int nbox = io.nbox;
+  if (nbox > grids_fit(lay, G)) nbox = fetch_int(io.nbox_dev, s);
+  if (nbox <= 0) return 0;
+  DBuf<double> grids;
+  const int nc = DERIV ? 1 : io.ncomp_max, held = alloc_grids(grids, lay, G, nbox, s);
+  const int runs = ceil_div(nbox, held) * io.nd * nc;
   DBuf<int> next;
   next.alloc_zeroed(runs, s);
   const size_t sm = sizeof(EvalSmem64<W, DERIV>);
@@ -1123,8 +1169,8 @@ static int launch_eval64(const PWArgs<double>& a, const Eval64& io, cudaStream_t
   int run = 0;
   for (int id = 0; id < io.nd; id++)
     for (int c = 0; c < nc; c++)
-      for (int i0 = 0; i0 < io.nbox; i0 += held, run++) {
-        const int i1 = std::min(io.nbox, i0 + held);
+      for (int i0 = 0; i0 < nbox; i0 += held, run++) {
+        const int i1 = std::min(nbox, i0 + held);
         auto planes = [&](auto gtc) {
           constexpr int GT = decltype(gtc)::value;
           const size_t tb = sizeof(double) * 32 * GT * (2 * ceil_div(K + 1, 4) + ceil_div(2 * (K + 1), 4));

@@ -698,9 +698,9 @@ void execute(const Setup& u, const Call& c, const fgt_opts& o, fgt_stats* st, cu
   double pairs = 0;
   NearPacked packed;
   DBuf<float4> near_rec;
+  // no room for the records: the list walk, which needs none
   if (u.near_total > 0 && nd == 1 && c.ifcharge && !c.ifdipole && c.ifpgh <= 2 &&
-      c.ifpghtarg <= 2) {
-    near_rec.alloc((size_t)u.near_total * (sizeof(T) == 4 ? 4 : 2), s);
+      c.ifpghtarg <= 2 && near_rec.try_alloc((size_t)u.near_total * (sizeof(T) == 4 ? 4 : 2), s)) {
     near_lists_fill<T>(g, L, src, t.trg_lo, t.trg_hi, u.near_pos, near_rec.get(), s);
     launches++;
     packed.pos = u.near_pos;

@@ -326,12 +326,22 @@ class HostStage {
     }
     return true;
   }
+  // An array in device memory, which a memcpy would fault on, is copied by the
+  // driver.
   void h2d(void* dev, const void* host, size_t bytes, cudaStream_t s) {
+    if (on_device(host)) {
+      FGT_CUDA(cudaMemcpyAsync(dev, host, bytes, cudaMemcpyDefault, s));
+      return;
+    }
     char* p = take(bytes);
     memcpy(p, host, bytes);
     FGT_CUDA(cudaMemcpyAsync(dev, p, bytes, cudaMemcpyHostToDevice, s));
   }
   void d2h(void* host, const void* dev, size_t bytes, cudaStream_t s) {
+    if (on_device(host)) {
+      FGT_CUDA(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDefault, s));
+      return;
+    }
     char* p = take(bytes);
     FGT_CUDA(cudaMemcpyAsync(p, dev, bytes, cudaMemcpyDeviceToHost, s));
     out_.push_back({host, p, bytes});
@@ -351,6 +361,12 @@ class HostStage {
     const char* p;
     size_t bytes;
   };
+  static bool on_device(const void* p) {
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) == cudaSuccess) return at.type == cudaMemoryTypeDevice;
+    (void)cudaGetLastError();
+    return false;
+  }
   char* take(size_t bytes) {
     FGT_REQUIRE(used_ + bytes <= cap_, FGT_ERR_NOMEM, "staging buffer too small");
     char* p = p_ + used_;

@@ -1,16 +1,19 @@
 """Small host-array calls and their pinned staging: after a call that failed
 half way on a stream of the caller's, which the caller then destroys, the
-thread's next small call gives the results of a call in a fresh thread.
+thread's next small call gives the results of a call in a fresh thread; and
+strengths or outputs that lie in device memory do not end the process.
 
 Tolerance: equal calls differ by the order of FP32 atomics only, as in
 test_gpu_failure.py (1e-6)."""
 import ctypes as C
+import subprocess
+import sys
 import threading
 
 import numpy as np
 import pytest
 
-from conftest import relerr
+from conftest import ROOT, relerr
 
 pytestmark = pytest.mark.gpu
 
@@ -67,3 +70,30 @@ def test_call_after_a_failed_call_whose_stream_is_gone(fgt):
     for rc, a, b in after:
         assert rc == fgt.FGT_OK
         assert relerr(pot, a) < 1e-6 and relerr(pt, b) < 1e-6
+
+
+def test_device_arrays_among_host_arrays():
+    """Host sources, so the call is staged; the charges and the potential in
+    device memory.  In a child: a fault there would end the process."""
+    code = r"""
+import ctypes as C, numpy as np, torch, fgt_b200 as F
+rng = np.random.default_rng(12)
+n = 2000
+src, q = rng.uniform(-0.5, 0.5, (n, 3)), rng.standard_normal((n, 1))
+ref = F.pfgt(1, 3, 1e-3, 1e-6, 0, src, charge=q, ifpgh=2)
+dq = torch.from_numpy(q).cuda()
+pot = torch.zeros(n, 1, dtype=torch.float64, device="cuda")
+grad = np.zeros((n, 3, 1))
+torch.cuda.synchronize()
+b0, c0 = C.c_double(1.0), np.zeros(3)
+p = lambda a: a.ctypes.data_as(C.c_void_p)
+rc = F.lib().fgt_pfgt_c(None, 1, 3, 1e-3, 1e-6, 0, C.byref(b0),
+                        c0.ctypes.data_as(C.POINTER(C.c_double)), n, p(src), 1, dq.data_ptr(), 0,
+                        None, None, 2, pot.data_ptr(), p(grad), None, 0, None, 0, None, None, None)
+assert rc == F.FGT_OK, F.last_error()
+rel = lambda a, b: np.linalg.norm(a - b) / np.linalg.norm(a)
+assert rel(ref["pot"], pot.cpu().numpy()) < 1e-6 and rel(ref["grad"], grad) < 1e-6
+"""
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0, (r.returncode, r.stderr[-2000:])

@@ -216,13 +216,12 @@ __global__ void k_gather_out_aos(const double* __restrict__ aos, int n, int npot
 // the outputs are first transposed to AoS so a point's components are one
 // contiguous read (config-3-like calls: nd = 4, pot + grad).
 void reorder_outputs(const double* srt, int n, int nd, int dim, int pgh, const uint32_t* inv,
-                     double* pot, double* grad, double* hess, cudaStream_t s, int& launches) {
+                     double* pot, double* grad, double* hess, cudaStream_t s) {
   const int nh = dim * (dim + 1) / 2;
   const int npot = nd, ngrad = pgh >= 2 ? nd * dim : 0, nhess = pgh >= 3 ? nd * nh : 0;
   if (npot + ngrad + nhess < 8) {
     k_gather_out<<<grid_for(n, 256), 256, 0, s>>>(srt, n, nd, dim, pgh, inv, pot, grad, hess);
     FGT_LAUNCH_CHECK();
-    launches++;
     return;
   }
   DBuf<double> aos((size_t)n * (npot + ngrad + nhess), s);
@@ -231,7 +230,6 @@ void reorder_outputs(const double* srt, int n, int nd, int dim, int pgh, const u
   k_gather_out_aos<<<grid_for(n, 256), 256, 0, s>>>(aos, n, npot, ngrad, nhess, inv, pot, grad,
                                                      hess);
   FGT_LAUNCH_CHECK();
-  launches += 2;
 }
 
 struct DevicePool {
@@ -470,7 +468,6 @@ struct Setup {
   // built) and the positions of every list entry's records
   long long near_total = -1;
   DBuf<int> near_pos;
-  int launches = 0;
 };
 
 // Records of the packed list-1 sources are 64 bytes (FP64: 32); above this count (16 GiB,
@@ -536,7 +533,6 @@ void setup_geometry(Setup& u, const Call& c, double* bs0_io, double* cen0_io, co
   u.nt = c.nt;
   u.delta = c.delta;
   u.eps = c.eps;
-  int launches = 0;
   // --- scalar set-up (pfgt.f:110-140)
   int npwlevel = 0;
   double bs0 = *bs0_io, cen0[FGT_MAXDIM] = {0, 0, 0};
@@ -549,7 +545,6 @@ void setup_geometry(Setup& u, const Call& c, double* bs0_io, double* cen0_io, co
   } else {
     tree_setup_scalars(dim, c.delta, c.eps, c.iperiod, c.src, c.ns, c.trg, c.nt, &npwlevel, &bs0,
                        cen0, s);
-    launches += (c.iperiod != 1) ? 2 : 0;
   }
   if (c.iperiod != 1 && !fixed_root) {
     *bs0_io = bs0;
@@ -561,7 +556,6 @@ void setup_geometry(Setup& u, const Call& c, double* bs0_io, double* cen0_io, co
   // --- tree (pts_tree_mem/build, pts_tree_sort)
   Tree& t = u.t;
   tree_build(t, dim, c.iperiod, npwlevel, ndiv, bs0, cen0, c.src, c.ns, c.trg, c.nt, s);
-  launches += 12 + 6 * t.nlevels;
   tm.mark(1);
   const int nlevels = t.nlevels;
   // --- expansion length (pfgt.f:321-334, fgtterms.f:72-141)
@@ -604,7 +598,6 @@ void setup_geometry(Setup& u, const Call& c, double* bs0_io, double* cen0_io, co
     nlevend = 0;
   }
   build_lists(t, npwlevel, iperiod0, nlevend, do_pw, u.L, s);
-  launches += do_pw ? 8 : 2;
   tm.mark(3);
   // --- gather (dreorderf, fmmcommon2d.f:3-27) as offsets from reference boxes
   u.soff.alloc((size_t)c.ns * dim, s);
@@ -614,18 +607,15 @@ void setup_geometry(Setup& u, const Call& c, double* bs0_io, double* cen0_io, co
   u.inv_t.alloc(std::max(c.nt, 1), s);
   launch_gather_coords<double>(dim, c.src, c.ns, t.isrc, t.src_ref, t.center, t.nboxes, u.soff,
                                u.inv_s, s);
-  launches++;
   if (c.nt > 0) {
     launch_gather_coords<double>(dim, c.trg, c.nt, t.itrg, t.trg_ref, t.center, t.nboxes, u.toff,
                                  u.inv_t, s);
-    launches++;
   }
   u.npwlevel = npwlevel;
   u.iperiod0 = iperiod0;
   if (near_lists && u.L.n_l1 > 0) {
     u.near_total = near_lists_count(direct_geom(u), u.L, t.src_lo, t.src_hi, t.trg_lo, t.trg_hi,
                                     u.soff, c.ns, near_pack_max(), u.near_pos, s);
-    launches += 2;
   }
   u.ndiv = ndiv;
   u.nlevels = nlevels;
@@ -634,7 +624,6 @@ void setup_geometry(Setup& u, const Call& c, double* bs0_io, double* cen0_io, co
   u.periodic_nodes = periodic_nodes;
   u.nlevend = nlevend;
   u.do_pw = do_pw;
-  u.launches = launches;
 }
 
 // Strength-dependent part of a call on a prepared geometry.
@@ -644,14 +633,12 @@ void execute(const Setup& u, const Call& c, const fgt_opts& o, fgt_stats* st, cu
   const int dim = u.dim, nd = u.nd, nhess = dim * (dim + 1) / 2;
   const Tree& t = u.t;
   const Lists& L = u.L;
-  int launches = u.launches;
   if (c.strengths_ready) FGT_CUDA(cudaStreamWaitEvent(s, c.strengths_ready, 0));
   DBuf<T> qs, dss, rns;
   if (c.ifcharge) {
     qs.alloc((size_t)c.ns * nd, s);
     k_gather_vals<T><<<grid_for(c.ns, 256), 256, 0, s>>>(c.q, c.ns, nd, t.isrc, qs);
     FGT_LAUNCH_CHECK();
-    launches++;
   }
   if (c.ifdipole) {
     dss.alloc((size_t)c.ns * nd, s);
@@ -661,7 +648,6 @@ void execute(const Setup& u, const Call& c, const fgt_opts& o, fgt_stats* st, cu
     // rnormal(dim,ns) -> SoA [dim][n]
     k_gather_vals<T><<<grid_for(c.ns, 256), 256, 0, s>>>(c.rn, c.ns, dim, t.isrc, rns);
     FGT_LAUNCH_CHECK();
-    launches += 2;
   }
   // sorted outputs, FP64
   int ncs = c.ifpgh >= 1 ? (1 + (c.ifpgh >= 2 ? dim : 0) + (c.ifpgh >= 3 ? nhess : 0)) : 0;
@@ -670,7 +656,6 @@ void execute(const Setup& u, const Call& c, const fgt_opts& o, fgt_stats* st, cu
   DBuf<double> outt((size_t)std::max(nct, 1) * nd * std::max(c.nt, 1), s);
   if (ncs > 0) outs.zero();
   if (nct > 0 && c.nt > 0) outt.zero();
-  launches += 2;
   SourceSet<T> src;
   src.n = c.ns;
   src.off = u.soff;
@@ -698,11 +683,11 @@ void execute(const Setup& u, const Call& c, const fgt_opts& o, fgt_stats* st, cu
   if (pw) {
     pw_setup(P, dim, nd, u.npw, u.pmax, u.periodic_nodes ? 1 : 0, t.boxsize[0], c.delta, c.eps,
              t.boxsize[t.ncutoff], o.spread_width);
-    launches += pw_form<T>(P, t, L, src, D, wk, s);
+    pw_form<T>(P, t, L, src, D, wk, s);
     tm.mark(4);
-    launches += pw_translate<T>(P, L, D, wk, s);
+    pw_translate<T>(P, L, D, wk, s);
     tm.mark(5);
-    launches += pw_eval<T>(P, t, L, D, es, split_sets ? none : et, se, wk, s);
+    pw_eval<T>(P, t, L, D, es, split_sets ? none : et, se, wk, s);
     tm.mark(6);
     if (st) {
       st->spread_width = P.w;
@@ -718,29 +703,27 @@ void execute(const Setup& u, const Call& c, const fgt_opts& o, fgt_stats* st, cu
   if (u.near_total > 0 && nd == 1 && c.ifcharge && !c.ifdipole && c.ifpgh <= 2 &&
       c.ifpghtarg <= 2 && near_rec.try_alloc((size_t)u.near_total * (sizeof(T) == 4 ? 4 : 2), s)) {
     near_lists_fill<T>(g, L, src, t.trg_lo, t.trg_hi, u.near_pos, near_rec.get(), s);
-    launches++;
     packed.pos = u.near_pos;
     packed.rec = near_rec.get();
   }
   if (c.sources_done) {
     // sources first, then signal; the targets follow
-    launches += direct_near_field<T>(g, L, src, es, st ? &pairs : nullptr, s, &packed);
+    direct_near_field<T>(g, L, src, es, st ? &pairs : nullptr, s, &packed);
     if (c.ifpgh >= 1)
-      reorder_outputs(outs, c.ns, nd, dim, c.ifpgh, u.inv_s, c.pot, c.grad, c.hess, s, launches);
+      reorder_outputs(outs, c.ns, nd, dim, c.ifpgh, u.inv_s, c.pot, c.grad, c.hess, s);
     FGT_CUDA(cudaEventRecord(c.sources_done, s));
-    if (pw && split_sets) launches += pw_eval<T>(P, t, L, D, none, et, se, wk, s);
-    launches += direct_near_field<T>(g, L, src, et, st ? &pairs : nullptr, s, &packed);
+    if (pw && split_sets) pw_eval<T>(P, t, L, D, none, et, se, wk, s);
+    direct_near_field<T>(g, L, src, et, st ? &pairs : nullptr, s, &packed);
   } else {
-    launches += direct_near_field<T>(g, L, src, et, st ? &pairs : nullptr, s, &packed);
-    launches += direct_near_field<T>(g, L, src, es, st ? &pairs : nullptr, s, &packed);
+    direct_near_field<T>(g, L, src, et, st ? &pairs : nullptr, s, &packed);
+    direct_near_field<T>(g, L, src, es, st ? &pairs : nullptr, s, &packed);
   }
   tm.mark(7);
   // --- back to input order
   if (c.ifpgh >= 1 && !c.sources_done)
-    reorder_outputs(outs, c.ns, nd, dim, c.ifpgh, u.inv_s, c.pot, c.grad, c.hess, s, launches);
+    reorder_outputs(outs, c.ns, nd, dim, c.ifpgh, u.inv_s, c.pot, c.grad, c.hess, s);
   if (c.ifpghtarg >= 1 && c.nt > 0)
-    reorder_outputs(outt, c.nt, nd, dim, c.ifpghtarg, u.inv_t, c.pott, c.gradt, c.hesst, s,
-                    launches);
+    reorder_outputs(outt, c.nt, nd, dim, c.ifpghtarg, u.inv_t, c.pott, c.gradt, c.hesst, s);
   tm.mark(8);
   if (st) {
     st->nlevels = u.nlevels;
@@ -770,7 +753,6 @@ void execute(const Setup& u, const Call& c, const fgt_opts& o, fgt_stats* st, cu
     }
     st->n_translations = L.n_trans;
     st->near_pairs = pairs;
-    st->n_kernel_launches = launches;
     st->bs0 = u.bs0;
     for (int k = 0; k < dim; k++) st->cen0[k] = u.cen0[k];
   }
@@ -990,6 +972,7 @@ int pfgt_impl(const fgt_opts* opts_in, int nd, int dim, double delta, double eps
   const bool logging = log_requested();
   fgt_stats* st = o.stats ? o.stats : (logging ? &local_stats : nullptr);
   if (st) memset(st, 0, sizeof(*st));
+  const long long launches0 = launch_count();
   Timer tm((o.timing || logging) && st, s);
   int nhess = dim * (dim + 1) / 2;
   int prec = o.precision;
@@ -1087,6 +1070,7 @@ int pfgt_impl(const fgt_opts* opts_in, int nd, int dim, double delta, double eps
   raise_failed_checks(s);
   if (staged) stage.finish();
   if (st) {
+    st->n_kernel_launches = (int)(launch_count() - launches0);
     st->precision_used = prec;
     tm.finish(st->ms);
     if (logging) log_call(*st, nd, dim, ns, nt, delta, eps);

@@ -27,7 +27,15 @@ struct Error {
     }                                                                          \
   } while (0)
 
-#define FGT_LAUNCH_CHECK() FGT_CUDA(cudaGetLastError())
+// After every kernel launch, one for one: counts it and raises its error.
+namespace fgt {
+long long& launch_count();  // kernels launched by this host thread
+}
+#define FGT_LAUNCH_CHECK()        \
+  do {                            \
+    fgt::launch_count()++;        \
+    FGT_CUDA(cudaGetLastError()); \
+  } while (0)
 
 #define FGT_REQUIRE(cond, code, msg)                                           \
   do {                                                                         \

@@ -1187,10 +1187,10 @@ void launch_packed(const DArgs<float>& a, const NearPacked& p, int* next, cudaSt
 }  // namespace
 
 template <typename T>
-int direct_near_field(const DirectGeom& g, const Lists& L, const SourceSet<T>& src,
-                      const EvalSet<T>& e, double* pairs, cudaStream_t s, const NearPacked* packed) {
-  if (e.pgh <= 0 || e.n <= 0 || L.n_l1 <= 0) return 0;
-  int nb = g.nboxes, launches = 0;
+void direct_near_field(const DirectGeom& g, const Lists& L, const SourceSet<T>& src,
+                       const EvalSet<T>& e, double* pairs, cudaStream_t s, const NearPacked* packed) {
+  if (e.pgh <= 0 || e.n <= 0 || L.n_l1 <= 0) return;
+  int nb = g.nboxes;
   bool chg = src.q != nullptr, dip = src.ds != nullptr;
   // two evaluation points per lane: FP32, charges only, pot or pot + grad, one density
   const bool paired = sizeof(T) == 4 && chg && !dip && e.pgh <= 2 && g.nd == 1;
@@ -1210,7 +1210,6 @@ int direct_near_field(const DirectGeom& g, const Lists& L, const SourceSet<T>& s
     FGT_CUDA(cudaStreamSynchronize(s));
     *pairs += h;
   }
-  launches++;
   DArgs<T> a;
   a.n_items = n_items;
   a.n_items_dev = tot;
@@ -1252,7 +1251,7 @@ int direct_near_field(const DirectGeom& g, const Lists& L, const SourceSet<T>& s
       if (g.dim == 1) e.pgh == 1 ? go(k_direct64p<1, 1>) : go(k_direct64p<1, 2>);
       else if (g.dim == 2) e.pgh == 1 ? go(k_direct64p<2, 1>) : go(k_direct64p<2, 2>);
       else e.pgh == 1 ? go(k_direct64p<3, 1>) : go(k_direct64p<3, 2>);
-      return launches + 1;
+      return;
     }
   }
   if constexpr (sizeof(T) == 4) {
@@ -1271,7 +1270,7 @@ int direct_near_field(const DirectGeom& g, const Lists& L, const SourceSet<T>& s
         if (e.pgh == 1) launch_packed<3, 1>(af, *packed, next, s);
         else launch_packed<3, 2>(af, *packed, next, s);
       }
-      return launches + 1;
+      return;
     }
     if (paired) {
       a.d0 = 0;
@@ -1288,24 +1287,22 @@ int direct_near_field(const DirectGeom& g, const Lists& L, const SourceSet<T>& s
         else k_direct32x2<3, 2><<<grid, DW * 32, 0, s>>>(af);
       }
       FGT_LAUNCH_CHECK();
-      return launches + 1;
+      return;
     }
   }
   for (int d0 = 0; d0 < g.nd; d0 += (g.nd == 1 ? 1 : 4)) {
     a.d0 = d0;
     if (g.nd == 1) dispatch_dim<T, 1>(a, g.dim, e.pgh, chg, dip, s);
     else dispatch_dim<T, 4>(a, g.dim, e.pgh, chg, dip, s);
-    launches++;
   }
-  return launches;
 }
 
-template int direct_near_field<float>(const DirectGeom&, const Lists&, const SourceSet<float>&,
-                                      const EvalSet<float>&, double*, cudaStream_t,
-                                      const NearPacked*);
-template int direct_near_field<double>(const DirectGeom&, const Lists&, const SourceSet<double>&,
-                                       const EvalSet<double>&, double*, cudaStream_t,
+template void direct_near_field<float>(const DirectGeom&, const Lists&, const SourceSet<float>&,
+                                       const EvalSet<float>&, double*, cudaStream_t,
                                        const NearPacked*);
+template void direct_near_field<double>(const DirectGeom&, const Lists&, const SourceSet<double>&,
+                                        const EvalSet<double>&, double*, cudaStream_t,
+                                        const NearPacked*);
 
 }  // namespace fgt
 

@@ -65,14 +65,14 @@ int near_wait_status(cudaStream_t s);
 // which then covers it.
 void near_status_fetch(cudaStream_t s);
 
-// Adds the list-1 interactions onto every point of `e`.  Returns the number
-// of kernel launches; *pairs receives the near-field pair count if not null.
+// Adds the list-1 interactions onto every point of `e`; *pairs receives the
+// near-field pair count if not null.
 // With packed records (charges, one density, pgh <= 2) the near field
 // streams them instead of walking the list.
 template <typename T>
-int direct_near_field(const DirectGeom& g, const Lists& L, const SourceSet<T>& src,
-                      const EvalSet<T>& e, double* pairs, cudaStream_t s,
-                      const NearPacked* packed = nullptr);
+void direct_near_field(const DirectGeom& g, const Lists& L, const SourceSet<T>& src,
+                       const EvalSet<T>& e, double* pairs, cudaStream_t s,
+                       const NearPacked* packed = nullptr);
 
 }  // namespace fgt
 

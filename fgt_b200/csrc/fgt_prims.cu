@@ -12,6 +12,11 @@
 
 namespace fgt {
 
+long long& launch_count() {
+  static thread_local long long n = 0;
+  return n;
+}
+
 namespace {
 struct TuneCache {
   std::mutex mu;

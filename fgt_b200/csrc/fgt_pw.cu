@@ -993,7 +993,7 @@ Form64 form64_args(const FormIO& io, const FormPtrs<double>& fp) {
 }
 
 template <typename T, int DIM, int W>
-int launch_form(PWArgs<T>& a, const FormIO& io, const FormPtrs<T>& fp, DBuf<T>& gs, cudaStream_t s) {
+void launch_form(PWArgs<T>& a, const FormIO& io, const FormPtrs<T>& fp, DBuf<T>& gs, cudaStream_t s) {
   if constexpr (std::is_same<T, double>::value && DIM == 3) {
     if (io.f64) {
       return form64_launch(W, &a, form64_args(io, fp), s);
@@ -1010,7 +1010,7 @@ int launch_form(PWArgs<T>& a, const FormIO& io, const FormPtrs<T>& fp, DBuf<T>& 
       set_smem(k, tneed);
       k<<<grid, PW_THREADS, tneed, s>>>(a, io, fp);
       FGT_LAUNCH_CHECK();
-      return 1;
+      return;
     }
   }
   if constexpr (std::is_same<T, float>::value && DIM == 3) {
@@ -1021,7 +1021,7 @@ int launch_form(PWArgs<T>& a, const FormIO& io, const FormPtrs<T>& fp, DBuf<T>& 
       set_smem(k, sm);
       k<<<grid, PW_THREADS, sm, s>>>(a, io, fp);
       FGT_LAUNCH_CHECK();
-      return 1;
+      return;
     }
   }
   if (need <= (size_t)MAXSMEM) {
@@ -1036,11 +1036,10 @@ int launch_form(PWArgs<T>& a, const FormIO& io, const FormPtrs<T>& fp, DBuf<T>& 
     k<<<grid, PW_THREADS, fix, s>>>(a, io, fp);
   }
   FGT_LAUNCH_CHECK();
-  return 1;
 }
 
 template <typename T, int DIM>
-int form_w(int w, PWArgs<T>& a, const FormIO& io, const FormPtrs<T>& fp, DBuf<T>& gs, cudaStream_t s) {
+void form_w(int w, PWArgs<T>& a, const FormIO& io, const FormPtrs<T>& fp, DBuf<T>& gs, cudaStream_t s) {
   switch (w) {
     case 6: return launch_form<T, DIM, 6>(a, io, fp, gs, s);
     case 8: return launch_form<T, DIM, 8>(a, io, fp, gs, s);
@@ -1050,7 +1049,6 @@ int form_w(int w, PWArgs<T>& a, const FormIO& io, const FormPtrs<T>& fp, DBuf<T>
     case 16: return launch_form<T, DIM, 16>(a, io, fp, gs, s);
     default: FGT_REQUIRE(false, FGT_ERR_UNSUPPORTED, "no form kernel for this width");
   }
-  return 0;
 }
 // Shared memory of k_form_small2 and its warps per CTA (0: does not fit).
 template <typename T>
@@ -1223,11 +1221,11 @@ double pw_pass_flops(const PWParams& P) {
 }
 
 template <typename T>
-int pw_form(const PWParams& P, const Tree& t, const Lists& L, const SourceSet<T>& src,
-            PWData<T>& D, PWWork* work, cudaStream_t s) {
+void pw_form(const PWParams& P, const Tree& t, const Lists& L, const SourceSet<T>& src,
+             PWData<T>& D, PWWork* work, cudaStream_t s) {
   if (L.n_form <= 0) {
     D.mp.alloc(2, s);
-    return 0;
+    return;
   }
   PWArgs<T> a;
   DevTables<T> tb;
@@ -1299,37 +1297,30 @@ int pw_form(const PWParams& P, const Tree& t, const Lists& L, const SourceSet<T>
   DBuf<T> part((size_t)(io.f64 ? 1 : std::max(il.max_partial, 1)) * P.nd * 2 * P.nexp, s);
   fp.partial = part;
   DBuf<T> gs;
-  int n;
-  if (P.dim == 1) n = form_w<T, 1>(P.w, a, io, fp, gs, s);
-  else if (P.dim == 2) n = form_w<T, 2>(P.w, a, io, fp, gs, s);
-  else n = form_w<T, 3>(P.w, a, io, fp, gs, s);
-  if (small2) {
-    form_small2_w<T>(P.w, a, io, fp, oval, first, next2, s);
-    n += 2;
-  }
+  if (P.dim == 1) form_w<T, 1>(P.w, a, io, fp, gs, s);
+  else if (P.dim == 2) form_w<T, 2>(P.w, a, io, fp, gs, s);
+  else form_w<T, 3>(P.w, a, io, fp, gs, s);
+  if (small2) form_small2_w<T>(P.w, a, io, fp, oval, first, next2, s);
   if (!io.f64) {
     k_form_reduce<T><<<kSMs * 4, 256, 0, s>>>(il.split, il.n_split, P.nd, P.nexp, part, D.mp);
     FGT_LAUNCH_CHECK();
   }
-  n += 6;
   if (work) {
     DBuf<unsigned long long> c(1, s);
     c.zero();
     k_count_points<<<grid_for(L.n_form, 256), 256, 0, s>>>(L.n_form, L.form_box, src.lo, src.hi, c);
-    FGT_LAUNCH_CHECK();
+    FGT_CUDA(cudaGetLastError());  // not one of the call's launches
     unsigned long long h = 0;
     FGT_CUDA(cudaMemcpyAsync(&h, c.get(), sizeof(h), cudaMemcpyDeviceToHost, s));
     FGT_CUDA(cudaStreamSynchronize(s));
     const double wd = pow((double)P.w, P.dim), tr = (double)io.ncomp * P.nd;
     work->pts_form = (double)h;
     work->flops_form = tr * (L.n_form * pw_pass_flops(P) + (double)h * 2 * wd);
-    n++;
   }
-  return n;
 }
 
 template <typename T>
-int pw_translate(const PWParams& P, const Lists& L, PWData<T>& D, PWWork* work, cudaStream_t s) {
+void pw_translate(const PWParams& P, const Lists& L, PWData<T>& D, PWWork* work, cudaStream_t s) {
   int nsh = P.dim == 1 ? 3 : (P.dim == 2 ? 9 : 27);
   D.wtab.alloc((size_t)nsh * 2 * P.nexp, s);
   DBuf<double> ts64(P.ts.size(), s);
@@ -1345,7 +1336,7 @@ int pw_translate(const PWParams& P, const Lists& L, PWData<T>& D, PWWork* work, 
   if (work)
     work->bytes_translate = (double)sizeof(T) * 2 * P.nexp * P.nd *
                             ((double)L.n_trans + 2.0 * L.n_eval);
-  if (L.n_eval == 0) return 1;
+  if (L.n_eval == 0) return;
   // FP64 and 2D read memory less often by groups: 10^7 points in a periodic
   // square 2.1 -> 0.78 ms, spheres of 4e6 points at 1e-9 2.7 -> 1.9 and of 2e6
   // at 1e-6 1.2 -> 1.0.  In FP32 3D the expansions fit the L2 and the kernel by
@@ -1362,7 +1353,7 @@ int pw_translate(const PWParams& P, const Lists& L, PWData<T>& D, PWWork* work, 
     if (P.dim == 1) go(k_translate_groups<T, 1>);
     else if (P.dim == 2) go(k_translate_groups<T, 2>);
     else if constexpr (sizeof(T) == 8) go(k_translate_groups3<T>);
-    return 2;
+    return;
   }
   // a thread runs TRANS_MPT modes of TGE consecutive eval boxes, which
   // share most of their source expansions: the repeated reads hit L1
@@ -1376,16 +1367,15 @@ int pw_translate(const PWParams& P, const Lists& L, PWData<T>& D, PWWork* work, 
                                         D.wtab, D.loc.get() + (size_t)e0 * P.nd * 2 * P.nexp);
     FGT_LAUNCH_CHECK();
   }
-  return 2;
 }
 
-template int pw_form<float>(const PWParams&, const Tree&, const Lists&, const SourceSet<float>&,
-                            PWData<float>&, PWWork*, cudaStream_t);
-template int pw_form<double>(const PWParams&, const Tree&, const Lists&, const SourceSet<double>&,
-                             PWData<double>&, PWWork*, cudaStream_t);
-template int pw_translate<float>(const PWParams&, const Lists&, PWData<float>&, PWWork*,
+template void pw_form<float>(const PWParams&, const Tree&, const Lists&, const SourceSet<float>&,
+                             PWData<float>&, PWWork*, cudaStream_t);
+template void pw_form<double>(const PWParams&, const Tree&, const Lists&, const SourceSet<double>&,
+                              PWData<double>&, PWWork*, cudaStream_t);
+template void pw_translate<float>(const PWParams&, const Lists&, PWData<float>&, PWWork*,
                                  cudaStream_t);
-template int pw_translate<double>(const PWParams&, const Lists&, PWData<double>&, PWWork*,
+template void pw_translate<double>(const PWParams&, const Lists&, PWData<double>&, PWWork*,
                                   cudaStream_t);
 
 }  // namespace fgt

@@ -57,15 +57,15 @@ struct PWWork {
   int slabs_form = 1, slabs_eval = 1;  // x-slabs per sub-grid (1: whole grids)
 };
 
-// Forms the expansions of all form boxes.  Returns launches.
+// Forms the expansions of all form boxes.
 template <typename T>
-int pw_form(const PWParams& P, const Tree& t, const Lists& L, const SourceSet<T>& src,
-            PWData<T>& D, PWWork* work, cudaStream_t s);
+void pw_form(const PWParams& P, const Tree& t, const Lists& L, const SourceSet<T>& src,
+             PWData<T>& D, PWWork* work, cudaStream_t s);
 template <typename T>
-int pw_translate(const PWParams& P, const Lists& L, PWData<T>& D, PWWork* work, cudaStream_t s);
+void pw_translate(const PWParams& P, const Lists& L, PWData<T>& D, PWWork* work, cudaStream_t s);
 template <typename T>
-int pw_eval(const PWParams& P, const Tree& t, const Lists& L, const PWData<T>& D,
-            const EvalSet<T>& e0, const EvalSet<T>& e1, int small_eval, PWWork* work,
-            cudaStream_t s);
+void pw_eval(const PWParams& P, const Tree& t, const Lists& L, const PWData<T>& D,
+             const EvalSet<T>& e0, const EvalSet<T>& e1, int small_eval, PWWork* work,
+             cudaStream_t s);
 
 }  // namespace fgt

@@ -1094,9 +1094,9 @@ struct ArenaMark {
 };
 
 template <int W>
-static int launch_form64(const PWArgs<double>& a, const Form64& io, cudaStream_t s) {
+static void launch_form64(const PWArgs<double>& a, const Form64& io, cudaStream_t s) {
   const int G = a.g.G, K = a.g.K, NF = 2 * K + 1, ksg = (G + 3) / 4;
-  if (io.n_form <= 0) return 0;
+  if (io.n_form <= 0) return;
   const Lay64 lay(G, K);
   const ArenaMark mark;
   DBuf<double> grids;
@@ -1131,9 +1131,8 @@ static int launch_form64(const PWArgs<double>& a, const Form64& io, cudaStream_t
       else if (mt == 3) transforms(std::integral_constant<int, 3>{});
       else transforms(std::integral_constant<int, 4>{});
     }
-  return 3 * runs;
 }
-int form64_launch(int w, const void* av, const Form64& io, cudaStream_t s) {
+void form64_launch(int w, const void* av, const Form64& io, cudaStream_t s) {
   const PWArgs<double>& a = *static_cast<const PWArgs<double>*>(av);
   switch (w) {
     case 6: return launch_form64<6>(a, io, s);
@@ -1143,11 +1142,10 @@ int form64_launch(int w, const void* av, const Form64& io, cudaStream_t s) {
     case 14: return launch_form64<14>(a, io, s);
     default: FGT_REQUIRE(false, FGT_ERR_UNSUPPORTED, "no FP64 form kernel for this width");
   }
-  return 0;
 }
 
 template <int W, bool DERIV>
-static int launch_eval64(const PWArgs<double>& a, const Eval64& io, cudaStream_t s) {
+static void launch_eval64(const PWArgs<double>& a, const Eval64& io, cudaStream_t s) {
   const int G = a.g.G, K = a.g.K;
   const Lay64 lay(G, K);
   const ArenaMark mark;
@@ -1155,7 +1153,7 @@ static int launch_eval64(const PWArgs<double>& a, const Eval64& io, cudaStream_t
   // several runs (~15 us against the empty ones and the memory)
   int nbox = io.nbox;
   if (nbox > grids_fit(lay, G)) nbox = fetch_int(io.nbox_dev, s);
-  if (nbox <= 0) return 0;
+  if (nbox <= 0) return;
   DBuf<double> grids;
   const int nc = DERIV ? 1 : io.ncomp_max, held = alloc_grids(grids, lay, G, nbox, s);
   const int runs = ceil_div(nbox, held) * io.nd * nc;
@@ -1188,9 +1186,8 @@ static int launch_eval64(const PWArgs<double>& a, const Eval64& io, cudaStream_t
         k_eval64<W, DERIV><<<kSMs, T64, sm, s>>>(a, es, io, id, c, i0, i1, next.get() + run, grids);
         FGT_LAUNCH_CHECK();
       }
-  return 2 * runs;
 }
-int eval64_launch(int w, bool deriv, const void* av, const Eval64& io, cudaStream_t s) {
+void eval64_launch(int w, bool deriv, const void* av, const Eval64& io, cudaStream_t s) {
   const PWArgs<double>& a = *static_cast<const PWArgs<double>*>(av);
 #define FGT_E64(WW)                                                \
   case WW:                                                         \
@@ -1203,7 +1200,6 @@ int eval64_launch(int w, bool deriv, const void* av, const Eval64& io, cudaStrea
     default: FGT_REQUIRE(false, FGT_ERR_UNSUPPORTED, "no FP64 evaluation kernel for this width");
   }
 #undef FGT_E64
-  return 0;
 }
 
 bool modal64_launch(const void* av, const Eval64& io, int pmax, size_t smem, cudaStream_t s) {

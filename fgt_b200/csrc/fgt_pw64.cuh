@@ -41,13 +41,13 @@ constexpr int SLAB64 = 16;
 bool form64_takes(int w, int K, int G, bool wrap);
 bool eval64_takes(int w, int K, int G, bool wrap);
 // Launches on stream s, grids from the call's workspace; `a`: the launch's
-// PWArgs<double> (host pointer).  Return the number of launches.
-int form64_launch(int w, const void* a, const Form64& io, cudaStream_t s);
+// PWArgs<double> (host pointer).
+void form64_launch(int w, const void* a, const Form64& io, cudaStream_t s);
 // Modal sums of the boxes with at most pmax points (3D; smem: dynamic shared
 // memory, at least 3 (2K+1) pmax complex + (2K+1) + 256 doubles); false: not
 // taken (hessians, expansions too long).
 bool modal64_launch(const void* a, const Eval64& io, int pmax, size_t smem, cudaStream_t s);
-int eval64_launch(int w, bool deriv, const void* a, const Eval64& io, cudaStream_t s);
+void eval64_launch(int w, bool deriv, const void* a, const Eval64& io, cudaStream_t s);
 
 // Small 2D boxes (fgt_pw64_2d.cu): the boxes from *first on of the order, one
 // warp per (box, density); next: work counter, zero.

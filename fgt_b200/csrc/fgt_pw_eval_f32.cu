@@ -4,7 +4,7 @@
 
 namespace fgt {
 
-template int pw_eval<float>(const PWParams&, const Tree&, const Lists&, const PWData<float>&,
-                          const EvalSet<float>&, const EvalSet<float>&, int, PWWork*, cudaStream_t);
+template void pw_eval<float>(const PWParams&, const Tree&, const Lists&, const PWData<float>&,
+                           const EvalSet<float>&, const EvalSet<float>&, int, PWWork*, cudaStream_t);
 
 }  // namespace fgt

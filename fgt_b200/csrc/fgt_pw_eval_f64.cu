@@ -4,7 +4,7 @@
 
 namespace fgt {
 
-template int pw_eval<double>(const PWParams&, const Tree&, const Lists&, const PWData<double>&,
-                          const EvalSet<double>&, const EvalSet<double>&, int, PWWork*, cudaStream_t);
+template void pw_eval<double>(const PWParams&, const Tree&, const Lists&, const PWData<double>&,
+                           const EvalSet<double>&, const EvalSet<double>&, int, PWWork*, cudaStream_t);
 
 }  // namespace fgt

@@ -940,7 +940,7 @@ inline Eval64 eval64_args(const EvalPtrs<double>& ep) {
 }
 
 template <typename T, int DIM, int W, bool DERIV>
-int launch_eval_k(PWArgs<T>& a, const EvalPtrs<T>& ep, DBuf<T>& gs, cudaStream_t s) {
+void launch_eval_k(PWArgs<T>& a, const EvalPtrs<T>& ep, DBuf<T>& gs, cudaStream_t s) {
   size_t fix = eval_offset<T>(a.g.G, a.g.K);
   size_t need = fix + sizeof(T) * (size_t)a.g.bufsz;
   int grid = std::max(1, std::min(ep.max_items, kSMs));
@@ -968,7 +968,7 @@ int launch_eval_k(PWArgs<T>& a, const EvalPtrs<T>& ep, DBuf<T>& gs, cudaStream_t
       set_smem(k, ss);
       k<<<grid, PW_THREADS, ss, s>>>(a, epk);
       FGT_LAUNCH_CHECK();
-      return 1;
+      return;
     }
   }
   if (gb) {
@@ -986,7 +986,6 @@ int launch_eval_k(PWArgs<T>& a, const EvalPtrs<T>& ep, DBuf<T>& gs, cudaStream_t
     k<<<grid, eval_threads<T, DIM, W, false, DERIV>(), sm, s>>>(a, epk);
   }
   FGT_LAUNCH_CHECK();
-  return 1;
 }
 
 template <typename T>
@@ -1033,11 +1032,10 @@ void eval_small2_w(int w, bool deriv, PWArgs<T>& a, const EvalPtrs<T>& ep, const
 
 // deriv: gradients through the kernel derivative (widths 8..16 only)
 template <typename T, int DIM, int W>
-int launch_eval(PWArgs<T>& a, const EvalPtrs<T>& ep, bool deriv, DBuf<T>& gs, cudaStream_t s) {
+void launch_eval(PWArgs<T>& a, const EvalPtrs<T>& ep, bool deriv, DBuf<T>& gs, cudaStream_t s) {
   if constexpr (W % 2 == 1) {  // odd widths: FP32 derivative evaluation only
     FGT_REQUIRE(deriv && sizeof(T) == 4, FGT_ERR_UNSUPPORTED, "odd kernel width outside the FP32 gradient path");
-    if constexpr (sizeof(T) == 4) return launch_eval_k<T, DIM, W, true>(a, ep, gs, s);
-    return 0;
+    if constexpr (sizeof(T) == 4) launch_eval_k<T, DIM, W, true>(a, ep, gs, s);
   } else {
     if constexpr (W >= 8) {
       if (deriv) return launch_eval_k<T, DIM, W, true>(a, ep, gs, s);
@@ -1048,7 +1046,7 @@ int launch_eval(PWArgs<T>& a, const EvalPtrs<T>& ep, bool deriv, DBuf<T>& gs, cu
 }
 
 template <typename T, int DIM>
-int eval_w(int w, PWArgs<T>& a, const EvalPtrs<T>& ep, bool deriv, DBuf<T>& gs, cudaStream_t s) {
+void eval_w(int w, PWArgs<T>& a, const EvalPtrs<T>& ep, bool deriv, DBuf<T>& gs, cudaStream_t s) {
   switch (w) {
     case 6: return launch_eval<T, DIM, 6>(a, ep, deriv, gs, s);
     case 7: return launch_eval<T, DIM, 7>(a, ep, deriv, gs, s);
@@ -1060,10 +1058,9 @@ int eval_w(int w, PWArgs<T>& a, const EvalPtrs<T>& ep, bool deriv, DBuf<T>& gs, 
     case 16: return launch_eval<T, DIM, 16>(a, ep, deriv, gs, s);
     default: FGT_REQUIRE(false, FGT_ERR_UNSUPPORTED, "no evaluation kernel for this width");
   }
-  return 0;
 }
 template <typename T>
-int eval_dim(int dim, int w, PWArgs<T>& a, const EvalPtrs<T>& ep, bool deriv, DBuf<T>& gs,
+void eval_dim(int dim, int w, PWArgs<T>& a, const EvalPtrs<T>& ep, bool deriv, DBuf<T>& gs,
              cudaStream_t s) {
   if (dim == 1) return eval_w<T, 1>(w, a, ep, deriv, gs, s);
   if (dim == 2) return eval_w<T, 2>(w, a, ep, deriv, gs, s);
@@ -1073,12 +1070,12 @@ int eval_dim(int dim, int w, PWArgs<T>& a, const EvalPtrs<T>& ep, bool deriv, DB
 }  // namespace
 
 template <typename T>
-int pw_eval(const PWParams& P, const Tree& t, const Lists& L, const PWData<T>& D,
-            const EvalSet<T>& e0, const EvalSet<T>& e1, int small_eval, PWWork* work,
-            cudaStream_t s) {
+void pw_eval(const PWParams& P, const Tree& t, const Lists& L, const PWData<T>& D,
+             const EvalSet<T>& e0, const EvalSet<T>& e1, int small_eval, PWWork* work,
+             cudaStream_t s) {
   // both evaluation sets (sources, targets) share the grid of every box
   const bool u0 = e0.pgh > 0 && e0.n > 0, u1 = e1.pgh > 0 && e1.n > 0;
-  if (!(u0 || u1) || L.n_eval <= 0) return 0;
+  if (!(u0 || u1) || L.n_eval <= 0) return;
   const int pgh_max = std::max(u0 ? e0.pgh : 0, u1 ? e1.pgh : 0);
   // Grids of the evaluation: potential only (width w); potential and
   // gradient from one grid through the kernel derivative, whose aliasing
@@ -1099,7 +1096,6 @@ int pw_eval(const PWParams& P, const Tree& t, const Lists& L, const PWData<T>& D
   PWArgs<T> a;
   DevTables<T> tb;
   make_args<T>(Pe, a, tb, s, false, 1);
-  int launches = 0;
   // boxes with at most thr evaluation points use the modal sums; thr is
   // capped by the modal kernel's shared memory (per point: FP64 partials of
   // every warp and the phase factors)
@@ -1121,7 +1117,6 @@ int pw_eval(const PWParams& P, const Tree& t, const Lists& L, const PWData<T>& D
   k_split_fill<<<grid_for(L.n_eval, 256), 256, 0, s>>>(L.n_eval, big, pos, lbig, lsmall, tot,
                                                         counts);
   FGT_LAUNCH_CHECK();
-  launches += 3;
   int nh = P.dim * (P.dim + 1) / 2;
   auto ncomp = [&](int pgh) { return pgh <= 0 ? 0 : 1 + (pgh >= 2 ? P.dim : 0) + (pgh >= 3 ? nh : 0); };
   EvalPtrs<T> ep;
@@ -1196,11 +1191,8 @@ int pw_eval(const PWParams& P, const Tree& t, const Lists& L, const PWData<T>& D
     ep.item_off = il.ioff;
     ep.n_items = il.n_items;
     ep.max_items = il.max_items;
-    launches += 6 + eval_dim<T>(P.dim, Pe.w, a, ep, deriv, gs, s);
-    if (small2) {
-      eval_small2_w<T>(Pe.w, deriv, a, ep, first2, next2, s);
-      launches += 2;
-    }
+    eval_dim<T>(P.dim, Pe.w, a, ep, deriv, gs, s);
+    if (small2) eval_small2_w<T>(Pe.w, deriv, a, ep, first2, next2, s);
   }
   {
     ep.boxes = lsmall;
@@ -1245,7 +1237,6 @@ int pw_eval(const PWParams& P, const Tree& t, const Lists& L, const PWData<T>& D
       k_eval_modal<T, 3><<<grid, MODAL_THREADS, sm, s>>>(a, ep, thr);
     }
     FGT_LAUNCH_CHECK();
-    launches++;
   }
   if (work) {
     unsigned long long h[2] = {0, 0};
@@ -1266,7 +1257,6 @@ int pw_eval(const PWParams& P, const Tree& t, const Lists& L, const PWData<T>& D
     work->w_eval = Pe.w;
     work->G_eval = Pe.G;
   }
-  return launches;
 }
 
 }  // namespace fgt

@@ -51,7 +51,8 @@ typedef struct fgt_stats {
   int n_translations;    /* sum over boxes of the PW list length */
   int spread_width;      /* kernel width of the spreader */
   int grid_cells;        /* spreading sub-grid cells per dimension */
-  int n_kernel_launches; /* kernels launched by this call */
+  int n_kernel_launches; /* kernels launched by this call (without those that
+                            only count for these statistics) */
   double near_pairs;     /* source/target pairs of the direct near field */
   /* algorithmic work of the call (FP32 or FP64 flops, HBM bytes) */
   double flops_form;     /* spreading stencils + DFT passes of the form kernel */

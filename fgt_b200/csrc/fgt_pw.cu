@@ -969,6 +969,21 @@ __global__ void k_count_points(int n, const int* __restrict__ box, const int* __
     atomicAdd(cnt, (unsigned long long)(hi[box[i]] - lo[box[i]]));
 }
 
+// Expansions that the sibling groups read (statistics): entries of `np` per
+// group, to the closing one where the list is closed, else those not empty.
+__global__ void k_count_sources(int n_grp, int np, bool closed, const int* __restrict__ gsrc,
+                                unsigned long long* __restrict__ cnt) {
+  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < n_grp; g += gridDim.x * blockDim.x) {
+    int c = 0;
+    for (int i = 0; i < np; i++) {
+      const bool on = gsrc[(size_t)g * np + i] >= 0;
+      if (!on && closed) break;
+      c += on;
+    }
+    if (c) atomicAdd(cnt, (unsigned long long)c);
+  }
+}
+
 // The launch's arguments for the FP64 matrix-instruction kernels.
 Form64 form64_args(const FormIO& io, const FormPtrs<double>& fp) {
   Form64 f;
@@ -1333,15 +1348,28 @@ void pw_translate(const PWParams& P, const Lists& L, PWData<T>& D, PWWork* work,
                                                                    P.xmin, D.wtab);
   FGT_LAUNCH_CHECK();
   D.loc.alloc((size_t)std::max(L.n_eval, 1) * P.nd * 2 * P.nexp, s);
-  if (work)
-    work->bytes_translate = (double)sizeof(T) * 2 * P.nexp * P.nd *
-                            ((double)L.n_trans + 2.0 * L.n_eval);
   if (L.n_eval == 0) return;
   // FP64 and 2D read memory less often by groups: 10^7 points in a periodic
   // square 2.1 -> 0.78 ms, spheres of 4e6 points at 1e-9 2.7 -> 1.9 and of 2e6
   // at 1e-6 1.2 -> 1.0.  In FP32 3D the expansions fit the L2 and the kernel by
   // lists is as fast (0.56 / 0.57 ms at 1e6 points, 0.74 / 0.71 at 10^7).
-  if (L.n_grp > 0 && (P.dim < 3 || sizeof(T) == 8)) {
+  const bool groups = L.n_grp > 0 && (P.dim < 3 || sizeof(T) == 8);
+  if (work) {  // every expansion read once per group, or once per list entry, and written once
+    double reads = (double)L.n_trans + L.n_eval;
+    if (groups) {
+      DBuf<unsigned long long> c;
+      c.alloc_zeroed(1, s);
+      k_count_sources<<<grid_for(L.n_grp, 256), 256, 0, s>>>(L.n_grp, 1 << (2 * P.dim), P.dim == 3,
+                                                            L.grp_src, c);
+      FGT_CUDA(cudaGetLastError());  // not one of the call's launches
+      unsigned long long h = 0;
+      FGT_CUDA(cudaMemcpyAsync(&h, c.get(), sizeof(h), cudaMemcpyDeviceToHost, s));
+      FGT_CUDA(cudaStreamSynchronize(s));
+      reads = (double)h;
+    }
+    work->bytes_translate = (double)sizeof(T) * 2 * P.nexp * P.nd * (reads + L.n_eval);
+  }
+  if (groups) {
     // a few waves of blocks; a thread's factors serve all its groups
     const int gx = ceil_div(P.nexp, TG_THREADS);
     const dim3 grid(gx, std::max(1, std::min({L.n_grp, 65535, ceil_div(12 * kSMs, gx)})));

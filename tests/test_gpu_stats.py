@@ -1,11 +1,12 @@
 """fgt_stats against what ran: the launch count against the kernels that the
-profiler saw.  Whole numbers: no tolerance."""
+profiler saw, the translation's bytes against the lists of the debug tree.
+Whole numbers: no tolerance."""
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
 
-COUNTERS = ("k_count_points",)  # kernels of the statistics themselves
+COUNTERS = ("k_count_points", "k_count_sources")  # kernels of the statistics themselves
 
 
 def _kernels(f):
@@ -53,3 +54,32 @@ def test_launch_count(fgt, monkeypatch, name, tree):
     r, names = _kernels(lambda: fgt.pfgt(**CASES[name]))
     assert names, "the profiler saw no kernel"
     assert r["stats"]["n_kernel_launches"] == len(names)
+
+
+@pytest.mark.parametrize("dim,delta,nd,prec", [
+    (1, 1e-4, 1, "fp64"), (1, 1e-4, 1, "mixed"), (2, 1e-3, 2, "fp64"), (2, 1e-3, 1, "mixed"),
+    (3, 4e-3, 1, "fp64"), (3, 4e-3, 2, "mixed"),
+])
+def test_translation_bytes(fgt, dim, delta, nd, prec):
+    """By groups (1D, 2D, FP64) the children of one parent read every expansion
+    around them once; by lists every box reads its own and its list's."""
+    rng = np.random.default_rng(8)
+    n = {1: 3000, 2: 9000, 3: 20000}[dim]
+    src = rng.uniform(-0.5, 0.5, (n, dim)) ** 3 * 4  # dense in the middle: some boxes are leaves
+    fp64 = prec == "fp64"
+    st = fgt.pfgt(nd, dim, delta, 1e-6, 0, src, charge=rng.standard_normal((n, nd)), stats=True,
+                  precision=fgt.PREC_FP64 if fp64 else fgt.PREC_MIXED)["stats"]
+    t = fgt.debug_tree(dim, delta, 1e-6, 0, src, None)
+    ptr, lst, own = t["trans_ptr"], t["trans_src"], t["eval_self"]
+    assert t["n_trans"] > 0 and t["n_form"] < t["n_eval"]
+    if dim < 3 or fp64:
+        sets = {}
+        for e, b in enumerate(t["eval_box"]):
+            s = sets.setdefault(t["parent"][b], set())
+            s.update(lst[ptr[e]:ptr[e + 1]])
+            s.update([own[e]] if own[e] >= 0 else [])
+        reads = sum(len(s) for s in sets.values())
+    else:
+        reads = t["n_trans"] + t["n_eval"]
+    nexp = (st["npw"] + 1) ** (dim - 1) * (st["npw"] // 2 + 1)  # modes -npw/2 .. npw/2, half of one
+    assert st["bytes_translate"] == (16 if fp64 else 8) * nexp * nd * (reads + t["n_eval"])

@@ -1209,7 +1209,6 @@ bool modal64_launch(const void* av, const Eval64& io, int pmax, size_t smem, cud
   auto go = [&](auto kern) {
     set_smem(kern, smem);
     kern<<<std::max(1, std::min(io.nbox, kSMs * 4)), T64, smem, s>>>(a, io, pmax);
-    FGT_LAUNCH_CHECK();
   };
   const bool grad = io.ncomp_max > 1;
   if (ks <= 8) grad ? go(k_modal64<8, true>) : go(k_modal64<8, false>);

@@ -45,7 +45,7 @@ bool eval64_takes(int w, int K, int G, bool wrap);
 void form64_launch(int w, const void* a, const Form64& io, cudaStream_t s);
 // Modal sums of the boxes with at most pmax points (3D; smem: dynamic shared
 // memory, at least 3 (2K+1) pmax complex + (2K+1) + 256 doubles); false: not
-// taken (hessians, expansions too long).
+// taken (hessians, expansions too long).  The caller checks the launch.
 bool modal64_launch(const void* a, const Eval64& io, int pmax, size_t smem, cudaStream_t s);
 void eval64_launch(int w, bool deriv, const void* a, const Eval64& io, cudaStream_t s);
 

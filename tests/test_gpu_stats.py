@@ -32,15 +32,17 @@ def _case(dim, n, nt, delta, eps, nd=1, pgh=1, dip=False, period=0, **kw):
     return c
 
 
+# ndiv below the points of a box of the cut-off's size: plane waves in all but the last two
 CASES = {
-    "3d_mixed_small": _case(3, 3001, 0, 1e-3, 1e-6),
-    "3d_mixed_split_sets": _case(3, 300001, 30001, 1e-3, 1e-3, pgh=2),  # two launches of inverses
-    "3d_fp64": _case(3, 9001, 500, 4e-3, 1e-9, pgh=2),
-    "3d_fp64_hess": _case(3, 9001, 0, 4e-3, 1e-9, pgh=3, dip=True, nd=2),
-    "3d_periodic": _case(3, 9001, 0, 4e-3, 1e-6, period=1),
-    "2d_fp64_nd5": _case(2, 20001, 900, 1e-4, 1e-9, nd=5, pgh=2),
-    "2d_mixed": _case(2, 20001, 0, 1e-4, 1e-6, pgh=3),
-    "1d_deep": _case(1, 5001, 100, 1e-9, 1e-6, ndiv=3),
+    "3d_mixed_small": _case(3, 3001, 0, 1e-3, 1e-6, ndiv=2),
+    "3d_mixed_split_sets": _case(3, 300001, 30001, 1e-3, 1e-3, pgh=2, ndiv=20),  # two launches of inverses
+    "3d_fp64": _case(3, 9001, 500, 4e-3, 1e-9, pgh=2, ndiv=20),
+    "3d_fp64_hess": _case(3, 9001, 0, 4e-3, 1e-9, pgh=3, dip=True, nd=2, ndiv=20),
+    "3d_periodic": _case(3, 9001, 0, 4e-3, 1e-6, period=1, ndiv=20),
+    "2d_fp64_nd5": _case(2, 20001, 900, 1e-4, 1e-9, nd=5, pgh=2, ndiv=10),
+    "2d_mixed": _case(2, 20001, 0, 1e-4, 1e-6, pgh=3, ndiv=10),
+    "1d": _case(1, 5001, 100, 1e-6, 1e-6, ndiv=3),
+    "1d_deep": _case(1, 5001, 100, 1e-12, 1e-6),
     "root_only": _case(3, 100, 0, 1e-1, 1e-6),
 }
 
@@ -53,6 +55,7 @@ def test_launch_count(fgt, monkeypatch, name, tree):
     fgt.pfgt(**CASES[name])
     r, names = _kernels(lambda: fgt.pfgt(**CASES[name]))
     assert names, "the profiler saw no kernel"
+    assert (r["stats"]["n_form_boxes"] > 0) == (name not in ("1d_deep", "root_only"))
     assert r["stats"]["n_kernel_launches"] == len(names)
 
 

@@ -522,9 +522,10 @@ DirectGeom direct_geom(const Setup& u) {
 }
 
 // near_lists: build the positions of the packed list-1 sources (one density;
-// used by executions with charges only and pgh <= 2).
+// used by executions with charges only and pgh <= 2).  fp64: the executions'
+// arithmetic.
 void setup_geometry(Setup& u, const Call& c, double* bs0_io, double* cen0_io, const fgt_opts& o,
-                    bool near_lists, cudaStream_t s, Timer& tm) {
+                    bool near_lists, bool fp64, cudaStream_t s, Timer& tm) {
   const int dim = c.dim;
   u.dim = dim;
   u.nd = c.nd;
@@ -597,7 +598,7 @@ void setup_geometry(Setup& u, const Call& c, double* bs0_io, double* cen0_io, co
     do_pw = false;
     nlevend = 0;
   }
-  build_lists(t, npwlevel, iperiod0, nlevend, do_pw, u.L, s);
+  build_lists(t, npwlevel, iperiod0, nlevend, do_pw, translates_by_groups(dim, fp64), u.L, s);
   tm.mark(3);
   // --- gather (dreorderf, fmmcommon2d.f:3-27) as offsets from reference boxes
   u.soff.alloc((size_t)c.ns * dim, s);
@@ -842,7 +843,7 @@ void run_pfgt(const Call& c, double* bs0_io, double* cen0_io, const fgt_opts& o,
   // the packed near-field path: one density, charges only, pgh <= 2
   const bool near = c.nd == 1 && c.ifcharge && !c.ifdipole && c.ifpgh <= 2 &&
                     c.ifpghtarg <= 2;
-  setup_geometry(u, c, bs0_io, cen0_io, o, near, s, tm);
+  setup_geometry(u, c, bs0_io, cen0_io, o, near, sizeof(T) == 8, s, tm);
   fgt_opts oo = o;
   int tuned = 0;
   if (o.autotune > 0 && o.small_eval < 0 && u.do_pw) {
@@ -1157,7 +1158,7 @@ fgt_plan* plan_create_impl(const fgt_opts* opts_in, int nd, int dim, double delt
       }
     }
     Timer tm(false, s);
-    setup_geometry(pl->u, c, bs0, cen0, o, nd == 1, s, tm);
+    setup_geometry(pl->u, c, bs0, cen0, o, nd == 1, pl->prec == FGT_PREC_FP64, s, tm);
     FGT_CUDA(cudaStreamSynchronize(s));
   } catch (...) {
     cudaStreamSynchronize(s);
@@ -1424,7 +1425,7 @@ extern "C" void* fgt_debug_tree_build(int dim, double delta, double eps, int ipe
       nlevend = 0;
     }
     Lists L;
-    build_lists(t, npwlevel, iperiod0, nlevend, do_pw, L, s);
+    build_lists(t, npwlevel, iperiod0, nlevend, do_pw, true, L, s);
     DebugTree* d = new DebugTree();
     tree_download(t, d->th, s);
     lists_download(L, t.nboxes, d->lh, s);

@@ -374,8 +374,8 @@ __global__ void k_eval_self(int n_eval, const int* __restrict__ eval_box,
 }
 }  // namespace
 
-void build_lists(const Tree& t, int npwlevel, int iperiod0, int nlevend, bool do_pw, Lists& L,
-                 cudaStream_t s) {
+void build_lists(const Tree& t, int npwlevel, int iperiod0, int nlevend, bool do_pw, bool groups,
+                 Lists& L, cudaStream_t s) {
   TV tv = make_tv(t, npwlevel, iperiod0, nlevend);
   int nb = t.nboxes;
   // direct near field: list lengths; the plane-wave box flags are counted
@@ -430,7 +430,8 @@ void build_lists(const Tree& t, int npwlevel, int iperiod0, int nlevend, bool do
     FGT_LAUNCH_CHECK();
   }
   // levels of two boxes a side and up: no position around a group repeats
-  if (t.ncutoff >= 1 && (iperiod0 != 1 || t.ncutoff >= 2) && L.n_eval > 0 && L.n_form < (1 << 25)) {
+  if (groups && t.ncutoff >= 1 && (iperiod0 != 1 || t.ncutoff >= 2) && L.n_eval > 0 &&
+      L.n_form < (1 << 25)) {
     L.n_grp = n / t.mc;
     L.grp_src.alloc((size_t)L.n_grp << (2 * t.dim), s);
     L.grp_trg.alloc((size_t)L.n_grp * t.mc, s);

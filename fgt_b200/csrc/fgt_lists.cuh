@@ -26,9 +26,17 @@ struct Lists {
   int n_l1 = 0;
 };
 
-// nlevend / iperiod0 follow pfgtmain (src/pfgt/pfgt.f:618-650).
-void build_lists(const Tree& t, int npwlevel, int iperiod0, int nlevend, bool do_pw, Lists& L,
-                 cudaStream_t s);
+// Whether the translation goes by sibling groups.  FP64 and 2D read memory less
+// often so: 10^7 points in a periodic square 2.1 -> 0.78 ms, spheres of 4e6
+// points at 1e-9 2.7 -> 1.9 and of 2e6 at 1e-6 1.2 -> 1.0.  In FP32 3D the
+// expansions fit the L2 and the kernel by lists is as fast (0.56 / 0.57 ms at
+// 1e6 points, 0.74 / 0.71 at 10^7).
+inline bool translates_by_groups(int dim, bool fp64) { return dim < 3 || fp64; }
+
+// nlevend / iperiod0 follow pfgtmain (src/pfgt/pfgt.f:618-650); groups: build
+// the sibling groups too.
+void build_lists(const Tree& t, int npwlevel, int iperiod0, int nlevend, bool do_pw, bool groups,
+                 Lists& L, cudaStream_t s);
 
 struct ListsHost {
   std::vector<int> form_box, eval_box, eval_self, trans_ptr, trans_src, trans_w, l1_ptr, l1_src;

@@ -1349,11 +1349,7 @@ void pw_translate(const PWParams& P, const Lists& L, PWData<T>& D, PWWork* work,
   FGT_LAUNCH_CHECK();
   D.loc.alloc((size_t)std::max(L.n_eval, 1) * P.nd * 2 * P.nexp, s);
   if (L.n_eval == 0) return;
-  // FP64 and 2D read memory less often by groups: 10^7 points in a periodic
-  // square 2.1 -> 0.78 ms, spheres of 4e6 points at 1e-9 2.7 -> 1.9 and of 2e6
-  // at 1e-6 1.2 -> 1.0.  In FP32 3D the expansions fit the L2 and the kernel by
-  // lists is as fast (0.56 / 0.57 ms at 1e6 points, 0.74 / 0.71 at 10^7).
-  const bool groups = L.n_grp > 0 && (P.dim < 3 || sizeof(T) == 8);
+  const bool groups = L.n_grp > 0 && translates_by_groups(P.dim, sizeof(T) == 8);
   if (work) {  // every expansion read once per group, or once per list entry, and written once
     double reads = (double)L.n_trans + L.n_eval;
     if (groups) {

@@ -1,6 +1,6 @@
 """fgt_stats against what ran: the launch count against the kernels that the
-profiler saw, the translation's bytes against the lists of the debug tree.
-Whole numbers: no tolerance."""
+profiler saw, the translation's bytes against the lists of the debug tree; and
+no group tables in calls that translate by lists.  Whole numbers: no tolerance."""
 import numpy as np
 import pytest
 
@@ -86,3 +86,11 @@ def test_translation_bytes(fgt, dim, delta, nd, prec):
         reads = t["n_trans"] + t["n_eval"]
     nexp = (st["npw"] + 1) ** (dim - 1) * (st["npw"] // 2 + 1)  # modes -npw/2 .. npw/2, half of one
     assert st["bytes_translate"] == (16 if fp64 else 8) * nexp * nd * (reads + t["n_eval"])
+
+
+@pytest.mark.parametrize("name", ["3d_mixed_split_sets", "3d_periodic", "3d_fp64", "2d_mixed"])
+def test_groups_only_where_they_are_read(fgt, name):
+    fgt.pfgt(**CASES[name])
+    _, names = _kernels(lambda: fgt.pfgt(**CASES[name]))
+    assert any("k_translate" in n for n in names)
+    assert any("k_groups" in n for n in names) == any("k_translate_groups" in n for n in names)

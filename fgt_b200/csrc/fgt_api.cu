@@ -627,9 +627,10 @@ void setup_geometry(Setup& u, const Call& c, double* bs0_io, double* cen0_io, co
   u.do_pw = do_pw;
 }
 
-// Strength-dependent part of a call on a prepared geometry.
+// Strength-dependent part of a call on a prepared geometry.  Returns the packed
+// records of the near field, 0 where it walked the list.
 template <typename T>
-void execute(const Setup& u, const Call& c, const fgt_opts& o, fgt_stats* st, cudaStream_t s,
+long long execute(const Setup& u, const Call& c, const fgt_opts& o, fgt_stats* st, cudaStream_t s,
              Timer& tm) {
   const int dim = u.dim, nd = u.nd, nhess = dim * (dim + 1) / 2;
   const Tree& t = u.t;
@@ -757,6 +758,7 @@ void execute(const Setup& u, const Call& c, const fgt_opts& o, fgt_stats* st, cu
     st->bs0 = u.bs0;
     for (int k = 0; k < dim; k++) st->cen0[k] = u.cen0[k];
   }
+  return packed.rec ? u.near_total : 0;
 }
 
 // ---------------------------------------------------------------- autotuner
@@ -837,7 +839,7 @@ int tune_small_eval(const Setup& u, const Call& c, const fgt_opts& o, cudaStream
 }
 
 template <typename T>
-void run_pfgt(const Call& c, double* bs0_io, double* cen0_io, const fgt_opts& o, fgt_stats* st,
+long long run_pfgt(const Call& c, double* bs0_io, double* cen0_io, const fgt_opts& o, fgt_stats* st,
               cudaStream_t s, Timer& tm) {
   Setup u;
   // the packed near-field path: one density, charges only, pgh <= 2
@@ -857,11 +859,12 @@ void run_pfgt(const Call& c, double* bs0_io, double* cen0_io, const fgt_opts& o,
       tuned = 1;
     }
   }
-  execute<T>(u, c, oo, st, s, tm);
+  const long long near_records = execute<T>(u, c, oo, st, s, tm);
   if (st) {
     st->small_eval_used = oo.small_eval >= 0 ? oo.small_eval : default_small_eval(c.dim);
     st->tuned = tuned;
   }
+  return near_records;
 }
 
 bool fault_requested(const char* what) {
@@ -878,7 +881,7 @@ bool log_requested() {
   return f && *f && strcmp(f, "0") != 0;
 }
 
-void log_call(const fgt_stats& st, int nd, int dim, int ns, int nt, double delta, double eps) {
+void log_call(const fgt_stats& st, long long near_records, int nd, int dim, int ns, int nt, double delta, double eps) {
   static std::mutex mu;
   char ms[512];
   int k = snprintf(ms, sizeof(ms), "{");
@@ -892,12 +895,12 @@ void log_call(const fgt_stats& st, int nd, int dim, int ns, int nt, double delta
           "{\"fgt\": \"pfgt\", \"nd\": %d, \"dim\": %d, \"ns\": %d, \"nt\": %d, "
           "\"delta\": %.6g, \"eps\": %.6g, \"precision\": \"%s\", \"nlevels\": %d, "
           "\"nboxes\": %d, \"npwlevel\": %d, \"npw\": %d, \"n_form_boxes\": %d, "
-          "\"n_eval_boxes\": %d, \"n_translations\": %d, \"near_pairs\": %.6g, "
+          "\"n_eval_boxes\": %d, \"n_translations\": %d, \"near_pairs\": %.6g, \"near_records\": %lld, "
           "\"kernel_launches\": %d, \"ms\": %s, \"tflops\": {\"form\": %.4g, "
           "\"eval\": %.4g, \"direct\": %.4g}, \"translate_gbs\": %.4g}\n",
           nd, dim, ns, nt, delta, eps, st.precision_used == FGT_PREC_FP64 ? "fp64" : "mixed",
           st.nlevels, st.nboxes, st.npwlevel, st.npw, st.n_form_boxes, st.n_eval_boxes,
-          st.n_translations, st.near_pairs, st.n_kernel_launches, ms,
+          st.n_translations, st.near_pairs, near_records, st.n_kernel_launches, ms,
           rate(st.flops_form, st.ms[4]) * 1e-12, rate(st.flops_eval, st.ms[6]) * 1e-12,
           rate(st.flops_direct, st.ms[7]) * 1e-12, rate(st.bytes_translate, st.ms[5]) * 1e-9);
   fflush(stderr);
@@ -1041,8 +1044,9 @@ int pfgt_impl(const fgt_opts* opts_in, int nd, int dim, double delta, double eps
   c.gradt = c.ifpghtarg >= 2 ? dout(d_gt, gradtarg, (size_t)nt * nd * dim) : nullptr;
   c.hesst = c.ifpghtarg >= 3 ? dout(d_ht, hesstarg, (size_t)nt * nd * nhess) : nullptr;
   tm.mark(0);
-  if (prec == FGT_PREC_FP64) run_pfgt<double>(c, bs0, cen0, o, st, s, tm);
-  else run_pfgt<float>(c, bs0, cen0, o, st, s, tm);
+  const long long near_records = prec == FGT_PREC_FP64
+                                     ? run_pfgt<double>(c, bs0, cen0, o, st, s, tm)
+                                     : run_pfgt<float>(c, bs0, cen0, o, st, s, tm);
   if (!o.device_ptrs) {
     // source outputs on the side stream once they are final, target outputs
     // on the call's stream
@@ -1074,7 +1078,7 @@ int pfgt_impl(const fgt_opts* opts_in, int nd, int dim, double delta, double eps
     st->n_kernel_launches = (int)(launch_count() - launches0);
     st->precision_used = prec;
     tm.finish(st->ms);
-    if (logging) log_call(*st, nd, dim, ns, nt, delta, eps);
+    if (logging) log_call(*st, near_records, nd, dim, ns, nt, delta, eps);
   }
   return FGT_OK;
 }

@@ -878,6 +878,9 @@ __global__ void __launch_bounds__(T64, 1)
           }
         }
       }
+      // the next unit's kernel sums and cells take the place of those just read:
+      // the shuffle that hands out the unit orders no memory
+      __syncwarp();
       }
       __syncthreads();
     }

@@ -287,7 +287,7 @@ __global__ void k_scan_apply(const int* in, int* out, int n, const int* __restri
     s += v[j];
   }
   int tot;
-  int ex = block_excl_scan(s, &tot) + (part ? part[blockIdx.x] : 0);
+  int ex = block_excl_scan(s, &tot) + part[blockIdx.x];
   for (int j = 0; j < SCAN_ITEMS; j++) {
     int i = base + threadIdx.x * SCAN_ITEMS + j;
     if (i < n) out[i] = ex;
@@ -582,11 +582,6 @@ void exclusive_scan_i32(const int* in, int* out, int n, int* total, cudaStream_t
     return;
   }
   int nb = ceil_div(n, SCAN_TILE);
-  if (nb == 1) {
-    k_scan_apply<<<1, SCAN_THREADS, 0, s>>>(in, out, n, nullptr, total, 1);
-    FGT_LAUNCH_CHECK();
-    return;
-  }
   DBuf<int> part(nb, s);
   k_scan_reduce<<<nb, SCAN_THREADS, 0, s>>>(in, n, part);
   FGT_LAUNCH_CHECK();

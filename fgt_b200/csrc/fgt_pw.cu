@@ -691,10 +691,10 @@ __global__ void k_translate(int n_eval, int n_form, int nsh, int nexp, int nd, i
 // The same sums by sibling groups: a thread holds one mode's 3^DIM shift
 // factors in registers and, for every group, the sums of its 2^DIM children;
 // each of the 4^DIM expansions around them is read once for all of them
-// instead of once per child, and the factors once for many groups.  In 1D and
-// 2D row by row with the next row in flight.  A child's own
-// expansion comes first, then its neighbours with the first coordinate
-// fastest: the order of its list.  With the roundings written out (left to
+// instead of once per child, and the factors once for many groups.  Here 1D and
+// 2D, row by row with the next row in flight.  A child's own expansion comes
+// first, then its neighbours with the first coordinate fastest: the order of
+// its list.  With the roundings written out (left to
 // the compiler, they change with the code around them) the FP32 sums are
 // k_translate's bit for bit.
 __device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
@@ -707,7 +707,7 @@ __global__ void __launch_bounds__(128)
                        const int* __restrict__ gtrg, const T* __restrict__ mp,
                        const T* __restrict__ wtab, T* __restrict__ loc) {
   using V = typename std::conditional<sizeof(T) == 4, float2, double2>::type;
-  constexpr int MC = 1 << DIM, NP = 1 << (2 * DIM), NW = DIM == 3 ? 27 : (DIM == 2 ? 9 : 3);
+  constexpr int MC = 1 << DIM, NP = 1 << (2 * DIM), NW = DIM == 2 ? 9 : 3;
   constexpr int ROWS = NP / 4;
   const V* mpv = reinterpret_cast<const V*>(mp);
   V* lv = reinterpret_cast<V*>(loc);
@@ -838,29 +838,25 @@ __device__ __forceinline__ void vzero(V* v) {
 #pragma unroll
   for (int i = 0; i < N; i++) v[i].x = v[i].y = 0;
 }
-template <typename T, int MODES = 1>
+template <typename T>
 __global__ void __launch_bounds__(TG_THREADS, 5)
     k_translate_groups3(int n_grp, int n_form, int nexp, int nd, const int* __restrict__ gsrc,
                         const int* __restrict__ gtrg, const T* __restrict__ mp,
                         const T* __restrict__ wtab, T* __restrict__ loc) {
   using V = typename std::conditional<sizeof(T) == 4, float2, double2>::type;
-  __shared__ V ring[TG_RING][MODES][TG_THREADS];
+  __shared__ V ring[TG_RING][TG_THREADS];
   const V* mpv = reinterpret_cast<const V*>(mp);
   V* lv = reinterpret_cast<V*>(loc);
   const int lane = threadIdx.x & 31;
-  int m[MODES];          // idle lanes read a valid mode and write none
-  V wm[MODES][3], wp[MODES][3];  // shifts by -1 and +1 along each dimension
+  // idle lanes read a valid mode and write none
+  const int m = blockIdx.x * TG_THREADS + threadIdx.x, mc = min(m, nexp - 1);
+  V wm[3], wp[3];  // shifts by -1 and +1 along each dimension
 #pragma unroll
-  for (int k = 0; k < MODES; k++) {
-    m[k] = (blockIdx.x * MODES + k) * TG_THREADS + threadIdx.x;
-    const int mc = min(m[k], nexp - 1);
-#pragma unroll
-    for (int d = 0, inc = 1; d < 3; d++, inc *= 3) {
-      wm[k][d] = reinterpret_cast<const V*>(wtab)[(size_t)(13 - inc) * nexp + mc];
-      wp[k][d] = reinterpret_cast<const V*>(wtab)[(size_t)(13 + inc) * nexp + mc];
-    }
+  for (int d = 0, inc = 1; d < 3; d++, inc *= 3) {
+    wm[d] = reinterpret_cast<const V*>(wtab)[(size_t)(13 - inc) * nexp + mc];
+    wp[d] = reinterpret_cast<const V*>(wtab)[(size_t)(13 + inc) * nexp + mc];
   }
-  const unsigned ring0 = (unsigned)__cvta_generic_to_shared(&ring[0][0][threadIdx.x]);
+  const unsigned ring0 = (unsigned)__cvta_generic_to_shared(&ring[0][threadIdx.x]);
   // a run of groups: neighbours in Morton order read the same expansions
   const int g1 = (int)((long long)n_grp * (blockIdx.y + 1) / gridDim.y);
   for (int g = (int)((long long)n_grp * blockIdx.y / gridDim.y); g < g1; g++) {
@@ -877,26 +873,20 @@ __global__ void __launch_bounds__(TG_THREADS, 5)
           const int sl = __shfl_sync(0xffffffffu, j < 32 ? e0 : e1, j & 31) >> 6;
           if (FGT_DCHECK(sl < n_form, 205)) {
             const V* p = mpv + ((size_t)sl * nd + id) * nexp;
-            const unsigned dst = ring0 + (j % TG_RING) * (unsigned)(MODES * TG_THREADS * sizeof(V));
-#pragma unroll
-            for (int k = 0; k < MODES; k++)
-              asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
-                               dst + k * (unsigned)(TG_THREADS * sizeof(V))),
-                           "l"(p + min(m[k], nexp - 1)), "n"(sizeof(V))
-                           : "memory");
+            const unsigned dst = ring0 + (j % TG_RING) * (unsigned)(TG_THREADS * sizeof(V));
+            asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(p + mc),
+                         "n"(sizeof(V))
+                         : "memory");
           }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
       };
 #pragma unroll 1
       for (int j = 0; j < TG_RING - 1; j++) issue(j);
-      V acc[MODES][8], pl[MODES][4], rw[MODES][2];  // acc, pl: x fastest
-#pragma unroll
-      for (int k = 0; k < MODES; k++) {
-        vzero<8>(acc[k]);
-        vzero<4>(pl[k]);
-        vzero<2>(rw[k]);
-      }
+      V acc[8], pl[4], rw[2];  // acc, pl: x fastest
+      vzero<8>(acc);
+      vzero<4>(pl);
+      vzero<2>(rw);
 #pragma unroll 1
       for (int j = 0; j < n; j++) {
         issue(j + TG_RING - 1);
@@ -904,23 +894,14 @@ __global__ void __launch_bounds__(TG_THREADS, 5)
         const int jn = j + 1;
         const int pn = jn < n ? __shfl_sync(0xffffffffu, jn < 32 ? e0 : e1, jn & 31) & 63 : 64;
         asm volatile("cp.async.wait_group %0;" ::"n"(TG_RING - 1) : "memory");
-#pragma unroll
-        for (int k = 0; k < MODES; k++) {
-          const V a = ring[j % TG_RING][k][threadIdx.x];
-          tg_add<1>(p & 3, &rw[k][0], &rw[k][1], &a, wp[k][0], wm[k][0]);
-        }
+        const V a = ring[j % TG_RING][threadIdx.x];
+        tg_add<1>(p & 3, &rw[0], &rw[1], &a, wp[0], wm[0]);
         if (p >> 2 != pn >> 2) {  // the row's last
-#pragma unroll
-          for (int k = 0; k < MODES; k++) {
-            tg_add<2>((p >> 2) & 3, pl[k], pl[k] + 2, rw[k], wp[k][1], wm[k][1]);
-            vzero<2>(rw[k]);
-          }
+          tg_add<2>((p >> 2) & 3, pl, pl + 2, rw, wp[1], wm[1]);
+          vzero<2>(rw);
           if (p >> 4 != pn >> 4) {  // the plane's last
-#pragma unroll
-            for (int k = 0; k < MODES; k++) {
-              tg_add<4>(p >> 4, acc[k], acc[k] + 4, pl[k], wp[k][2], wm[k][2]);
-              vzero<4>(pl[k]);
-            }
+            tg_add<4>(p >> 4, acc, acc + 4, pl, wp[2], wm[2]);
+            vzero<4>(pl);
           }
         }
       }
@@ -928,9 +909,7 @@ __global__ void __launch_bounds__(TG_THREADS, 5)
 #pragma unroll
       for (int c = 0; c < 8; c++) {
         const int e = __shfl_sync(0xffffffffu, et, c);
-#pragma unroll
-        for (int k = 0; k < MODES; k++)
-          if (e >= 0 && m[k] < nexp) __stcs(lv + ((size_t)e * nd + id) * nexp + m[k], acc[k][c]);
+        if (e >= 0 && m < nexp) __stcs(lv + ((size_t)e * nd + id) * nexp + m, acc[c]);
       }
     }
   }

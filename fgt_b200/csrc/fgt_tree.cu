@@ -868,15 +868,7 @@ void tree_build_dense(Tree& t, const KeyParams& kp, const double* d_src, const d
   else if (dim == 2) keys(std::integral_constant<int, 2>{});
   else keys(std::integral_constant<int, 3>{});
   if (T <= TREE_ONE) {  // steps 2-4 in one block
-    const size_t sm = 5 * (size_t)T + 16;
-    static thread_local unsigned long long allowed = 0;  // devices, by bit
-    int dev = 0;
-    FGT_CUDA(cudaGetDevice(&dev));
-    if (dev >= 64 || !((allowed >> dev) & 1)) {
-      FGT_CUDA(cudaFuncSetAttribute(k_tree_one, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    5 * TREE_ONE + 16));
-      if (dev < 64) allowed |= 1ull << dev;
-    }
+    const size_t sm = 5 * (size_t)T + 16;  // 27 KB at most
     k_tree_one<<<1, 1024, sm, s>>>(cl, t.ndiv, hist, flag, rank, lev, base, table);
     FGT_LAUNCH_CHECK();
   } else {

@@ -162,8 +162,8 @@ def roofline(a, stats, ms_phase):
     ach = flops[dom] / (ms * 1e-3) / 1e12
     return {"bound": "fp32" if a.precision == "mixed" else "fp64", "kernel": names[dom],
             "achieved": ach, "peak": pk, "unit": "TFLOP/s", "frac": ach / pk, "traffic": tr,
-            "peak_source": "measured cuBLAS %s GEMM in bench.py (no tensor-core path: "
-                           "no step is a dense contraction)" % ("FP32" if dt == torch.float32 else "FP64"),
+            "peak_source": "measured cuBLAS %s GEMM in bench.py (FP32 sums run on the "
+                           "vector units; FP64 vector and matrix units share a rate)" % ("FP32" if dt == torch.float32 else "FP64"),
             "ms": ms, "flops": flops[dom]}
 
 

@@ -2,7 +2,7 @@
 // lane held in registers, list-1 sources staged through shared memory and
 // read as broadcasts.  Mixed precision: FP32 offsets from FP64 box centres,
 // FP32 exp (ex2.approx) and FP32 per-item accumulation, FP64 output
-// accumulation.  FP64 path: same kernel in double.
+// accumulation.  The FP64 path has kernels of its own (k_direct, k_direct64p).
 #include <stdlib.h>
 
 #include <algorithm>
@@ -95,9 +95,9 @@ __device__ __forceinline__ double exp_tab(const ExpTab& tab, double t) {
 // entries, into batches of 32 in shared memory and read as broadcasts.  An
 // item of at most 16, 8 or 4 points gives 2, 4 or 8 groups of lanes, each
 // with every 2nd, 4th or 8th source.  Bound by the FP64 pipe (26 instructions
-// a pair with the gradient): 2.5e9 listed pairs of config-2 clusters 6.9 ->
-// NEARMS ms against unpacked batches with the library exponential and a branch
-// on the cut-off.
+// a pair with the gradient).  Against unpacked batches with the library
+// exponential and a branch on the cut-off: clusters, N = M = 2e6, eps = 1e-9
+// (2.5e9 listed pairs), pot + grad of charges, 6.9 -> 5.9 ms.
 template <int DIM, int PGH, bool CHG, bool DIP, int NDC>
 __global__ void __launch_bounds__(DW * 32) k_direct(DArgs<double> a) {
   constexpr int NH = DIM * (DIM + 1) / 2;
@@ -699,10 +699,11 @@ __global__ void k_near_lists(NearArgs n) {
 // in batches of 32 through shared memory (the next batch in registers), items
 // of 32 points from a device counter.  An item of at most 16, 8 or 4 points
 // gives 2, 4 or 8 groups of lanes, each with every 2nd, 4th or 8th record.
-// Bound by the FP64 pipe (22 instructions a pair with the gradient, ~45 with
-// the library exponential).  Against the list walk with unpacked batches:
-// clusters, N = M = 2e6 (2.5e9 listed pairs, eps = 1e-9) 6.9 -> 4.1 ms plus
-// 0.2 for the records' positions, sphere, N = M = 2e6, eps = 1e-6 3.2 -> 2.3.
+// FP64 pipe (22 instructions a pair with the gradient, ~45 with the library
+// exponential; 56% busy, issue slots 61% on 1e6 points on a sphere).  Against the
+// list walk with unpacked batches: clusters, N = M = 2e6 (2.5e9 listed pairs,
+// eps = 1e-9) 6.9 -> 3.9 ms plus 0.2 for the records' positions (k_direct:
+// 5.9), sphere, N = M = 2e6, eps = 1e-6 3.2 -> 2.3.
 template <int DIM, int PGH>
 __global__ void __launch_bounds__(DW * 32) k_direct64p(DArgs<double> a, const int* __restrict__ pos,
                                                        const double2* __restrict__ rec,

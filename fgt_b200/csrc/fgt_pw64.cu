@@ -10,15 +10,16 @@
 // Every box has its grid in global memory; a form is spread -> (z, y) per
 // slab of x-planes -> x, an evaluation x, y, z per slab -> interpolate.
 //
-// Bound by the FP64 pipe.  Against W^3 atomics per point into a global grid,
+// FP64 pipe 42-64% busy (1e6 points on a sphere, eps = 1e-9), the rest waits
+// for operands at one or two CTAs per SM.  Against W^3 atomics per point into a global grid,
 // SIMT line transforms on one CTA per box and one stencil load per FMA
 // (N = M = 4e6 on a sphere, pot + grad, delta = 1e-4, eps = 1e-9): form 39.6
 // -> 3.9 ms, evaluation 37.2 -> 11.2 ms; N = M = 1.5e6, delta = 1e-2, eps =
-// 1e-12: 33.7 -> 2.1 and 21.1 -> 6.6 ms.  One fused kernel per direction
+// 1e-12: 33.7 -> 1.6 and 21.1 -> 5.0 ms.  One fused kernel per direction
 // (spreading and transforms of a box in one 256-thread CTA) took 4.9 and
 // 15.6 ms: the transforms want the 16 warps of two CTAs to hide their loads,
 // the spreading and the interpolation 200+ registers per thread.  Grids that
-// fit in shared memory gain too (N = M = 2e6, eps = 1e-6: form 3.2 -> 2.0,
+// fit in shared memory gain too (N = M = 2e6, eps = 1e-6: form 3.2 -> 1.9,
 // evaluation 7.8 -> 4.0 ms against a 200 KB grid and a SIMT stencil per CTA;
 // N = 1e5, eps = 1e-3: 0.43 -> 0.22 and 0.37 -> 0.17).
 #include <limits.h>

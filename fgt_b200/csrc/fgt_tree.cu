@@ -830,12 +830,16 @@ __global__ void k_dense_ranges(CellLevels cl, int nboxes, const uint64_t* __rest
 
 // The dense tables hold 2^(dim (D-1)) cells at the finest level they cover:
 // taken when clearing and scanning them (about 20 bytes a cell) stays small
-// against the points; up to 2^21 cells (~20 us) always.  Bound by launches
-// for few points and by HBM for many.  Tree phase against sorted keys, level
-// by level with a read-back each: uniform N = 1e5 (D = 6) 0.64 -> 0.27 ms,
-// N = 3e3 (D = 5) 0.43 -> 0.22 ms, clusters N + M = 4e6 (D = 8) 1.76 -> 0.83
-// ms, 2D periodic N = 1e7 2.14 -> 1.07 ms.  FGT_TREE_SORTED=1 takes the sorted
-// keys, to compare the two.
+// against the points, up to 2^21 cells always.  Bound by launches for few
+// points and by HBM for many.  Tree phase against sorted keys, level by level
+// with a read-back each, as both were at first and as it is now: uniform N = 1e5
+// (D = 6) 0.64 -> 0.16 ms, N = 3e3 (D = 5) 0.43 -> 0.12, clusters N + M = 4e6
+// (D = 8) 1.76 -> 0.59, 2D periodic N = 1e7 2.14 -> 0.83.  At the line, 2^21
+// cells in 3D, a whole call takes 0.44 ms against 0.38 by sorted keys for N =
+// 500, the same for 3e3 to 1e4 points, 0.47 / 0.56 for 3e4 and 0.55 / 0.75 for
+// 1e5; with 2^18 cells 0.27 / 0.36 for N = 500 and 0.41 / 0.79 for 1e5; with 2^20
+// in 2D 0.35 / 0.41 and 0.42 / 0.89.  FGT_TREE_SORTED=1 takes the sorted keys,
+// to compare the two.
 bool dense_tree_takes(int dim, int D, int ns, int nt) {
   if (D < 1 || dim * (D - 1) > 24 || ns < 1) return false;
   const char* e = getenv("FGT_TREE_SORTED");

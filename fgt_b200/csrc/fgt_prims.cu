@@ -133,8 +133,9 @@ void* Arena::try_alloc(size_t bytes) {
     (void)cudaGetLastError();
     if (want != bytes) continue;
     if (chunks.empty() || chunks.back().off) break;
+    (void)cudaDeviceSynchronize();  // kernels of this call may still use them
     while (!chunks.empty() && chunks.back().off == 0) {
-      cudaFree(chunks.back().p);  // waits for the kernels that used it
+      cudaFree(chunks.back().p);
       chunks.pop_back();
     }
   }
